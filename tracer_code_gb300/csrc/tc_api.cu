@@ -190,6 +190,7 @@ struct Handle {
     // queues its host work in `deferred`, which runs after every launch of
     // the graph in the order the eager step would have run it; the WHILE
     // bodies of the step's loops are captured on body_st
+    bool in_ensemble = false;  // stepped by tc_ensemble_run / tc_ensemble_step: no launches that need the whole GPU
     bool capturing = false;
     cudaStream_t body_st = nullptr;
     DevScalars* hsnap = nullptr;  // pinned, kMaxSnap entries
@@ -844,14 +845,28 @@ static void sweep_factors(int Niter, int n, int dir, bool cheb_pp, double* c, do
     *c = (dir != 1 && !cheb_pp) ? 2.0 / (-lb - la + (lb - la) * *temp) : 1.0;
 }
 
+// How the mixed solve's tile smoother (k_tile.cu) runs a visit of `level`: in one
+// cluster where the level fits (the other SMs stay free), else over the grid, a
+// cooperative launch that waits for all SMs: not in an ensemble, whose cases
+// share them.
+enum { kTileNone = 0, kTileCluster, kTileGrid };
+static int tile_form(const Handle* h, int level, int per_point) {
+    const Level& lv = h->lev[level];
+    if (!(h->p.solver_precision == 1 && h->fuse_visits && lv.fuse && lv.visit_cfg == 0 && level < h->grids))
+        return kTileNone;
+    if (tile_visit_fits(lv.L, h->p.Nmulti, per_point)) return kTileCluster;
+    return (lv.tile_inbox != nullptr && !h->in_ensemble) ? kTileGrid : kTileNone;
+}
+
 // Would iterate_stream / iterate_stream32 smooth `level` in direction dir as
-// one cluster visit?  (the conditions under which launch_visit_cluster runs)
+// one fused visit?  (the conditions under which launch_visit_cluster runs)
 static bool visit_fuses(Handle* h, int level, int dir) {
     const Level& lv = h->lev[level];
     const bool mixed = (h->p.solver_precision == 1);
     if (!(h->fuse_visits && lv.fuse && level > 1 && level < h->grids && h->p.Nmulti <= 128)) return false;
-    if (!visit_cluster_fits(lv.L, h->p.Nmulti, mixed ? 1 : 0, lv.visit_cfg)) return false;
     const bool pp = (dir != 1 && level == h->ratio_level);
+    if (tile_form(h, level, pp ? 1 : 0) != kTileNone) return true;
+    if (!visit_cluster_fits(lv.L, h->p.Nmulti, mixed ? 1 : 0, lv.visit_cfg)) return false;
     return mixed || !pp || h->ctab_level == level;
 }
 
@@ -1014,7 +1029,10 @@ void iterate_stream32(Handle* h, int level, int dir, int pro = 0, int rst = 0, i
     const int Niter = h->p.Nmulti;
     const bool cheb_pp = (level == h->ratio_level);
     const int pp = (dir != 1 && cheb_pp) ? 1 : 0;
-    if (h->fuse_visits && lv.fuse && level > 1 && Niter <= 128) {
+    // lv.fuse with no explicit shape: the tile smoother (k_tile.cu), the whole visit
+    // in one launch
+    const int tiles = tile_form(h, level, pp);
+    if (h->fuse_visits && lv.fuse && Niter <= 128) {
         double cv[128], tv[128];
         cheb_temps(Niter, dir, tv, cv);
         VisitXfer<float> x;
@@ -1030,8 +1048,19 @@ void iterate_stream32(Handle* h, int level, int dir, int pro = 0, int rst = 0, i
                 x.zn = h->lev[level + 1].L.plane;
             }
         }
-        if (launch_visit_cluster32(h->st, lv, cur_e32(h, level), cv, tv, Niter, pp, h->p.Vbc,
-                                   &h->ds->visit_timeout, &x, h->wait_test ? &h->ds->never_set : nullptr) == 0)
+        const int* tf = h->wait_test ? &h->ds->never_set : nullptr;
+        if (tiles != kTileNone) {
+            float cf[128], tf32[128];
+            for (int n = 0; n < Niter; n++) {
+                cf[n] = (float)cv[n];
+                tf32[n] = (float)tv[n];
+            }
+            if (launch_tile_visit(h->st, lv, tiles == kTileGrid, cur_e32(h, level), cf, tf32, Niter, pp, h->p.Vbc,
+                                  level > 1 ? lv.res32 : nullptr, &h->ds->visit_timeout, &x, tf) == 0)
+                return;
+        }
+        if (level > 1 && launch_visit_cluster32(h->st, lv, cur_e32(h, level), cv, tv, Niter, pp, h->p.Vbc,
+                                                &h->ds->visit_timeout, &x, tf) == 0)
             return;
     }
     if (pro) launch_prolong32(h->st, h->lev[level + 1], lv, cur_e32(h, level + 1), cur_e32(h, level), h->p.Vbc);
@@ -2035,6 +2064,16 @@ tc_status create(Handle* h, const tc_params* in) {
             float** f32[] = {&lv.dts32, &lv.cA32, &lv.cB32, &lv.rhs32, &lv.res32, &lv.e32[0], &lv.e32[1]};
             for (float** q : f32) TRY(dalloc_t(h, q, lp));
         }
+        lv.tile_inbox = nullptr;
+        lv.tile_count = nullptr;
+        if (p.solver_precision == 1 && h->fuse_visits && l < G && !tile_visit_fits(lv.L, p.Nmulti, 0)) {
+            size_t words = 0;
+            const int tiles = tile_grid_tiles(lv.L, p.Nmulti, &words);
+            if (tiles > 0) {
+                TRY(dalloc_t(h, &lv.tile_inbox, words));
+                TRY(dalloc_t(h, &lv.tile_count, (size_t)tiles));
+            }
+        }
         tcs::LevSpacing s;
         tcs::level_spacing(p.aspect, lv.L.a, lv.L.b, s);
         LevConst& c = lv.c;
@@ -2265,6 +2304,19 @@ void drop_step_graphs(Handle* h) {
     }
     h->step_graphs.clear();
     h->epoch++;
+}
+
+// From its first ensemble step on a handle uses no launch that waits for the
+// whole GPU (tile_form): its graphs are captured again without them.
+void enter_ensemble(Handle* h) {
+    if (h->in_ensemble) return;
+    h->in_ensemble = true;
+    CycleGraphs& cg = *h->graphs;
+    if (cg.l1) cudaGraphExecDestroy(cg.l1);
+    if (cg.rest) cudaGraphExecDestroy(cg.rest);
+    if (cg.loop) cudaGraphExecDestroy(cg.loop);
+    cg.l1 = cg.rest = cg.loop = nullptr;
+    drop_step_graphs(h);
 }
 
 // The step can run as one captured graph: every loop of it on the device,
@@ -2834,13 +2886,17 @@ tc_status tc_autotune(tc_handle* H, int32_t* choices) {
         }
         lv.blk = best_blk;
         int best_cfg = -1;  // -1 = unfused
-        if (l > 1 && h->fuse_visits && visit_cluster_fits(lv.L, h->p.Nmulti, mixed ? 1 : 0)) {
+        const bool cluster = l > 1 && visit_cluster_fits(lv.L, h->p.Nmulti, mixed ? 1 : 0);
+        lv.fuse = 1;
+        const bool tile = tile_form(h, l, 0) != kTileNone;
+        if (h->fuse_visits && (cluster || tile)) {
             lv.fuse = 1;
             std::vector<int> cfgs = {0};
-            for (int p : {1, 2})
-                for (int c : {1, 2, 4, 8, 16}) cfgs.push_back(100 * p + c);
+            if (l > 1)
+                for (int p : {1, 2})
+                    for (int c : {1, 2, 4, 8, 16}) cfgs.push_back(100 * p + c);
             for (int cfg : cfgs) {
-                if (!visit_cluster_fits(lv.L, h->p.Nmulti, mixed ? 1 : 0, cfg)) continue;
+                if (!(cfg == 0 && tile) && !visit_cluster_fits(lv.L, h->p.Nmulti, mixed ? 1 : 0, cfg)) continue;
                 lv.visit_cfg = cfg;
                 double ms = 0;
                 TRY(time_visits(&ms));
@@ -2909,6 +2965,7 @@ tc_status tc_ensemble_step(tc_handle* const* hs, int32_t n, int32_t nthreads, tc
     if (!hs || n < 1 || nthreads < 1) return TC_ERR_ARG;
     for (int i = 0; i < n; i++)
         if (!hs[i]) return TC_ERR_ARG;
+    for (int i = 0; i < n; i++) enter_ensemble(&hs[i]->h);
     std::atomic<int> next{0};
     std::vector<tc_status> st((size_t)n, TC_OK);
     auto work = [&]() {
@@ -2970,6 +3027,7 @@ tc_status tc_ensemble_run(tc_ensemble* e, tc_handle* const* hs, int32_t n, tc_st
     bool ready = !e->failed;
     for (int i = 0; i < n; i++) {
         if (!hs[i]) return TC_ERR_ARG;
+        enter_ensemble(&hs[i]->h);
         ready = ready && step_graph_ready(&hs[i]->h, false) && hs[i]->h.device == e->device;
     }
     tc_ensemble::Entry* en = nullptr;

@@ -184,6 +184,10 @@ struct Level {
     int sweep_bx, sweep_by;
     int fuse;       // 1 = one cluster launch per visit when the level fits, 0 = one launch per sweep
     int visit_cfg;  // shape of the fused visit: 0 = default, else 100*points per strip + CTAs
+    // exchange of a visit over the whole grid (k_tile.cu): the tiles' inboxes and
+    // their exchange counts (null: the level does not use it)
+    unsigned long long* tile_inbox;
+    unsigned* tile_count;
     int blk;        // when not fused: 0 = one k_sweep / k_sweep32 launch per sweep, n = n sweeps per k_sweep_blk launch
     MetricFold mfold;  // stretched grids: the tap weights of the computational derivatives
 };
@@ -259,6 +263,18 @@ int launch_visit_cluster(cudaStream_t s, const Level& lv, double* S, const doubl
 int launch_visit_cluster32(cudaStream_t s, const Level& lv, float* S, const double* cvals, const double* tvals,
                            int nsweeps, int per_point, int Vbc, int* timeout_flag,
                            const VisitXfer<float>* x = nullptr, const int* test_flag = nullptr);
+
+// (k_tile.cu) FP32 smoother visits on register patches, a whole visit in one
+// launch: one cluster (grid = false), or one tile per SM of a cooperative
+// launch (grid = true, for levels with tile_inbox).  c, temp: the sweeps'
+// factors rounded to float; res: the residual's plane or null; returns 0 =
+// launched, 1 = the level does not fit, 2 = launch error.  tile_grid_tiles:
+// tiles and inbox words of a level's visits over the grid (0: none).
+bool tile_visit_fits(const Lay& L, int nsweeps, int per_point);
+int tile_grid_tiles(const Lay& L, int nsweeps, size_t* words);
+int launch_tile_visit(cudaStream_t s, const Level& lv, bool grid, float* S, const float* c, const float* temp,
+                      int nsweeps, int per_point, int Vbc, float* res, int* timeout_flag,
+                      const VisitXfer<float>* x = nullptr, const int* test_flag = nullptr);
 
 // (k_subcycle.cu) the bottom of the W-cycle (smoothing of level S = grids-1
 // and the coarsest solves between a restriction into S and the prolongation
