@@ -241,6 +241,36 @@ static unsigned conv_grid(int ntiles) {
 
 using namespace nn;
 
+int nn_sm_count() {
+    static int nsm = 0;
+    if (nsm == 0) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+        if (nsm <= 0) nsm = 1;
+    }
+    return nsm;
+}
+
+// map of an NHWC BF16 tensor [nb][H][W][ctot] with boxes {c, bx, by, 1}; swizzle:
+// 0 or the bytes of a box row (32, 64 or 128)
+bool nn_tensor_map(CUtensorMap* map, const __nv_bfloat16* x, int nb, int H, int W, int ctot, int c, int bx, int by,
+                   int swizzle) {
+    auto enc = encode_fn();
+    if (!enc) return false;
+    cuuint64_t dims[4] = {(cuuint64_t)ctot, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)nb};
+    cuuint64_t strides[3] = {(cuuint64_t)ctot * 2, (cuuint64_t)W * ctot * 2, (cuuint64_t)H * W * ctot * 2};
+    cuuint32_t box[4] = {(cuuint32_t)c, (cuuint32_t)bx, (cuuint32_t)by, 1};
+    cuuint32_t es[4] = {1, 1, 1, 1};
+    const CUtensorMapSwizzle sw = swizzle == 128  ? CU_TENSOR_MAP_SWIZZLE_128B
+                                  : swizzle == 64 ? CU_TENSOR_MAP_SWIZZLE_64B
+                                  : swizzle == 32 ? CU_TENSOR_MAP_SWIZZLE_32B
+                                                  : CU_TENSOR_MAP_SWIZZLE_NONE;
+    return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, (void*)x, dims, strides, box, es,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 // x: [nb][H][W][cin_tot] BF16; computes channels [0, N) of the GEMM and stores
 // the first cout_store of them at out[..][cout_off + c] of an output tensor
 // with cout_tot channels.
@@ -253,17 +283,8 @@ int conv3x3_launch(cudaStream_t s, const __nv_bfloat16* x, int nb, int H, int W,
     if (128 % bx) return 1;
     const int by = 128 / bx;
     if (W % bx || H % by) return 1;
-    auto enc = encode_fn();
-    if (!enc) return 2;
     CUtensorMap map;
-    cuuint64_t dims[4] = {(cuuint64_t)cin_tot, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)nb};
-    cuuint64_t strides[3] = {(cuuint64_t)cin_tot * 2, (cuuint64_t)W * cin_tot * 2, (cuuint64_t)H * W * cin_tot * 2};
-    cuuint32_t box[4] = {8, (cuuint32_t)bx, (cuuint32_t)by, 1};
-    cuuint32_t es[4] = {1, 1, 1, 1};
-    if (enc(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, (void*)x, dims, strides, box, es,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-        return 3;
+    if (!nn_tensor_map(&map, x, nb, H, W, cin_tot, 8, bx, by, 0)) return 3;
     ConvArgs a;
     a.nb = nb; a.H = H; a.W = W; a.bx = bx; a.by = by;
     a.cin = cin; a.cin_off = cin_off; a.kc = conv_kc(cin);
