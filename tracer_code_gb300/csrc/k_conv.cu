@@ -59,7 +59,9 @@ __device__ __forceinline__ void mbar_arrive1(uint64_t* b) {
 
 template <int N>
 __global__ void __launch_bounds__(192, 1) k_conv3x3p(const __grid_constant__ CUtensorMap xmap, ConvArgs a) {
-    extern __shared__ __align__(1024) unsigned char smem[];
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    unsigned char* smem =  // swizzled boxes start on 1024 bytes
+        reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     __shared__ __align__(8) uint64_t full[kStages], empty[kStages], accf[2], acce[2];
     __shared__ uint32_t tmem_base;
     __shared__ int bad;
@@ -127,8 +129,7 @@ __global__ void __launch_bounds__(192, 1) k_conv3x3p(const __grid_constant__ CUt
                     unsigned char* As = smem + (size_t)s * st_bytes;
                     unsigned char* Bs = As + a_bytes;
                     mbar_expect_tx(&full[s], (uint32_t)st_bytes);
-                    for (int q = 0; q < a.kc / 8; q++)
-                        tma_load4(As + q * 2048, &xmap, a.cin_off + ch * a.kc + q * 8, x0 + dx, y0 + dy, n, &full[s]);
+                    tma_load4(As, &xmap, a.cin_off + ch * a.kc, x0 + dx, y0 + dy, n, &full[s]);
                     bulk_load(Bs, a.wpack + (size_t)i * N * a.kc, (uint32_t)b_bytes, &full[s]);
                 }
             }
@@ -148,7 +149,7 @@ __global__ void __launch_bounds__(192, 1) k_conv3x3p(const __grid_constant__ CUt
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint32_t As = saddr(smem + (size_t)s * st_bytes), Bs = As + a_bytes;
                     for (int kk = 0; kk < a.kc / 16; kk++) {
-                        const uint64_t ad = smem_desc(As + kk * 2 * 2048, 2048, 128);
+                        const uint64_t ad = smem_desc_swizzled(As + kk * 32, 16, 16 * a.kc, 2 * a.kc);
                         const uint64_t bd = smem_desc(Bs + kk * 2 * N * 16, N * 16, 128);
                         umma_bf16(acc, ad, bd, idesc, (i > 0 || kk > 0) ? 1u : 0u);
                     }
@@ -213,7 +214,7 @@ template <int N>
 static bool conv_attr() {
     static bool done = false;
     if (!done) {
-        const int smax = kStages * (64 * 256 + N * 64 * 2);
+        const int smax = kStages * (64 * 256 + N * 64 * 2) + 1024;
         if (cudaFuncSetAttribute(k_conv3x3p<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, smax) != cudaSuccess)
             return false;
         done = true;
@@ -284,13 +285,13 @@ int conv3x3_launch(cudaStream_t s, const __nv_bfloat16* x, int nb, int H, int W,
     const int by = 128 / bx;
     if (W % bx || H % by) return 1;
     CUtensorMap map;
-    if (!nn_tensor_map(&map, x, nb, H, W, cin_tot, 8, bx, by, 0)) return 3;
+    if (!nn_tensor_map(&map, x, nb, H, W, cin_tot, conv_kc(cin), bx, by, 2 * conv_kc(cin))) return 3;
     ConvArgs a;
     a.nb = nb; a.H = H; a.W = W; a.bx = bx; a.by = by;
     a.cin = cin; a.cin_off = cin_off; a.kc = conv_kc(cin);
     a.cout_store = cout_store; a.cout_off = cout_off; a.cout_tot = cout_tot;
     a.relu = relu; a.wpack = wpack; a.bias = bias; a.out = out; a.fail = fail; a.test_flag = test_flag;
-    const int smem = kStages * (a.kc * 256 + N * a.kc * 2);
+    const int smem = kStages * (a.kc * 256 + N * a.kc * 2) + 1024;
     const int ntiles = nb * (H / by) * (W / bx);
     switch (N) {
         case 32: if (!conv_attr<32>()) return 4; k_conv3x3p<32><<<conv_grid<32>(ntiles), 192, smem, s>>>(map, a); break;

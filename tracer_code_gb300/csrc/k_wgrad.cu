@@ -44,11 +44,6 @@ struct WgradArgs {
     const int* test_flag;       // timeout-path test, as ConvArgs
 };
 
-__device__ __forceinline__ uint64_t desc_mn(uint32_t addr, uint32_t lbo, uint32_t sbo, int row_bytes) {
-    const uint64_t swizzle = row_bytes == 128 ? 2 : (row_bytes == 64 ? 4 : 6);
-    return smem_desc(addr, lbo, sbo) | swizzle << 61;
-}
-
 // 16 accumulator columns of this warp's lanes (the caller waits for the loads)
 __device__ __forceinline__ void tmem_ld16(uint32_t addr, uint32_t (&r)[16]) {
     asm volatile(
@@ -149,8 +144,8 @@ __global__ void __launch_bounds__(320, 1) k_wgrad(const __grid_constant__ CUtens
                 for (int d = 0; d < 3; d++)
                     for (int k = 0; k < kWgTile / 16; k++) {
                         // 128 output channels: the boxes in turn, or one box again and again
-                        const uint64_t ad = desc_mn(zs + k * 16 * zrow, a.cout == 128 ? zbox : 0, 8 * zrow, zrow);
-                        const uint64_t bd = desc_mn(xs + d * xtile + k * 16 * xrow, xbox, 8 * xrow, xrow);
+                        const uint64_t ad = smem_desc_swizzled(zs + k * 16 * zrow, a.cout == 128 ? zbox : 0, 8 * zrow, zrow);
+                        const uint64_t bd = smem_desc_swizzled(xs + d * xtile + k * 16 * xrow, xbox, 8 * xrow, xrow);
                         umma_bf16(tmem + (uint32_t)(b * NCOL + d * CC), ad, bd, idesc, k > 0 ? 1u : 0u);
                     }
                 umma_commit(&empty[s]);

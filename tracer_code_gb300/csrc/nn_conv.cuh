@@ -1,14 +1,16 @@
 // nn_conv.cuh -- Blackwell primitives of the learned initial guess: tensor
 // maps, mbarriers, TMA and bulk copies, tcgen05 MMA/TMEM access.
 //
-// Operand layout for tcgen05.mma kind::f16 (BF16 in, FP32 accumulate in
-// TMEM) is the no-swizzle K-major core-matrix layout: a core matrix is 8
-// rows x 16 bytes (8 BF16 along K) stored contiguously; core matrices
-// adjacent along K are LBO bytes apart, along M/N SBO bytes apart.  A TMA box
-// of {8 channels, 128 pixels} of an NHWC BF16 tensor lands in shared memory
-// as exactly 16 such core matrices stacked along M (SBO = 128 B), so the
-// activation operand of an implicit-GEMM convolution is one box per 8 input
-// channels, boxes 2 KB apart (LBO = 2048 B).
+// Operand layouts for tcgen05.mma kind::f16 (BF16 in, FP32 accumulate in TMEM).
+// Weights: the no-swizzle K-major core-matrix layout; a core matrix is 8 rows x 16
+// bytes (8 BF16 along K) stored contiguously, core matrices adjacent along K are
+// LBO bytes apart, along M/N SBO bytes apart.  Activations: a TMA box of {c
+// channels, pixels} of an NHWC BF16 tensor with the 2c-byte swizzle (c = 16, 32 or
+// 64), read K-major by the convolutions (rows are pixels, K the channels; K
+// advances by 32 bytes inside the swizzle) and MN-major by the weight gradients
+// (rows are channels, K the pixels).  One box of 2c-byte rows replaced c / 8 boxes
+// of 16-byte rows, whose rows the TMA unit took one at a time: it bound the
+// convolutions.
 #pragma once
 
 #include <cuda.h>
@@ -66,6 +68,12 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint3
     d |= (uint64_t)((sbo >> 4) & 0x3FFF) << 32;
     d |= (uint64_t)1 << 46;  // descriptor version; base offset 0, no swizzle
     return d;
+}
+// the same for operands that TMA stored with a 32, 64 or 128-byte swizzle
+// (bytes: that many; K-major: sbo = 8 rows of it, MN-major: see k_wgrad.cu)
+__device__ __forceinline__ uint64_t smem_desc_swizzled(uint32_t addr, uint32_t lbo, uint32_t sbo, int bytes) {
+    const uint64_t mode = bytes == 128 ? 2 : (bytes == 64 ? 4 : 6);
+    return smem_desc(addr, lbo, sbo) | mode << 61;
 }
 // kind::f16 instruction descriptor: D F32, A/B BF16, both K-major, M x N
 __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
