@@ -290,6 +290,8 @@ __global__ void k_dt(Phys P, DevScalars* ds, double courant, double dt_manual) {
         dt = dt_manual;
     }
     ds->dt = courant * dt;
+    ds->dt_half = 0.5 * ds->dt;
+    ds->dt_sixth = ds->dt / 6.0;
 }
 void launch_stability(cudaStream_t s, const Lay& L, const Phys& P, const double* conduct, const double* conduct_r,
                       const double* conduct_s, const double* u, const double* w, double courant, double dt_manual,

@@ -62,46 +62,64 @@ __device__ __forceinline__ int quot_nint(double x, double h, double hinv) {
 // DER(1,i,k) and a 3-point s-stencil; int() truncates, as in Fortran.  The
 // position part (cell, offsets, branch) is shared by every field
 // interpolated at the same point.
+//
+// What bounds the tracer stages is the FP64 pipe (2 lanes a cycle per SM), so the
+// arithmetic is written with as few FP64 operations as give the same bits: bounds
+// and branches compare the doubles' bits as integers (a <= b for b > 0 and any a
+// that is no NaN), i*dr comes from a table of the same products, only the three
+// rows that the branch uses are formed, and the division by ds is a product with
+// its reciprocal where that is exact, else quot_round.  About 30 FP64
+// operations a tracer and stage where the expressions as written take about 75.
+__device__ __forceinline__ long long dbits(double x) { return __double_as_longlong(x); }
+
+// 0 < x < b (b > 0) and, for outside, x <= 0 or x >= b; both false for a NaN
+__device__ __forceinline__ bool inside(double x, double b) {
+    return (unsigned long long)dbits(x) - 1ull < (unsigned long long)dbits(b) - 1ull;
+}
+__device__ __forceinline__ bool outside(double x, double b) {
+    return !inside(x, b) && ((unsigned long long)dbits(x) & ~(1ull << 63)) <= (0x7ffull << 52);
+}
+
+// RN(x / h) for h > 0 from hinv = RN(1/h): two Newton corrections of x * hinv with
+// exact remainders; by Markstein's theorem (P. W. Markstein, Computation of
+// elementary functions on the IBM RISC System/6000 processor, IBM J. Res. Dev. 34,
+// 1990) the second, applied to a quotient within one ulp, rounds correctly.
+// Exponents near the ends of the range, where a remainder could underflow, and
+// zero are divided.
+__device__ __forceinline__ double quot_round(double x, double h, double hinv) {
+    const unsigned ex = (unsigned)(dbits(x) >> 52) & 0x7ffu;
+    if (ex - 200u > 1600u) return x / h;
+    double q = x * hinv;
+    q = fma(fma(-q, h, x), hinv, q);
+    return fma(fma(-q, h, x), hinv, q);
+}
+
 struct TaylorPos {
-    int i, k;      // column of the r-Taylor step (i or i+1) and the s cell
-    double a1;     // r offset from that column
-    double hs;     // s offset (from k, or ds minus it on the upper branch)
-    bool slo;      // hs <= ds/2
+    int i, k;   // column of the r-Taylor step (i or i+1) and row of the s-Taylor step (k or k+1)
+    double a1;  // r offset from that column
+    double b1;  // s offset from that row
 };
 __device__ __forceinline__ TaylorPos taylor_pos(const Phys& P, double r, double s) {
     TaylorPos t;
-    const int i = quot_trunc(r, P.dr, P.rdr);
-    t.k = quot_trunc(s, P.ds, P.rds);
-    double hr = r - (double)i * P.dr;
-    if (hr <= P.dro2) {
-        t.i = i;
-        t.a1 = hr / 1.0;
-    } else {
-        hr = P.dr - hr;
-        t.i = i + 1;
-        t.a1 = (-hr) / 1.0;
-    }
-    const double hs = s - (double)t.k * P.ds;
-    t.slo = hs <= P.dso2;
-    t.hs = t.slo ? hs : P.ds - hs;
+    const int i = quot_trunc(r, P.dr, P.rdr), k = quot_trunc(s, P.ds, P.rds);
+    const double hr = r - __ldg(P.xn + i), hs = s - __ldg(P.zn + k);
+    const bool rlo = dbits(hr) <= dbits(P.dro2), slo = dbits(hs) <= dbits(P.dso2);
+    t.i = rlo ? i : i + 1;
+    t.a1 = rlo ? hr : -(P.dr - hr);
+    t.k = slo ? k : k + 1;
+    t.b1 = slo ? hs : -(P.ds - hs);
     return t;
 }
 __device__ __forceinline__ double taylor_eval(const Lay& L, const Phys& P, const double* __restrict__ f,
                                               const double* __restrict__ der, const TaylorPos& t) {
-    const int i = t.i, k = t.k;
-    const double fR0 = __ldg(f + IX(L, i, k - 1)) + __ldg(der + IX(L, i, k - 1)) * t.a1;
-    const double fR1 = __ldg(f + IX(L, i, k)) + __ldg(der + IX(L, i, k)) * t.a1;
-    const double fR2 = __ldg(f + IX(L, i, k + 1)) + __ldg(der + IX(L, i, k + 1)) * t.a1;
-    const double fR3 = __ldg(f + IX(L, i, k + 2)) + __ldg(der + IX(L, i, k + 2)) * t.a1;
-    double fin;
-    if (t.slo) {
-        double DERs = (-0.5 * fR0 + 0.5 * fR2) / P.ds;
-        fin = fR1 + DERs * (t.hs / 1.0);
-    } else {
-        double DERs = (-0.5 * fR1 + 0.5 * fR3) / P.ds;
-        fin = fR2 + DERs * ((-t.hs) / 1.0);
-    }
-    return fin;
+    const size_t x = IX(L, t.i, t.k), ld = (size_t)L.ld;
+    const double fl = __ldg(f + x - ld) + __ldg(der + x - ld) * t.a1;
+    const double fc = __ldg(f + x) + __ldg(der + x) * t.a1;
+    const double fu = __ldg(f + x + ld) + __ldg(der + x + ld) * t.a1;
+    // (-0.5 fl + 0.5 fu) / ds: the halving is exact, so it may follow the difference
+    const double d = fu - fl;
+    const double DERs = P.ds_pow2 ? d * (0.5 * P.rds) : quot_round(0.5 * d, P.ds, P.rds);
+    return fc + DERs * t.b1;
 }
 __device__ __forceinline__ double interp_taylor(const Lay& L, const Phys& P, const double* __restrict__ f,
                                                 const double* __restrict__ der, double r, double s) {
@@ -130,11 +148,11 @@ __global__ void k_tracer_stage(Lay L, Phys P, int torder, int stage, int64_t ntr
                                const double* __restrict__ dw, const DevScalars* __restrict__ ds, TracerT tT) {
     int64_t id = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (id >= ntr) return;
-    const double dt = ds->dt;
+    const double dt = ds->dt, dt2 = ds->dt_half, dto6 = ds->dt_sixth;
     const double r = rin[id], s = sin[id];
     // positions outside the box were already reported by the histogram that
     // precedes every stage (the reference stops there); never index with them
-    if (!(r > 0.0 && r < P.aspect && s > 0.0 && s < 1.0)) return;
+    if (!inside(r, P.aspect) || !inside(s, 1.0)) return;
     const TaylorPos tp = taylor_pos(P, r, s);
     double tr = taylor_eval(L, P, u, du, tp);
     double ts = taylor_eval(L, P, w, dw, tp);
@@ -142,55 +160,52 @@ __global__ void k_tracer_stage(Lay L, Phys P, int torder, int stage, int64_t ntr
     // interpolated the same way (interpolate_xr / interpolate_zs,
     // composition.f90:938-998; energy.f90:195-203)
     if (P.M.gx) tr = tr / (mt(P.M.xr, tp.i) + mt(P.M.dxr, tp.i) * tp.a1);
-    if (P.M.gz)
-        ts = ts / (tp.slo ? mt(P.M.zs, tp.k) + mt(P.M.dzs, tp.k) * (tp.hs / 1.0)
-                          : mt(P.M.zs, tp.k + 1) + mt(P.M.dzs, tp.k + 1) * ((-tp.hs) / 1.0));
+    if (P.M.gz) ts = ts / (mt(P.M.zs, tp.k) + mt(P.M.dzs, tp.k) * tp.b1);
     if (tT.f) {
         // energy.f90:213-223, 292-310, 371-375, 437-440
         const double te = taylor_eval(L, P, tT.f, tT.der, tp);
         if (stage == 1) {
             tT.acc[id] = te;
-            tT.out[id] = tT.T0[id] + ((torder == 2) ? dt : 0.5 * dt) * te;
+            tT.out[id] = tT.T0[id] + ((torder == 2) ? dt : dt2) * te;
         } else if (stage == 2) {
             if (torder == 2) {
                 const double a = tT.acc[id] + te;
-                tT.acc[id] = tT.T0[id] + (0.5 * dt) * a;
+                tT.acc[id] = tT.T0[id] + dt2 * a;
             } else {
-                tT.acc[id] = tT.acc[id] + 2.0 * te;
-                tT.out[id] = tT.T0[id] + (0.5 * dt) * te;
+                tT.acc[id] = fma(2.0, te, tT.acc[id]);
+                tT.out[id] = tT.T0[id] + dt2 * te;
             }
         } else if (stage == 3) {
-            tT.acc[id] = tT.acc[id] + 2.0 * te;
+            tT.acc[id] = fma(2.0, te, tT.acc[id]);
             tT.out[id] = tT.T0[id] + dt * te;
         } else {
-            tT.acc[id] = tT.T0[id] + (dt / 6.0) * (tT.acc[id] + te);
+            tT.acc[id] = tT.T0[id] + dto6 * (tT.acc[id] + te);
         }
     }
     if (stage == 1) {
-        const double dtstage = (torder == 2) ? dt : 0.5 * dt;
+        const double dtstage = (torder == 2) ? dt : dt2;
         racc[id] = tr;
         sacc[id] = ts;
         rout[id] = r + dtstage * tr;
         sout[id] = s + dtstage * ts;
     } else if (stage == 2) {
-        const double dtstage = 0.5 * dt;
+        const double dtstage = dt2;
         if (torder == 2) {
             double a = racc[id] + tr, b = sacc[id] + ts;
             racc[id] = r0[id] + dtstage * a;
             sacc[id] = s0[id] + dtstage * b;
         } else {
-            racc[id] = racc[id] + 2.0 * tr;
-            sacc[id] = sacc[id] + 2.0 * ts;
+            racc[id] = fma(2.0, tr, racc[id]);  // 2 tr is exact: one rounding either way
+            sacc[id] = fma(2.0, ts, sacc[id]);
             rout[id] = r0[id] + dtstage * tr;
             sout[id] = s0[id] + dtstage * ts;
         }
     } else if (stage == 3) {
-        racc[id] = racc[id] + 2.0 * tr;
+        racc[id] = fma(2.0, tr, racc[id]);
         rout[id] = r0[id] + dt * tr;
-        sacc[id] = sacc[id] + 2.0 * ts;
+        sacc[id] = fma(2.0, ts, sacc[id]);
         sout[id] = s0[id] + dt * ts;
     } else {
-        const double dto6 = dt / 6.0;
         racc[id] = r0[id] + dto6 * (racc[id] + tr);
         sacc[id] = s0[id] + dto6 * (sacc[id] + ts);
     }
@@ -273,7 +288,7 @@ __global__ void k_histogram(Lay L, Phys P, int64_t ntr, const double* __restrict
     int key = -1;
     if (id < ntr) {
         const double r = rr[id], s = ss[id];
-        if (r <= 0.0 || r >= P.aspect || s <= 0.0 || s >= 1.0) {
+        if (outside(r, P.aspect) || outside(s, 1.0)) {
             atomicOr(flag, 1);
         } else {
             const int i = quot_nint(r, P.dr, P.rdr);

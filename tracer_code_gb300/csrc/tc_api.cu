@@ -1919,6 +1919,20 @@ tc_status create(Handle* h, const tc_params* in) {
     h->fuse_visits = (std::getenv("TC_NO_FUSED_VISITS") == nullptr) && visit_cluster_setup() > 0;
     // ---- allocations ----
     h->L1 = make_lay(nx, nz);
+    {
+        std::vector<double> xn((size_t)nx + 2), zn((size_t)nz + 2);
+        for (int i = 0; i < nx + 2; i++) xn[(size_t)i] = (double)i * P.dr;
+        for (int k = 0; k < nz + 2; k++) zn[(size_t)k] = (double)k * P.ds;
+        double *dx = nullptr, *dz = nullptr;
+        TRY(dalloc_t(h, &dx, xn.size()));
+        TRY(dalloc_t(h, &dz, zn.size()));
+        CK(cudaMemcpy(dx, xn.data(), sizeof(double) * xn.size(), cudaMemcpyHostToDevice));
+        CK(cudaMemcpy(dz, zn.data(), sizeof(double) * zn.size(), cudaMemcpyHostToDevice));
+        P.xn = dx;
+        P.zn = dz;
+        int e = 0;
+        P.ds_pow2 = (std::frexp(P.ds, &e) == 0.5) ? 1 : 0;
+    }
     const size_t pl = h->L1.plane;
     double** fine[] = {&h->T, &h->T0, &h->T1, &h->T2, &h->SF, &h->Tvis, &h->Tvis2, &h->Tbuoy, &h->u, &h->w,
                        &h->du, &h->dw, &h->conduct, &h->conduct_r, &h->conduct_s, &h->dts, &h->strain};

@@ -97,6 +97,7 @@ struct DevScalars {
     double res_mag[TC_MAXLEV + 1];
     double res_ref;
     double dt;
+    double dt_half, dt_sixth;  // 0.5 dt, dt / 6 (tracer stages)
     double eA_max, eD_max;
     double integ[32];
     double strain_max;
@@ -197,6 +198,8 @@ struct Phys {
     int nx, nz, ntype, comp, ivis, Tbot, Vbc, torder, tracer;
     double aspect, dr, ds, dr2, ds2, dro2, dso2;
     double rdr, rds;             // 1/dr, 1/ds rounded (tracer cell indices: quot_trunc, quot_nint)
+    const double *xn, *zn;       // i * dr for i = 0..nx+1, k * ds for k = 0..nz+1 (tracer offsets)
+    int ds_pow2;                 // ds is a power of two: x / ds = x * rds exactly
     double RaT, RaC[TC_MAX_TYPES], lnvisT, lnvisP, lnvisC[TC_MAX_TYPES], visT2, H, Htype[TC_MAX_TYPES];
     double lncf[TC_MAX_TYPES];   // log(1/conduct_factor)
     double courantT, courantC;
