@@ -1,0 +1,33 @@
+"""The banded LU of the coarsest matrix at the edges of its kernels.
+
+Solves whose coarsest grids have the narrowest bands, bands at both sides of one
+lane's second row (kl = 32), of the one-block kernel's limit (kl = 63) and beyond:
+cycle counts equal the oracle's and the stream function agrees within the bound of
+test_gpu_parity.py (1e-9 of its largest value).
+"""
+import numpy as np
+import pytest
+
+from oracle.pyoracle import Oracle
+from tracer_code_gb300 import Simulation
+from tests.cases import case_1024_like, fresh_state
+
+pytestmark = pytest.mark.gpu
+
+
+# kl = 2 nz / 2^(grids-1) + 2
+@pytest.mark.parametrize("nx,nz,grids,kl", [(64, 16, 3, 10), (96, 24, 3, 14), (48, 30, 2, 32), (48, 32, 2, 34),
+                                            (40, 60, 2, 62), (40, 62, 2, 64)])
+def test_solve_equals_oracle(gpu_lib, nx, nz, grids, kl):
+    p = case_1024_like(nx=nx, nz=nz, tpc=4, grids=grids)
+    p.aspect, p.max_cycles = nx / nz, 200
+    st = fresh_state(p, seed=nx)
+    g, o = Simulation(p), Oracle(p)
+    for s in (g, o):
+        s.upload(st)
+        s.compute_velocities()
+    assert (g.info.kl, g.info.ku, g.info.grids) == (kl, kl, grids)
+    assert g.multigrid() == o.multigrid()
+    a, b = g.download()["SF"], o.download()["SF"]
+    assert np.abs(b).max() > 0 and np.abs(a - b).max() <= 1e-9 * np.abs(b).max()
+    g.close()

@@ -541,16 +541,195 @@ void launch_coarse_build(cudaStream_t s, const Level& lv, double* band, double* 
     k_coarse_build<<<(n + 127) / 128, 128, 0, s>>>(lv.L, lv.coef, band, rowb, n, kl, ku, Vbc); tc_note_launch();
 }
 
-// dgbtf2 on one CTA.  The band lives in shared memory when it fits.
-__global__ void k_coarse_lu(double* __restrict__ ABg, int* __restrict__ ipiv, int n, int kl, int ku, int in_smem,
-                            int* info_out) {
+// dgbtf2 on one CTA, one block barrier per column.  The columns in reach of a step
+// (j..j+kl+ku) and the next few sit in a ring of column slots in shared memory.
+// At step j warp 0 already works on column j+1: it applies step j to it,
+// searches its pivot, swaps and scales, while the trailing warps apply step j to
+// the columns behind it, a few whole columns per warp and pass (so that a row
+// interchange needs no barrier), and the last warp writes column j back and loads
+// the column that enters the ring.  Every element sees dgbtf2's operations in
+// dgbtf2's order.
+//
+// What bounds it: the chain of warp 0, 1 us a column (update, search, reciprocal,
+// scaling, barrier: FP64 latencies), and for kl > 32 the FP64 pipe of one SM.
+// Against six barriers a column and the trailing update as one flat loop: 651 ->
+// 308 us at n = 297, kl = 20; 2044 -> 895 us at n = 1000, kl = 8; 3164 -> 2360 us at
+// n = 400, kl = 63.
+#define LU1_THREADS 512
+#define LU1_AHEAD 4   // columns loaded ahead of the window
+#define LU1_MAXKL 63  // two rows per lane of warp 0
+#define LU1_ROWS 6    // band rows per lane of the loading warp (2 kl + ku + 1 <= 192)
+__global__ void __launch_bounds__(LU1_THREADS) k_coarse_lu(double* __restrict__ ABg, int* __restrict__ ipiv, int n,
+                                                           int kl, int ku, int* info_out) {
     extern __shared__ double sm[];
+    const int ldab = 2 * kl + ku + 1, KV = ku + kl, C = KV + 1 + LU1_AHEAD;
+    __shared__ double mult[2][LU1_MAXKL + 1];
+    __shared__ int sCode[2];  // pivot row offset * 2 + (pivot != 0), per step parity
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr int NW = LU1_THREADS / 32;
+    // column cl (1-based) as an array of band rows 1..ldab; at = j % C
+    int at_j = 0;
+    auto col = [&](int cl) { return sm + (size_t)(cl % C) * ldab - 1; };
+    auto col_after = [&](int c) {  // column j + c, 0 <= c <= KV
+        int q = at_j + c;
+        if (q >= C) q -= C;
+        return sm + q * ldab - 1;
+    };
+    auto nonzero = [](double x) { return (unsigned long long)(__double_as_longlong(x) << 1) != 0ull; };
+    // loads column cl with dgbtf2's zeroed fill-in rows
+    auto load_col = [&](int cl, int t0, int nt) {
+        double* d = col(cl);
+        const double* g = ABg + (size_t)(cl - 1) * ldab - 1;
+        const int z0 = (cl > KV) ? 1 : KV - cl + 2;  // rows z0..kl of the columns ku+2.. are fill-in
+        for (int t = 1 + t0; t <= ldab; t += nt) d[t] = (cl >= ku + 2 && t >= z0 && t <= kl) ? 0.0 : g[t];
+    };
+    for (int cl = 1 + warp; cl <= min(n, KV + LU1_AHEAD); cl += NW) load_col(cl, lane, 32);
+    double pf[LU1_ROWS];  // the loader's next column, loaded a step before it is stored
+    int pf_col = 0;
+    __syncthreads();
+    int JU = 1, info = 0;
+    const int G = max(1, 64 / kl);  // columns of a trailing warp's pass
+    int code = 0;
+    for (int j = 0; j <= n; j++) {
+        // step j (j = 0: none) is prepared: pivot code, multipliers, column j
+        const int KM = min(kl, n - j), JP = code >> 1;
+        const bool nz = j > 0 && (code & 1) != 0;
+        const double* mj = mult[j & 1];
+        if (j > 0) {
+            if (nz) JU = max(JU, min(j + ku + JP - 1, n));
+            else if (info == 0) info = j;
+        }
+        if (warp == 0) {
+            if (j + 1 <= n) {
+                // column j+1: rows t = 0..KM1 below and on its diagonal, two per lane
+                const int KM1 = min(kl, n - j - 1);
+                double* a = col_after(1) + KV + 1;
+                double v[2];
+#pragma unroll
+                for (int u = 0; u < 2; u++) {
+                    const int t = lane + 32 * u;
+                    v[u] = t <= KM1 ? a[t] : 0.0;
+                }
+                if (nz && j + 1 <= JU) {
+                    const double oldtop = a[-1], top = a[JP - 2];
+                    const double temp = -top;
+#pragma unroll
+                    for (int u = 0; u < 2; u++) {
+                        const int t = lane + 32 * u;  // row t + 1 of step j
+                        if (t + 1 == JP - 1) v[u] = oldtop;
+                        if (t < KM && nonzero(temp)) v[u] = v[u] + mj[t + 1] * temp;
+                    }
+                    __syncwarp();
+                    if (lane == 0 && JP != 1) a[-1] = top;
+                }
+                // idamax: the first row of the largest |value| (as integers; a NaN is never the largest)
+                unsigned long long best = 0;
+                int bi = 1 << 30;
+#pragma unroll
+                for (int u = 0; u < 2; u++) {
+                    const int t = lane + 32 * u;
+                    unsigned long long k = (unsigned long long)__double_as_longlong(v[u]) & ~(1ull << 63);
+                    k = k > (0x7ffull << 52) ? 0 : k + 1;
+                    if (t <= KM1 && k > best) { best = k; bi = t; }
+                }
+                const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)(best >> 32));
+                const unsigned lo = __reduce_max_sync(0xffffffffu, (unsigned)(best >> 32) == hi ? (unsigned)best : 0u);
+                const bool is = (unsigned)(best >> 32) == hi && (unsigned)best == lo;
+                bi = (int)__reduce_min_sync(0xffffffffu, is ? (unsigned)bi : 1u << 30);
+                if (bi > KM1) bi = 0;
+                const double piv = __shfl_sync(0xffffffffu, bi < 32 ? v[0] : v[1], bi & 31);
+                const double first = __shfl_sync(0xffffffffu, v[0], 0);
+                const int nzp = nonzero(piv) ? 1 : 0;
+                if (nzp) {
+                    const double rcp = 1.0 / piv;
+#pragma unroll
+                    for (int u = 0; u < 2; u++) {
+                        const int t = lane + 32 * u;
+                        if (t == bi) v[u] = first;
+                        if (t == 0) v[u] = piv;
+                        else v[u] = rcp * v[u];
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < 2; u++) {
+                    const int t = lane + 32 * u;
+                    if (t <= KM1) {
+                        a[t] = v[u];
+                        mult[(j + 1) & 1][t] = v[u];
+                    }
+                }
+                if (lane == 0) {
+                    sCode[(j + 1) & 1] = (bi + 1) * 2 + nzp;
+                    ipiv[j] = bi + j + 1;
+                }
+            }
+        } else if (warp == NW - 1) {
+            if (j > 0) {
+                const double* d = col_after(0);
+                double* g = ABg + (size_t)(j - 1) * ldab - 1;
+                for (int t = 1 + lane; t <= ldab; t += 32) g[t] = d[t];
+            }
+            // column j+KV+AHEAD-1 takes the slot of column j-2, written back two
+            // steps ago (at j = 2 a slot that was never used)
+            if (pf_col > 0) {
+                double* e = col(pf_col);
+#pragma unroll
+                for (int u = 0; u < LU1_ROWS; u++) {
+                    const int t = 1 + lane + 32 * u;
+                    if (t <= ldab) e[t] = pf[u];
+                }
+            }
+            pf_col = (j >= 1 && j + KV + LU1_AHEAD <= n) ? j + KV + LU1_AHEAD : 0;
+            if (pf_col > 0) {
+                const double* g = ABg + (size_t)(pf_col - 1) * ldab - 1;
+#pragma unroll
+                for (int u = 0; u < LU1_ROWS; u++) {
+                    const int t = 1 + lane + 32 * u;
+                    pf[u] = (t <= ldab && t > kl) ? g[t] : 0.0;  // rows 1..kl: fill-in
+                }
+            }
+        } else if (nz) {
+            // columns j+2..JU, G at a time: at most 64 elements, two per lane
+            for (int c0 = 2 + (warp - 1) * G; c0 <= JU - j; c0 += (NW - 2) * G) {
+                double v[2], top[2];
+                double *at[2], *topat[2];
+#pragma unroll
+                for (int u = 0; u < 2; u++) {
+                    const int e = lane + 32 * u;
+                    at[u] = topat[u] = nullptr;
+                    int q = (e >= KM) + (e >= 2 * KM) + (e >= 3 * KM);
+                    if (G > 4) q = e / KM;
+                    const int c = c0 + q, t = 1 + e - q * KM;
+                    if (e >= G * KM || c > JU - j) continue;
+                    double* a = col_after(c) + KV + 1 - c;  // row j of column j + c
+                    top[u] = a[JP - 1];
+                    const double temp = -top[u];
+                    v[u] = (t == JP - 1) ? a[0] : a[t];
+                    if (nonzero(temp)) v[u] = v[u] + mj[t] * temp;
+                    at[u] = a + t;
+                    if (t == 1 && JP != 1) topat[u] = a;
+                }
+                __syncwarp();
+#pragma unroll
+                for (int u = 0; u < 2; u++) {
+                    if (at[u] != nullptr) *at[u] = v[u];
+                    if (topat[u] != nullptr) *topat[u] = top[u];
+                }
+                __syncwarp();
+            }
+        }
+        __syncthreads();
+        if (++at_j == C) at_j = 0;
+        if (j < n) code = sCode[(j + 1) & 1];
+    }
+    if (tid == 0) *info_out = info;
+}
+// dgbtf2 on one CTA with the band in global memory: bands too wide for the kernels
+// above and below.
+__global__ void k_coarse_lu_global(double* __restrict__ AB, int* __restrict__ ipiv, int n, int kl, int ku,
+                                   int* info_out) {
     const int ldab = 2 * kl + ku + 1, KV = ku + kl;
-    const size_t tot = (size_t)ldab * n;
-    double* AB = in_smem ? sm : ABg;
     const int tid = threadIdx.x, nth = blockDim.x;
-    if (in_smem)
-        for (size_t t = tid; t < tot; t += nth) sm[t] = ABg[t];
     __shared__ int sJP, sJU, sInfo;
     __shared__ double sPiv;
     if (tid == 0) { sJU = 1; sInfo = 0; }
@@ -611,8 +790,6 @@ __global__ void k_coarse_lu(double* __restrict__ ABg, int* __restrict__ ipiv, in
         __syncthreads();
     }
 #undef A_
-    if (in_smem)
-        for (size_t t = tid; t < tot; t += nth) ABg[t] = sm[t];
     if (tid == 0) *info_out = sInfo;
 }
 // The same factorisation for bands too large for one CTA's shared memory:
@@ -786,11 +963,18 @@ __global__ void __launch_bounds__(512) k_coarse_lu_cl(double* __restrict__ ABg, 
 }
 
 void launch_coarse_lu(cudaStream_t s, double* band, int* ipiv, int n, int kl, int ku, DevScalars* ds) {
-    size_t bytes = sizeof(double) * (size_t)(2 * kl + ku + 1) * n;
-    int in_smem = bytes <= 200 * 1024 ? 1 : 0;
+    const int ldab = 2 * kl + ku + 1;
+    const size_t ring = sizeof(double) * (size_t)ldab * (kl + ku + 1 + LU1_AHEAD);
+    // one CTA while its FP64 pipe does a column's update in about the time of the
+    // chain of its pivot (kl^2 cycles against some 1000); wider bands on a cluster
+    if (kl <= LU1_MAXKL && ldab <= 32 * LU1_ROWS && ring <= 200 * 1024) {
+        cudaFuncSetAttribute(k_coarse_lu, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        k_coarse_lu<<<1, LU1_THREADS, ring, s>>>(band, ipiv, n, kl, ku, &ds->lu_info); tc_note_launch();
+        return;
+    }
     const int R = kl + 1, C = kl + ku + 1, Cq = (C + LU_CL - 1) / LU_CL;
     const size_t win = sizeof(double) * ((size_t)R * Cq + 2 * (size_t)R);
-    if (!in_smem && win <= 200 * 1024) {
+    if (win <= 200 * 1024) {
         cudaFuncSetAttribute(k_coarse_lu_cl, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)win);
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(LU_CL, 1, 1);
@@ -807,12 +991,7 @@ void launch_coarse_lu(cudaStream_t s, double* band, int* ipiv, int n, int kl, in
         cudaLaunchKernelEx(&cfg, k_coarse_lu_cl, band, ipiv, n, kl, ku, &ds->lu_info); tc_note_launch();
         return;
     }
-    size_t sm = in_smem ? bytes : 0;
-    if (in_smem) cudaFuncSetAttribute(k_coarse_lu, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    // 512 threads: the rank-1 updates keep one SM's FP64 pipe busy (574 us
-    // for the 217-unknown coarse grid of 1024x256; 606 / 668 / 888 us / 1.30 ms
-    // with 256 / 128 / 64 / 32 threads, 775 us on the 8-CTA cluster variant)
-    k_coarse_lu<<<1, 512, sm, s>>>(band, ipiv, n, kl, ku, in_smem, &ds->lu_info); tc_note_launch();
+    k_coarse_lu_global<<<1, 512, 0, s>>>(band, ipiv, n, kl, ku, &ds->lu_info); tc_note_launch();
 }
 
 // Explicit inverse of the factored coarse matrix: column j of A^-1 is the
