@@ -1,8 +1,8 @@
 """The banded LU of the coarsest matrix at the edges of its kernels.
 
-Solves whose coarsest grids have the narrowest bands, bands at both sides of one
-lane's second row (kl = 32), of the one-block kernel's limit (kl = 63) and beyond:
-cycle counts equal the oracle's and the stream function agrees within the bound of
+Solves whose coarsest grids have the narrowest bands, bands at both sides of the
+one-block kernel's limit (kl = 20) and of the panel kernel's block sizes (kl = 32, 96 and
+224), the last panel full, of one column and in between: cycle counts equal the oracle's and the stream function agrees within the bound of
 test_gpu_parity.py (1e-9 of its largest value).
 """
 import numpy as np
@@ -15,9 +15,10 @@ from tests.cases import case_1024_like, fresh_state
 pytestmark = pytest.mark.gpu
 
 
-# kl = 2 nz / 2^(grids-1) + 2
-@pytest.mark.parametrize("nx,nz,grids,kl", [(64, 16, 3, 10), (96, 24, 3, 14), (48, 30, 2, 32), (48, 32, 2, 34),
-                                            (40, 60, 2, 62), (40, 62, 2, 64)])
+# n = (nx / 2^(grids-1) + 1) (nz / 2^(grids-1) + 1), kl = 2 nz / 2^(grids-1) + 2
+@pytest.mark.parametrize("nx,nz,grids,kl", [(64, 16, 3, 10), (48, 18, 2, 20), (48, 20, 2, 22), (44, 22, 2, 24),
+                                            (42, 30, 2, 32), (46, 32, 2, 34), (20, 94, 2, 96), (16, 96, 2, 98),
+                                            (14, 222, 2, 224), (16, 224, 2, 226)])
 def test_solve_equals_oracle(gpu_lib, nx, nz, grids, kl):
     p = case_1024_like(nx=nx, nz=nz, tpc=4, grids=grids)
     p.aspect, p.max_cycles = nx / nz, 200

@@ -13,6 +13,7 @@
 // The kernels specialise the metric terms to the uniform grid (xr=zs=1,
 // xrr=...=0), which leaves every retained product and sum of the reference
 // unchanged.
+#include "tc_cluster.cuh"
 #include "tc_device.cuh"
 #include <cooperative_groups.h>
 namespace cg = cooperative_groups;
@@ -550,15 +551,14 @@ void launch_coarse_build(cudaStream_t s, const Level& lv, double* band, double* 
 // the column that enters the ring.  Every element sees dgbtf2's operations in
 // dgbtf2's order.
 //
-// What bounds it: the chain of warp 0, 1 us a column (update, search, reciprocal,
-// scaling, barrier: FP64 latencies), and for kl > 32 the FP64 pipe of one SM.
-// Against six barriers a column and the trailing update as one flat loop: 651 ->
-// 308 us at n = 297, kl = 20; 2044 -> 895 us at n = 1000, kl = 8; 3164 -> 2360 us at
-// n = 400, kl = 63.
+// What bounds it: the chain of warp 0, 0.75 to 1 us a column (update, search,
+// reciprocal, scaling, barrier: FP64 latencies).  Against six barriers a column and the
+// trailing update as one flat loop: 598 -> 269 us at n = 297, kl = 20 without
+// interchanges, 709 -> 322 with; 1881 -> 751 us at n = 1000, kl = 8.
 #define LU1_THREADS 512
 #define LU1_AHEAD 4   // columns loaded ahead of the window
-#define LU1_MAXKL 63  // two rows per lane of warp 0
-#define LU1_ROWS 6    // band rows per lane of the loading warp (2 kl + ku + 1 <= 192)
+#define LU1_MAXKL 20  // see launch_coarse_lu; at most 31: a row per lane of warp 0
+#define LU1_ROWS 2    // band rows per lane of the loading warp (2 kl + ku + 1 <= 64)
 __global__ void __launch_bounds__(LU1_THREADS) k_coarse_lu(double* __restrict__ ABg, int* __restrict__ ipiv, int n,
                                                            int kl, int ku, int* info_out) {
     extern __shared__ double sm[];
@@ -604,59 +604,33 @@ __global__ void __launch_bounds__(LU1_THREADS) k_coarse_lu(double* __restrict__ 
                 // column j+1: rows t = 0..KM1 below and on its diagonal, two per lane
                 const int KM1 = min(kl, n - j - 1);
                 double* a = col_after(1) + KV + 1;
-                double v[2];
-#pragma unroll
-                for (int u = 0; u < 2; u++) {
-                    const int t = lane + 32 * u;
-                    v[u] = t <= KM1 ? a[t] : 0.0;
-                }
+                double v = lane <= KM1 ? a[lane] : 0.0;
                 if (nz && j + 1 <= JU) {
                     const double oldtop = a[-1], top = a[JP - 2];
                     const double temp = -top;
-#pragma unroll
-                    for (int u = 0; u < 2; u++) {
-                        const int t = lane + 32 * u;  // row t + 1 of step j
-                        if (t + 1 == JP - 1) v[u] = oldtop;
-                        if (t < KM && nonzero(temp)) v[u] = v[u] + mj[t + 1] * temp;
-                    }
+                    if (lane + 1 == JP - 1) v = oldtop;  // lane: row lane + 1 of step j
+                    if (lane < KM && nonzero(temp)) v = v + mj[lane + 1] * temp;
                     __syncwarp();
                     if (lane == 0 && JP != 1) a[-1] = top;
                 }
                 // idamax: the first row of the largest |value| (as integers; a NaN is never the largest)
-                unsigned long long best = 0;
-                int bi = 1 << 30;
-#pragma unroll
-                for (int u = 0; u < 2; u++) {
-                    const int t = lane + 32 * u;
-                    unsigned long long k = (unsigned long long)__double_as_longlong(v[u]) & ~(1ull << 63);
-                    k = k > (0x7ffull << 52) ? 0 : k + 1;
-                    if (t <= KM1 && k > best) { best = k; bi = t; }
-                }
-                const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)(best >> 32));
-                const unsigned lo = __reduce_max_sync(0xffffffffu, (unsigned)(best >> 32) == hi ? (unsigned)best : 0u);
-                const bool is = (unsigned)(best >> 32) == hi && (unsigned)best == lo;
-                bi = (int)__reduce_min_sync(0xffffffffu, is ? (unsigned)bi : 1u << 30);
-                if (bi > KM1) bi = 0;
-                const double piv = __shfl_sync(0xffffffffu, bi < 32 ? v[0] : v[1], bi & 31);
-                const double first = __shfl_sync(0xffffffffu, v[0], 0);
+                unsigned long long key = (unsigned long long)__double_as_longlong(v) & ~(1ull << 63);
+                key = (key > (0x7ffull << 52) || lane > KM1) ? 0 : key + 1;
+                const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)(key >> 32));
+                const bool tops = (unsigned)(key >> 32) == hi;
+                const unsigned lo = __reduce_max_sync(0xffffffffu, tops ? (unsigned)key : 0u);
+                const int bi = __ffs(__ballot_sync(0xffffffffu, tops && (unsigned)key == lo)) - 1;
+                const double piv = __shfl_sync(0xffffffffu, v, bi);
+                const double first = __shfl_sync(0xffffffffu, v, 0);
                 const int nzp = nonzero(piv) ? 1 : 0;
                 if (nzp) {
                     const double rcp = 1.0 / piv;
-#pragma unroll
-                    for (int u = 0; u < 2; u++) {
-                        const int t = lane + 32 * u;
-                        if (t == bi) v[u] = first;
-                        if (t == 0) v[u] = piv;
-                        else v[u] = rcp * v[u];
-                    }
+                    if (lane == bi) v = first;
+                    v = lane == 0 ? piv : rcp * v;
                 }
-#pragma unroll
-                for (int u = 0; u < 2; u++) {
-                    const int t = lane + 32 * u;
-                    if (t <= KM1) {
-                        a[t] = v[u];
-                        mult[(j + 1) & 1][t] = v[u];
-                    }
+                if (lane <= KM1) {
+                    a[lane] = v;
+                    mult[(j + 1) & 1][lane] = v;
                 }
                 if (lane == 0) {
                     sCode[(j + 1) & 1] = (bi + 1) * 2 + nzp;
@@ -725,7 +699,7 @@ __global__ void __launch_bounds__(LU1_THREADS) k_coarse_lu(double* __restrict__ 
     if (tid == 0) *info_out = info;
 }
 // dgbtf2 on one CTA with the band in global memory: bands too wide for the kernels
-// above and below.
+// above and below (kl > 480).
 __global__ void k_coarse_lu_global(double* __restrict__ AB, int* __restrict__ ipiv, int n, int kl, int ku,
                                    int* info_out) {
     const int ldab = 2 * kl + ku + 1, KV = ku + kl;
@@ -792,205 +766,350 @@ __global__ void k_coarse_lu_global(double* __restrict__ AB, int* __restrict__ ip
 #undef A_
     if (tid == 0) *info_out = sInfo;
 }
-// The same factorisation for bands too large for one CTA's shared memory:
-// at step j only rows j..j+kl of columns j..j+KV are active (KV = kl+ku),
-// so that block is kept in the shared memory of a cluster of LU_CL CTAs,
-// columns dealt round-robin by (column mod (KV+1)) and rows by (row mod
-// (kl+1)).  The owner of column j searches the pivot, swaps and scales
-// column j and pushes the multipliers into every CTA's shared memory; after
-// one cluster barrier every CTA swaps and updates its own columns, writes
-// back row j of them and column j (its owner), and loads the row and column
-// that enter the block.  Each element sees the operations of dgbtf2 in the
-// same order as in k_coarse_lu.
-#define LU_CL 8
-__global__ void __launch_bounds__(512) k_coarse_lu_cl(double* __restrict__ ABg, int* __restrict__ ipiv, int n,
-                                                      int kl, int ku, int* info_out) {
-    cg::cluster_group cl = cg::this_cluster();
-    const int rank = (int)cl.block_rank();
-    extern __shared__ double smw[];
-    const int ldab = 2 * kl + ku + 1, KV = ku + kl, R = kl + 1, C = KV + 1, Cq = (C + LU_CL - 1) / LU_CL;
-    double* Wl = smw;                       // [R][Cq]
-    double* buf = smw + (size_t)R * Cq;     // [2][R] multipliers of column j
-    __shared__ int sInfoPiv[2];             // pivot row offset * 2 + (pivot != 0), per step parity
-    __shared__ int sJP;
-    const int tid = threadIdx.x, nth = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nth >> 5;
-#define AB(rw, jc) ABg[(size_t)((rw) - 1) + (size_t)((jc) - 1) * ldab]
-    // dgbtf2's first loop: fill-in entries of columns ku+2..KV
-    if (rank == 0)
-        for (int jj = ku + 2; jj <= min(KV, n); jj++)
-            for (int i = KV - jj + 2 + tid; i <= kl; i += nth) AB(i, jj) = 0.0;
-    cl.sync();
-    // the block of step 1 (column 1+KV: rows 1..kl zeroed as dgbtf2 does at step 1)
-    for (int e = tid; e < R * Cq; e += nth) {
-        const int a = e / Cq, lc = e % Cq, cs = lc * LU_CL + rank;
-        if (cs >= C) continue;
-        // row 1+a sits in slot (1+a) mod R, column jc of 1..C in slot jc mod C
-        const int i = 1 + a, jc = (cs == 0) ? C : cs;
-        double v = 0.0;
-        if (i <= n && jc <= n) v = (jc == C && a < kl) ? 0.0 : AB(KV + 1 + i - jc, jc);
-        Wl[(size_t)(i % R) * Cq + lc] = v;
+// The same factorisation with a panel of LUP_NB columns per launch, for wider bands.
+// Launch p factors panel p and applies panel p-1 to the columns behind it, so that
+// only the panel's own chain of pivots is serial:
+//  - Cluster 0 takes one column of the panel per CTA, one row per thread.  Each CTA
+//    applies each step of the panel as it arrives, then searches its pivot.  While one
+//    warp does that and divides, the others send the unscaled column to the cluster's
+//    CTAs (st.async); the pivot and its reciprocal follow, and the receivers scale.
+//    The second half of its threads brings a column of panel p+1 up to date in the
+//    same way, with the steps of panel p-1 first.
+//  - The other CTAs apply the steps of panel p-1 to one column per warp, in registers.
+// A column sees the steps before it in order, each as interchange and update with a
+// separate multiply and add: dgbtf2's operations in dgbtf2's order.  The fill-in rows
+// of the band are zero on entry (launch_coarse_build clears the band).
+//
+// What bounds it: the chain of pivots, 2400 cycles a column at kl = 202 (1800 at 20):
+// update 750 (three dependent FP64 operations on seven warps, the pipe does 2 lanes a
+// cycle), search 600, reciprocal 620, message 400.  Everything else is kept off it.
+// Before, one cluster of 8 CTAs with the whole window in its shared memory, every
+// column's update on the chain: n = 10201, kl = 202 (a 200x200 grid halved once) 73 ms,
+// now 14.1; one CTA for n = 400, kl = 63: 2.36 ms, now 0.46.
+#define LUP_NB 16
+#define LUP_CL 16              // CTAs of the panel's cluster: one per column
+#define LUP_WAIT (1 << 20)     // polls of a wait for a column's multipliers
+template <int T>
+__global__ void __launch_bounds__(2 * T) k_lu_panel(double* ABg, int* ipiv, int n, int kl, int ku, int p, DevScalars* ds) {
+    constexpr int NB = LUP_NB, NW = T / 32, R = T / 32;  // NW: warps of a column
+    extern __shared__ __align__(16) double smd[];  // [2][NB][T]: multipliers of panel p-1, unscaled columns of this one
+    double* msg = smd + NB * T;
+    __shared__ __align__(8) unsigned long long bar[NB];
+    __shared__ __align__(16) unsigned long long head[NB][2];  // per column of the panel: code, reciprocal
+    __shared__ int s_ju[NB], s_op[NB], s_max;
+    __shared__ __align__(16) double s_cols[2][2][T];
+    __shared__ double s_rcp, s_val[2][NW];
+    __shared__ unsigned long long s_key[2][NW];
+    __shared__ int s_idx[2][NW], s_bi;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int ldab = 2 * kl + ku + 1, KV = kl + ku;
+    const int j0 = p * NB + 1, b0 = j0 - NB;  // first column (1-based); row of offset 0
+    const bool panel = blockIdx.x < LUP_CL;
+    const int c = blockIdx.x;                 // the panel's column of this CTA
+    const int last = min(LUP_CL, n - j0 + 1) - 1;
+    auto at = [&](int r, int q) { return ABg + (size_t)(q - 1) * ldab + (KV + r - q); };
+    auto nonzero = [](double x) { return (unsigned long long)(__double_as_longlong(x) << 1) != 0ull; };
+    // the first lane with the largest key
+    auto first_max = [](unsigned long long key) {
+        const unsigned hi = (unsigned)(key >> 32), top = __reduce_max_sync(0xffffffffu, hi);
+        unsigned who = __ballot_sync(0xffffffffu, hi == top);
+        if (__popc(who) > 1) {
+            const unsigned lo = __reduce_max_sync(0xffffffffu, hi == top ? (unsigned)key : 0u);
+            who = __ballot_sync(0xffffffffu, hi == top && (unsigned)key == lo);
+        }
+        return __ffs(who) - 1;
+    };
+    // rows sent of column i: its pivot rows, in 16-byte pairs
+    auto sent_from = [&](int i) { return (NB + i) & ~1; };
+    auto sent_bytes = [&](int i) { return 8 * (((NB + i + min(kl, n - j0 - i)) | 1) + 1 - sent_from(i)); };
+    if (panel) {
+        if (tid < NB) mbar_init(smem_addr(&bar[tid]), 1);
+        __syncthreads();
+        if (tid <= last) mbar_arrive_expect(smem_addr(&bar[tid]), sent_bytes(tid) + 16);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        cluster_arrive();
     }
-    int JU = 1, info = 0;
-    // one value per thread of the row entering at the next step, loaded a step
-    // ahead (when every column of the block has its own thread)
-    const bool prefetch = (C <= nth);
-    double pf = 0.0;
-    int pf_lc = -1;
+    pdl_entry();
+    pdl_done();
+    if (tid == 0) s_max = 0;
     __syncthreads();
-    for (int j = 1; j <= n; j++) {
-        const int r0 = j % R, c0 = j % C;
-        auto RS = [&](int a) { const int v = r0 + a; return v >= R ? v - R : v; };
-        // local column index of absolute column j + c (owned by this CTA or -1)
-        auto LC = [&](int c) { int cs = c0 + c; if (cs >= C) cs -= C; return (cs % LU_CL == rank) ? cs / LU_CL : -1; };
-        if (j >= 2) {
-            // rows j..j+kl-1 of the column that enters (j+KV) are zeroed, row j+kl enters
-            const int jcn = j + KV;
-            if (jcn <= n) {
-                const int lc = LC(KV);
-                if (lc >= 0)
-                    for (int a = tid; a < kl; a += nth) Wl[(size_t)RS(a) * Cq + lc] = 0.0;
-            }
-            const int i = j + kl;
-            if (prefetch) {
-                if (pf_lc >= 0) Wl[(size_t)RS(kl) * Cq + pf_lc] = pf;
-            } else if (i <= n) {
-                for (int c = tid; c <= KV; c += nth) {
-                    const int lc = LC(c), jc = j + c;
-                    if (lc >= 0) Wl[(size_t)RS(kl) * Cq + lc] = (jc <= n) ? AB(KV + 1 + i - jc, jc) : 0.0;
-                }
-            }
-            __syncthreads();
-        }
-        if (prefetch) {
-            // row j+1+kl over columns j+1..j+1+KV, for step j+1
-            pf_lc = -1;
-            const int i1 = j + 1 + kl, c = tid;
-            if (j + 1 <= n && i1 <= n && c <= KV) {
-                int cs = c0 + 1 + c;
-                while (cs >= C) cs -= C;
-                if (cs % LU_CL == rank) {
-                    const int jc = j + 1 + c;
-                    pf_lc = cs / LU_CL;
-                    pf = (jc <= n) ? AB(KV + 1 + i1 - jc, jc) : 0.0;
-                }
-            }
-        }
-        const int KM = min(kl, n - j);
-        const int owner = c0 % LU_CL;
-        if (rank == owner) {
-            const int lc = c0 / LU_CL;
-            if (warp == 0) {
-                double best = -1.0;
-                int bi = 1 << 30;
-                for (int t = 1 + lane; t <= KM + 1; t += 32) {
-                    const double v = fabs(Wl[(size_t)RS(t - 1) * Cq + lc]);
-                    if (v > best) { best = v; bi = t; }
-                }
-                for (int off = 16; off > 0; off >>= 1) {
-                    const double ob = __shfl_down_sync(0xffffffffu, best, off);
-                    const int oi = __shfl_down_sync(0xffffffffu, bi, off);
-                    if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
-                }
-                if (lane == 0) {
-                    sJP = bi;
-                    ipiv[j - 1] = bi + j - 1;
-                    const double pv = Wl[(size_t)RS(bi - 1) * Cq + lc];
-                    const int code = bi * 2 + (pv != 0.0 ? 1 : 0);
-                    if (pv != 0.0 && bi != 1) {
-                        Wl[(size_t)RS(bi - 1) * Cq + lc] = Wl[(size_t)RS(0) * Cq + lc];
-                        Wl[(size_t)RS(0) * Cq + lc] = pv;
-                    }
-                    for (int q = 0; q < LU_CL; q++) cl.map_shared_rank(sInfoPiv, q)[j & 1] = code;
-                }
-            }
-            __syncthreads();
-            if ((sInfoPiv[j & 1] & 1) && KM > 0) {
-                const double rcp = 1.0 / Wl[(size_t)RS(0) * Cq + lc];
-                for (int t = 1 + tid; t <= KM; t += nth) {
-                    const double v = rcp * Wl[(size_t)RS(t) * Cq + lc];
-                    Wl[(size_t)RS(t) * Cq + lc] = v;
-                    for (int q = 0; q < LU_CL; q++) cl.map_shared_rank(buf, q)[(j & 1) * R + t] = v;
-                }
-            }
-        }
-        cl.sync();  // multipliers and pivot of column j visible in every CTA
-        const int code = sInfoPiv[j & 1];
-        const int JP = code >> 1;
-        const bool nz = (code & 1) != 0;
-        if (nz) JU = max(JU, min(j + ku + JP - 1, n));
-        else if (info == 0) info = j;
-        if (nz) {
-            const double* mult = buf + (j & 1) * R;
-            // this CTA's columns of the block: local index lc holds slot lc*LU_CL+rank,
-            // i.e. column j + c with c = (slot - j) mod C
-            for (int lc = warp; lc < Cq; lc += nw) {
-                const int cs = lc * LU_CL + rank;
-                if (cs >= C) break;
-                int c = cs - c0;
-                if (c < 0) c += C;
-                if (c < 1 || c > JU - j) continue;
-                double* top = &Wl[(size_t)RS(0) * Cq + lc];
-                if (JP != 1 && lane == 0) {
-                    double* pr = &Wl[(size_t)RS(JP - 1) * Cq + lc];
-                    const double t0 = *pr;
-                    *pr = *top;
-                    *top = t0;
-                }
-                __syncwarp();
-                const double temp = -*top;
-                if (temp != 0.0)
-                    for (int t = 1 + lane; t <= KM; t += 32) {
-                        double* e = &Wl[(size_t)RS(t) * Cq + lc];
-                        *e = *e + mult[t] * temp;
-                    }
-            }
-        }
-        __syncthreads();
-        // write back column j (its owner) and row j (every CTA, its columns)
-        if (rank == owner) {
-            const int lc = c0 / LU_CL;
-            for (int a = tid; a <= kl; a += nth)
-                if (j + a <= n) AB(KV + 1 + a, j) = Wl[(size_t)RS(a) * Cq + lc];
-        }
-        for (int c = 1 + tid; c <= KV; c += nth) {
-            const int lc = LC(c), jc = j + c;
-            if (lc >= 0 && jc <= n) AB(KV + 1 - c, jc) = Wl[(size_t)RS(0) * Cq + lc];
-        }
-        __syncthreads();
+    if (p > 0 && tid < NB) {
+        const int ju = ld_state(&ds->lu_ju[(p - 1) & 1][tid]);
+        s_ju[tid] = ju;
+        s_op[tid] = ld_state(ipiv + b0 - 1 + tid) - b0;
+        atomicMax(&s_max, ju);
     }
-#undef AB
-    if (rank == 0 && tid == 0) *info_out = info;
+    if (panel) {
+        // threads 0..T-1: column c of the panel; T..2T-1: column c of the next panel,
+        // which follows the steps at its own pace
+        const bool ahead = tid >= T;
+        const int o = tid & (T - 1), jc = j0 + c + (ahead ? NB : 0), r = b0 + o;
+        const bool live = c <= last, valid = jc <= n && r >= max(1, jc - KV) && r <= min(n, jc + kl);
+        double v = valid ? ld_state(at(r, jc)) : 0.0;
+        double(*s_cur)[T] = s_cols[ahead ? 1 : 0];
+        // the column as its other threads see it: s_cur[x]
+        int x = 0;
+        auto publish = [&] {
+            x ^= 1;
+            s_cur[x][o] = v;
+            asm volatile("bar.sync %0, %1;" ::"r"(ahead ? 2 : 1), "n"(T) : "memory");
+        };
+        // step k (offset ok, pivot offset op) on this column: interchange and update
+        auto step = [&](bool on, int ok, int op, auto mult) {
+            const double top = s_cur[x][op], old = s_cur[x][ok], temp = -top;
+            if (on) {
+                if (o == op) v = old;
+                if (o == ok) v = top;
+                if (nonzero(temp) && o > ok && o <= ok + kl && r <= n) v = v + mult() * temp;
+            }
+        };
+        __syncthreads();
+        publish();
+        bool dead = false;
+        // the step of column i of this panel, once it is here; its JU and info.  Every thread passes the
+        // same barriers, also if a wait gave up
+        auto arrived = [&](int i, int& ju, int& info) {
+            int it = 0;
+            while (!mbar_try_wait(smem_addr(&bar[i]), 0))
+                if (dead || ++it > LUP_WAIT) { dead = true; break; }
+            const unsigned long long code = head[i][0];
+            const double rcp = __longlong_as_double((long long)head[i][1]);
+            const int ok = NB + i, op = (int)(code >> 1) & (T - 1);
+            ju = (int)(code >> 12) & 0xffffff;
+            info = (int)(code >> 36);
+            step((code & 1) && jc <= ju, ok, op, [&] { return rcp * msg[i * T + (o == op ? ok : o)]; });
+        };
+        if (ahead) {
+            // The FP64 pipe is the panel's while this CTA holds the pivot chain: these
+            // columns wait until it has passed -- at once, with the steps of panel p-1
+            // done, or just before it comes, by the time they have until then.
+            auto chain_passed = [] { asm volatile("bar.sync 3, %0;" ::"n"(2 * T) : "memory"); };
+            const int pause = c < 6 ? -1 : c < 10 ? 0 : c - 1;
+            int ju, info;
+            if (live && pause < 0) chain_passed();
+            if (p > 0) {
+#pragma unroll
+                for (int i = 0; i < NB; i++) {
+                    const int k = b0 + i;
+                    smd[i * T + o] = (r > k && r <= min(n, k + kl)) ? ld_state(at(r, k)) : 0.0;
+                }
+#pragma unroll 1
+                for (int i = 0; i < NB; i++) {
+                    step(jc <= s_ju[i], i, s_op[i], [&] { return smd[i * T + o]; });
+                    publish();
+                }
+            }
+            cluster_wait();  // every mbarrier of the cluster is set up
+#pragma unroll 1
+            for (int i = 0; live && i <= last; i++) {
+                if (i == pause) chain_passed();
+                arrived(i, ju, info);
+                publish();
+            }
+            if (valid) *at(r, jc) = v;
+            if (o == 0 && dead) atomicExch(&ds->visit_timeout, 1);
+            cluster_arrive_relaxed();
+            cluster_wait();
+            return;
+        }
+        cluster_wait();
+        int ju = 1, info = 0;
+        if (c == 0 && p > 0) {
+            ju = ld_state(&ds->lu_run);
+            info = ld_state(&ds->lu_info);
+        }
+        // the unscaled column to CTA c + 1 + l (modulo the columns of the panel)
+        auto send_column = [&](int l) {
+            const int q = c + 1 + l <= last ? c + 1 + l : c + l - last, t = sent_from(c);
+            bulk_to_cluster(cluster_addr(smem_addr(msg + c * T + t), q), smem_addr(&s_cur[x][t]), sent_bytes(c),
+                            cluster_addr(smem_addr(&bar[c]), q));
+        };
+        if (live) {
+            // The search and the division also run once before the first step: that brings
+            // their code into the instruction cache before the chain waits for it.
+            const int ok = NB + c, KM = min(kl, n - jc);
+#pragma unroll 1
+            for (int i = 0; i <= c; i++) {
+                if (i > 0) arrived(i - 1, ju, info);
+                if (i > 0 && i < c) {
+                    publish();
+                    continue;
+                }
+                // idamax (as integers; a NaN is never the largest)
+                unsigned long long key = (unsigned long long)__double_as_longlong(v) & ~(1ull << 63);
+                key = (key > (0x7ffull << 52) || o < ok || o > ok + KM) ? 0 : key + 1;
+                if (lane == first_max(key)) {
+                    s_key[x][warp] = key;
+                    s_idx[x][warp] = o;
+                    s_val[x][warp] = v;
+                }
+                const bool own = i == c;
+                if (own && o >= sent_from(c) && 8 * (o - sent_from(c)) < sent_bytes(c))
+                    st_async8(cluster_addr(smem_addr(msg + c * T + o), c < last ? c + 1 : 0),
+                              (unsigned long long)__double_as_longlong(v),
+                              cluster_addr(smem_addr(&bar[c]), c < last ? c + 1 : 0));
+                publish();
+                if (warp == 0) {
+                    key = lane < NW ? s_key[x ^ 1][lane] : 0;
+                    int op = lane < NW ? s_idx[x ^ 1][lane] : 0;
+                    double piv = lane < NW ? s_val[x ^ 1][lane] : 0.0;
+                    const int w = first_max(key);
+                    key = __shfl_sync(0xffffffffu, key, w);
+                    op = __shfl_sync(0xffffffffu, op, w);
+                    piv = __shfl_sync(0xffffffffu, piv, w);
+                    if (key == 0) {  // no number among them
+                        op = ok;
+                        piv = s_cur[x][ok];
+                    }
+                    const bool nz = nonzero(piv);
+                    double rcp = 0.0;
+                    if (nz) rcp = 1.0 / piv;
+                    if (own) {
+                        if (nz) ju = max(ju, min(b0 + op + ku, n));
+                        else if (info == 0) info = jc;
+                    }
+                    const unsigned long long code = (unsigned long long)info << 36 | (unsigned long long)ju << 12 |
+                                                    (unsigned long long)op << 1 | (nz ? 1 : 0);
+                    // to every CTA, the next one first
+                    if (own && lane <= last) {
+                        const int q = c + 1 + lane <= last ? c + 1 + lane : c + lane - last;
+                        st_async16(cluster_addr(smem_addr(head[c]), q), code,
+                                   (unsigned long long)__double_as_longlong(rcp), cluster_addr(smem_addr(&bar[c]), q));
+                    }
+                    if (lane == 0) {
+                        s_bi = op;
+                        s_rcp = rcp;
+                    }
+                }
+            }
+            asm volatile("bar.arrive 3, %0;" ::"n"(2 * T) : "memory");
+            fence_async();
+            asm volatile("bar.sync 1, %0;" ::"n"(T) : "memory");
+            if (tid >= 1 && tid <= last) send_column(tid);
+            const int op = s_bi;
+            const double piv = s_cur[x][op];
+            if (nonzero(piv)) {
+                if (o == op) v = s_cur[x][ok];
+                if (o == ok) v = piv;
+                if (o > ok && o <= ok + KM) v = s_rcp * v;
+            }
+            if (valid) *at(r, jc) = v;
+            if (tid == 0) {
+                ipiv[jc - 1] = b0 + op;
+                ds->lu_ju[p & 1][c] = nonzero(piv) ? ju : 0;
+                if (c == last) {
+                    ds->lu_run = ju;
+                    ds->lu_info = info;
+                }
+                if (dead) atomicExch(&ds->visit_timeout, 1);
+            }
+        }
+        cluster_arrive_relaxed();
+        cluster_wait();  // no CTA leaves while another still reads or writes its shared memory
+        return;
+    }
+    // columns behind these two panels: steps of panel p-1
+    if (tid < T) {
+        const int r = b0 + tid;
+#pragma unroll 4
+        for (int i = 0; i < NB; i++) {
+            const int k = b0 + i;
+            smd[i * T + tid] = (r > k && r <= min(n, k + kl)) ? ld_state(at(r, k)) : 0.0;
+        }
+    }
+    __syncthreads();
+    const int nct = gridDim.x - LUP_CL, reach = s_max;
+    for (int q = j0 + 2 * NB + (int)(blockIdx.x - LUP_CL) + warp * nct; q <= reach; q += nct * 2 * NW) {
+        const int rlo = max(1, q - KV), rhi = min(n, min(q + kl, b0 + NB - 1 + kl));
+        double v[R];
+#pragma unroll
+        for (int u = 0; u < R; u++) {
+            const int r = b0 + lane + 32 * u;
+            v[u] = (r >= rlo && r <= rhi) ? ld_state(at(r, q)) : 0.0;
+        }
+#pragma unroll 1
+        for (int i = 0; i < NB; i++) {
+            if (q > s_ju[i]) continue;
+            const int op = s_op[i], up = op >> 5, KM = min(kl, n - (b0 + i));
+            double x = v[0];
+#pragma unroll
+            for (int u = 1; u < R; u++)
+                if (u == up) x = v[u];
+            const double top = __shfl_sync(0xffffffffu, x, op & 31), old = __shfl_sync(0xffffffffu, v[0], i);
+            const double temp = -top;
+            if (lane == (op & 31)) {
+#pragma unroll
+                for (int u = 0; u < R; u++)
+                    if (u == up) v[u] = old;
+            }
+            if (lane == i) v[0] = top;
+            if (nonzero(temp)) {
+#pragma unroll
+                for (int u = 0; u < R; u++) {
+                    const int o = lane + 32 * u;
+                    if (o > i && o <= i + KM) v[u] = v[u] + smd[i * T + o] * temp;
+                }
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < R; u++) {
+            const int r = b0 + lane + 32 * u;
+            if (r >= rlo && r <= rhi) *at(r, q) = v[u];
+        }
+    }
+}
+// false where the device does not hold a cluster of LUP_CL such CTAs
+template <int T>
+bool launch_lu_panels(cudaStream_t s, double* band, int* ipiv, int n, int kl, int ku, DevScalars* ds) {
+    const size_t smem = sizeof(double) * 2 * LUP_NB * T;
+    cudaFuncSetAttribute(k_lu_panel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaFuncSetAttribute(k_lu_panel<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    // two to four columns behind the panel per SM, on up to eight clusters with the panel's
+    const int clusters = 1 + std::min(7, (kl + ku + 31) / 32);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(LUP_CL * clusters, 1, 1);
+    cfg.blockDim = dim3(2 * T, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = LUP_CL;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    static const int fits = [&] {
+        int c = 0;
+        if (cudaOccupancyMaxActiveClusters(&c, k_lu_panel<T>, &cfg) != cudaSuccess) { cudaGetLastError(); return 0; }
+        return c;
+    }();
+    if (fits < 1) return false;
+    cfg.numAttrs = 2;
+    for (int p = 0; p * LUP_NB < n; p++) {
+        if (p == 0) cfg.gridDim.x = LUP_CL;
+        else cfg.gridDim.x = LUP_CL * clusters;
+        cudaLaunchKernelEx(&cfg, k_lu_panel<T>, band, ipiv, n, kl, ku, p, ds); tc_note_launch();
+    }
+    return true;
 }
 
 void launch_coarse_lu(cudaStream_t s, double* band, int* ipiv, int n, int kl, int ku, DevScalars* ds) {
     const int ldab = 2 * kl + ku + 1;
     const size_t ring = sizeof(double) * (size_t)ldab * (kl + ku + 1 + LU1_AHEAD);
-    // one CTA while its FP64 pipe does a column's update in about the time of the
-    // chain of its pivot (kl^2 cycles against some 1000); wider bands on a cluster
-    if (kl <= LU1_MAXKL && ldab <= 32 * LU1_ROWS && ring <= 200 * 1024) {
-        cudaFuncSetAttribute(k_coarse_lu, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    // one CTA for the narrowest bands: no messages and no launches between the columns
+    // (n = 1000, kl = 8: 751 us against 1033 by panels), while its FP64 pipe keeps up with
+    // the chain of pivots (n = 552, kl = 24: 938 against 575)
+    if (kl <= LU1_MAXKL && ldab <= 32 * LU1_ROWS && ring <= 48 * 1024) {
         k_coarse_lu<<<1, LU1_THREADS, ring, s>>>(band, ipiv, n, kl, ku, &ds->lu_info); tc_note_launch();
         return;
     }
-    const int R = kl + 1, C = kl + ku + 1, Cq = (C + LU_CL - 1) / LU_CL;
-    const size_t win = sizeof(double) * ((size_t)R * Cq + 2 * (size_t)R);
-    if (win <= 200 * 1024) {
-        cudaFuncSetAttribute(k_coarse_lu_cl, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)win);
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(LU_CL, 1, 1);
-        cfg.blockDim = dim3(512, 1, 1);
-        cfg.dynamicSmemBytes = win;
-        cfg.stream = s;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = LU_CL;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        cudaLaunchKernelEx(&cfg, k_coarse_lu_cl, band, ipiv, n, kl, ku, &ds->lu_info); tc_note_launch();
-        return;
-    }
+    // one row per thread: the rows that two panels' steps reach
+    const int rows = kl + 2 * LUP_NB;
+    if (rows <= 64 ? launch_lu_panels<64>(s, band, ipiv, n, kl, ku, ds)
+        : rows <= 128 ? launch_lu_panels<128>(s, band, ipiv, n, kl, ku, ds)
+        : rows <= 256 ? launch_lu_panels<256>(s, band, ipiv, n, kl, ku, ds)
+        : rows <= 512 && launch_lu_panels<512>(s, band, ipiv, n, kl, ku, ds)) return;
     k_coarse_lu_global<<<1, 512, 0, s>>>(band, ipiv, n, kl, ku, &ds->lu_info); tc_note_launch();
 }
 

@@ -30,6 +30,7 @@
 // their order, c = 2/(cA + cB*temp) on the per-point Chebyshev level,
 // v = fma(c*dt, r, psi)), so a level ends in the same state bit for bit as
 // with one launch per sweep.
+#include "tc_cluster.cuh"
 #include "tc_device.cuh"
 
 #include <cooperative_groups.h>
@@ -311,40 +312,6 @@ __device__ __forceinline__ void load_tile(float* buf, int bsz, int R, const Lay&
                 }
         }
 }
-
-// ---- cluster primitives ------------------------------------------------------------
-__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ uint32_t cluster_addr(uint32_t a, int rank) {
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
-    return r;
-}
-__device__ __forceinline__ void st_async4(uint32_t raddr, float4 v, uint32_t rbar) {
-    asm volatile(
-        "st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(raddr),
-        "r"(__float_as_uint(v.x)), "r"(__float_as_uint(v.y)), "r"(__float_as_uint(v.z)), "r"(__float_as_uint(v.w)),
-        "r"(rbar)
-        : "memory");
-}
-__device__ __forceinline__ void mbar_init(uint32_t a, int count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(a), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive_expect(uint32_t a, int bytes) {
-    asm volatile("{ .reg .b64 st; mbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1; }" ::"r"(a), "r"(bytes)
-                 : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint32_t a, int parity) {
-    uint32_t ok;
-    asm volatile(
-        "{ .reg .pred p; mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2; "
-        "selp.u32 %0, 1, 0, p; }"
-        : "=r"(ok)
-        : "r"(a), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.aligned;" ::: "memory"); }
 
 // ---- a whole visit in one launch ------------------------------------------------------
 // The visit runs in periods of S sweeps, each followed by an exchange of the

@@ -105,6 +105,8 @@ struct DevScalars {
     int    flag_outside;     // tracer outside the domain
     int    flag_rk2;         // RK2 precondition failed
     int    lu_info;          // first zero pivot of the coarse LU (0 = none)
+    int    lu_run;           // coarse LU by panels: last column reached so far, and per step of the
+    int    lu_ju[2][16];     // newest two panels (0: a zero pivot, no columns updated)
     int    visit_timeout;    // a fused visit's bounded neighbour wait gave up
     int    pad;
     double acc_alpha[2];     // coefficients of the last correction of psi (k_accel.cu)
