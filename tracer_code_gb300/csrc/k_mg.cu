@@ -1207,14 +1207,235 @@ void launch_coarse_apply(cudaStream_t s, const Level& lv, const double* Ainv, co
 // Coarsest-level solve for coarse grids too large for an explicit inverse:
 // B = RowB .* RHS (Compute_coarse_vector), DGBTRS('N') with the band's LU
 // (row interchanges + unit-lower solve, then dtbsv), x to the interior
-// (Stream_grid_coarse with the stream BCs).  One block: the vector in shared
-// memory, one warp per substitution (the band is read once, from L2).
-#define CS_FW 8   // band rows below the diagonal per lane (kl <= 256) in the prefetched path
-#define CS_BW 16  // band rows above (kl + ku <= 512)
+// (Stream_grid_coarse with the stream BCs).  One cluster, the vector in the shared
+// memory of its first CTA; every element sees DGBTRS's operations in its order.
+//  - Forward, the first CTA: a row in reach per thread, re-based every 16 steps, the
+//    band's columns loaded four steps ahead, one barrier a step.
+//  - Backward, 32 rows at a time: a warp solves the block, one row per lane, and a second
+//    follows it with the next block's rows, so that it can go on from there (they take
+//    turns); meanwhile warps of the other CTAs apply the last block to the rows above.
+// What bounds it is the chain of FP64 operations: a warp's takes 64 cycles, whether it
+// depends on the one before or not, so the chain's warps share no scheduler with other
+// FP64 work.  Forward 620 cycles a step (two operations of two warps, exchange, barrier),
+// backward 720 (six operations, two of them the product with the pivot's reciprocal that
+// replaces most of a division).  Against one warp doing every step on the vector in shared
+// memory, at n = 10201, kl = 202: 27 -> 7.3 ms.
+#define CS_THREADS 256
+#define CS_CL 8
+#define CS_MAXKL 496
+#define CS_WAIT (1 << 20)  // polls of a wait for four solved rows
+// RN(x / d) from y + y2 = 1 / d to twice the precision: a quotient within one ulp, and
+// Markstein's correction with its exact remainder (IBM J. Res. Dev. 34, 1990).  y = 0: d
+// is near the ends of the range.
+__device__ __forceinline__ double solve_quot(double x, double d, double y, double y2) {
+    const double q0 = fma(x, y, x * y2);
+    double q = fma(fma(-q0, d, x), y, q0);
+    const unsigned hi = (unsigned)__double2hiint(x);
+    if ((hi >> 20 & 0x7ff) - 600u > 846u || __double2hiint(y) == 0) {
+        if (((hi << 1) | (unsigned)__double2loint(x)) != 0) q = x / d;  // 0 where x is
+    }
+    return q;
+}
+template <typename TR, int RR>
+__global__ void __launch_bounds__(CS_THREADS) k_coarse_solve(Lay L, const double* __restrict__ ABg,
+                                                             const int* __restrict__ ipiv,
+                                                             const double* __restrict__ rowb, const TR* rhs, int n,
+                                                             int kl, int ku, TR* err, int Vbc, int* timeout_flag) {
+    constexpr int NP = 16, D = 4;  // steps between re-basings, steps loaded ahead
+    extern __shared__ double Bv[];
+    __shared__ double s_d[32], s_y[32], s_y2[32];  // pivots of a block and their reciprocals
+    __shared__ __align__(8) unsigned long long bar[8];
+    pdl_entry();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int nzc = L.b, nxc = L.a, N = nzc + 1;
+    const int ldab = 2 * kl + ku + 1, KD = ku + kl + 1, K = kl + ku;
+    cg::cluster_group cl = cg::this_cluster();
+    const int rank = (int)cl.block_rank();
+    if (tid < 8) mbar_init(smem_addr(&bar[tid]), 32);
+    for (int q = tid; rank == 0 && q < n; q += CS_THREADS) {
+        const int kq = q % N, iq = q / N;
+        Bv[q] = (iq >= 1 && iq <= nxc - 1 && kq >= 1 && kq <= nzc - 1)
+                    ? (double)ld_state(rhs + IX(L, iq, kq)) * __ldg(rowb + q)
+                    : 0.0;
+    }
+    __syncthreads();
+    auto nonzero = [](double x) { return (unsigned long long)(__double_as_longlong(x) << 1) != 0ull; };
+#define A_(rw, cl) ABg[(size_t)((rw) - 1) + (size_t)((cl) - 1) * ldab]
+    if (rank == 0) {
+        // rows b0 + o of the 16 steps from b0 on, o = tid + CS_THREADS u; column k's entry of row
+        // b0 + o is in f, loaded D steps before
+        double v[RR], f[D][RR];
+        int piv[D];
+        const double* from = &A_(KD + tid, 1);  // of the next fetch
+        int kf = 1;
+        auto fetch = [&](double(&g)[RR], int& p) {
+            const int i = (kf - 1) & (NP - 1), KM = min(kl, n - kf);
+            if (kf < n) p = __ldg(ipiv + kf - 1) - (kf - i);
+#pragma unroll
+            for (int u = 0; u < RR; u++) {
+                const int t = tid + CS_THREADS * u - i;
+                g[u] = (t >= 1 && t <= KM) ? __ldg(from + CS_THREADS * u) : 0.0;
+            }
+            from += i == NP - 1 ? ldab + NP - 1 : ldab - 1;
+            kf++;
+        };
+#pragma unroll
+        for (int q = 0; q < D; q++) {
+            piv[q] = 0;
+            fetch(f[q], piv[q]);
+        }
+        for (int b0 = 1; b0 < n; b0 += NP) {
+#pragma unroll
+            for (int u = 0; u < RR; u++) {
+                const int r = b0 + tid + CS_THREADS * u;
+                v[u] = r <= n ? Bv[r - 1] : 0.0;
+            }
+#pragma unroll 1
+            for (int i0 = 0; i0 < NP && b0 + i0 < n; i0 += D) {
+#pragma unroll
+                for (int q = 0; q < D; q++) {
+                    const int i = i0 + q, KM = min(kl, n - b0 - i), op = piv[q];
+                    double* ex = s_d + 2 * (q & 1);
+                    if (b0 + i < n) {
+#pragma unroll
+                        for (int u = 0; u < RR; u++)
+                            if (tid + CS_THREADS * u == op) ex[0] = v[u];
+                        if (tid == i) ex[1] = v[0];
+                        __syncthreads();
+                        const double top = ex[0], old = ex[1], temp = -top;
+#pragma unroll
+                        for (int u = 0; u < RR; u++) {
+                            const int o = tid + CS_THREADS * u, t = o - i;
+                            if (o == op) v[u] = old;
+                            if (o == i) v[u] = top;
+                            if (nonzero(temp) && t >= 1 && t <= KM) v[u] = v[u] + f[q][u] * temp;
+                        }
+                    }
+                    fetch(f[q], piv[q]);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < RR; u++) {
+                const int r = b0 + tid + CS_THREADS * u;
+                if (r <= n) Bv[r - 1] = v[u];
+            }
+            __syncthreads();
+        }
+    }
+    cl.sync();
+    double* B0 = cl.map_shared_rank(Bv, 0);
+    // the warp's rows: e - 32 - 32 g - lane, or e - lane where it solves.  Warps 0 and 1
+    // of CTA 0 take turns at that; the other follows with the next block, g = 0
+    const int g = rank + (CS_CL - 1) * warp;
+    const bool far = rank > 0 && g <= (K - 1) / 32;
+    // a block's columns at row e - 32 - 32 g - lane
+    double f[32];
+    auto fetch = [&](int e, int g) {
+        const int i = e - 32 - 32 * g - lane;
+        const double* from = &A_(K + 1 + i - e, e);
+#pragma unroll
+        for (int l = 0; l < 32; l++) {
+            f[l] = (i >= 1 && e - l - i <= K) ? __ldg(from) : 0.0;
+            from -= ldab - 1;
+        }
+    };
+    double v = 0.0;  // of the chain: lane l has row e - l
+    double pivot = 1.0;
+    bool dead = false;
+    if (rank == 0 && warp == 0) {
+        if (n - lane >= 1) {
+            v = Bv[n - lane - 1];
+            pivot = __ldg(&A_(K + 1, n - lane));
+        }
+    }
+    if (far) fetch(n, g);
+    for (int e = n, it = 0; e >= 1; e -= 32, it++) {
+        const int i = e - lane, i2 = i - 32;
+        if (rank == 0 && warp == (it & 1)) {
+            const unsigned ed = (unsigned)__double2hiint(pivot) >> 20 & 0x7ff;
+            const double y = ed - 600u > 846u ? 0.0 : 1.0 / pivot;
+            s_d[lane] = pivot;
+            s_y[lane] = y;
+            s_y2[lane] = fma(-y, pivot, 1.0) * y;
+            __syncwarp();
+            // the block's columns, four steps ahead: column e - l at row i
+            double a[4];
+            const double* from = &A_(K + 1 - lane, e);
+            auto near = [&](int l) {
+                const double x = (lane > l && i >= 1 && lane - l <= K) ? __ldg(from) : 0.0;
+                from -= ldab - 1;
+                return x;
+            };
+#pragma unroll
+            for (int q = 0; q < 4; q++) a[q] = near(q);
+#pragma unroll 1
+            for (int l0 = 0; l0 < 32; l0 += 4) {
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    const int l = l0 + q;
+                    const double bj = __shfl_sync(0xffffffffu, v, l);
+                    const double temp = solve_quot(bj, s_d[l], s_y[l], s_y2[l]);
+                    const double w = v - temp * a[q];
+                    v = nonzero(bj) && lane > l && lane - l <= K ? w : v;  // rows below the first are zero
+                    if (nonzero(bj) && lane == l) v = temp;
+                    a[q] = l + 4 < 32 ? near(l + 4) : 0.0;
+                }
+                if (lane >= l0 && lane < l0 + 4 && i >= 1) Bv[i - 1] = v;
+                mbar_arrive(smem_addr(&bar[l0 / 4]));
+            }
+        }
+        if (it > 0) cluster_wait();  // the block before is applied everywhere
+        if (rank == 0 && warp == (~it & 1)) {
+            v = i2 >= 1 ? Bv[i2 - 1] : 0.0;
+            pivot = i2 >= 1 ? __ldg(&A_(K + 1, i2)) : 1.0;
+            fetch(e, 0);
+#pragma unroll
+            for (int l0 = 0; l0 < 32; l0 += 4) {
+                int spins = 0;
+                while (!dead && !mbar_try_wait(smem_addr(&bar[l0 / 4]), it & 1)) dead = ++spins > CS_WAIT;
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    const int l = l0 + q;
+                    const double temp = e - l >= 1 ? Bv[e - l - 1] : 0.0;
+                    const double w = v - temp * f[l];
+                    v = (nonzero(temp) && i2 >= 1 && lane + 32 - l <= K) ? w : v;
+                }
+            }
+        }
+        cluster_arrive();
+        cluster_wait();  // this block is solved
+        const int r = i2 - 32 * g;
+        if (far) {
+            const double temps = i >= 1 ? B0[i - 1] : 0.0;
+            double w = r >= 1 ? B0[r - 1] : 0.0;
+#pragma unroll
+            for (int l = 0; l < 32; l++) {
+                const double temp = __shfl_sync(0xffffffffu, temps, l);
+                const double x = w - temp * f[l];
+                w = (nonzero(temp) && 32 + 32 * g + lane - l <= K) ? x : w;
+            }
+            if (r >= 1) B0[r - 1] = w;
+            fetch(e - 32, g);
+        }
+        cluster_arrive();
+    }
+    cluster_wait();
+    if (dead) atomicExch(timeout_flag, 1);
+    if (rank != 0) return;
+#undef A_
+    for (int q = tid; q < n; q += CS_THREADS) {
+        const int kq = q % N, iq = q / N;
+        if (iq >= 1 && iq <= nxc - 1 && kq >= 1 && kq <= nzc - 1) store_stream<TR>(L, err, iq, kq, (TR)Bv[q], Vbc);
+    }
+    pdl_done();
+}
+// The same with one warp and no rows in registers: bands and vectors beyond the kernel
+// above (kl > 496, or a vector that leaves no room for the pivots).
 template <typename TR>
-__global__ void __launch_bounds__(256) k_coarse_solve(Lay L, const double* __restrict__ ABg,
-                                                      const int* __restrict__ ipiv, const double* __restrict__ rowb,
-                                                      const TR* rhs, int n, int kl, int ku, TR* err, int Vbc) {
+__global__ void __launch_bounds__(256) k_coarse_solve_wide(Lay L, const double* __restrict__ ABg,
+                                                           const int* __restrict__ ipiv,
+                                                           const double* __restrict__ rowb, const TR* rhs, int n,
+                                                           int kl, int ku, TR* err, int Vbc) {
     extern __shared__ double Bv[];
     pdl_entry();
     const int tid = threadIdx.x, lane = tid & 31;
@@ -1228,84 +1449,7 @@ __global__ void __launch_bounds__(256) k_coarse_solve(Lay L, const double* __res
     }
     __syncthreads();
 #define A_(rw, cl) ABg[(size_t)((rw) - 1) + (size_t)((cl) - 1) * ldab]
-    if (tid < 32 && kl <= 32 * CS_FW && K <= 32 * CS_BW) {
-        // the band column of the next step is loaded while this step runs
-        double nf[CS_FW];
-        int npiv = (n >= 2) ? __ldg(ipiv) : 0;
-        {
-            const int LM = min(kl, n - 1);
-#pragma unroll
-            for (int u = 0; u < CS_FW; u++) {
-                const int t = 1 + lane + 32 * u;
-                nf[u] = (n >= 2 && t <= LM) ? __ldg(&A_(KD + t, 1)) : 0.0;
-            }
-        }
-        for (int jj = 1; jj <= n - 1; jj++) {
-            const int LM = min(kl, n - jj);
-            double cf[CS_FW];
-#pragma unroll
-            for (int u = 0; u < CS_FW; u++) cf[u] = nf[u];
-            const int Lr = npiv;
-            if (jj + 1 <= n - 1) {
-                const int LM1 = min(kl, n - jj - 1);
-                npiv = __ldg(ipiv + jj);
-#pragma unroll
-                for (int u = 0; u < CS_FW; u++) {
-                    const int t = 1 + lane + 32 * u;
-                    nf[u] = (t <= LM1) ? __ldg(&A_(KD + t, jj + 1)) : 0.0;
-                }
-            }
-            if (Lr != jj) {
-                if (lane == 0) { const double t0 = Bv[Lr - 1]; Bv[Lr - 1] = Bv[jj - 1]; Bv[jj - 1] = t0; }
-                __syncwarp();
-            }
-            const double temp = -Bv[jj - 1];
-            if (temp != 0.0) {
-#pragma unroll
-                for (int u = 0; u < CS_FW; u++) {
-                    const int t = 1 + lane + 32 * u;
-                    if (t <= LM) Bv[jj + t - 1] = Bv[jj + t - 1] + cf[u] * temp;
-                }
-            }
-            __syncwarp();
-        }
-        double nb[CS_BW], nd = __ldg(&A_(K + 1, n));
-        {
-            const int jj = n, Lc = K + 1 - jj;
-#pragma unroll
-            for (int u = 0; u < CS_BW; u++) {
-                const int i = jj - 1 - lane - 32 * u;
-                nb[u] = (i >= max(1, jj - K)) ? __ldg(&A_(Lc + i, jj)) : 0.0;
-            }
-        }
-        for (int jj = n; jj >= 1; jj--) {
-            double cb[CS_BW];
-#pragma unroll
-            for (int u = 0; u < CS_BW; u++) cb[u] = nb[u];
-            const double dj = nd;
-            if (jj - 1 >= 1) {
-                const int j1 = jj - 1, Lc1 = K + 1 - j1;
-                nd = __ldg(&A_(K + 1, j1));
-#pragma unroll
-                for (int u = 0; u < CS_BW; u++) {
-                    const int i = j1 - 1 - lane - 32 * u;
-                    nb[u] = (i >= max(1, j1 - K)) ? __ldg(&A_(Lc1 + i, j1)) : 0.0;
-                }
-            }
-            const double bj = Bv[jj - 1];
-            if (bj != 0.0) {
-                const double temp = bj / dj;
-                __syncwarp();
-                if (lane == 0) Bv[jj - 1] = temp;
-#pragma unroll
-                for (int u = 0; u < CS_BW; u++) {
-                    const int i = jj - 1 - lane - 32 * u;
-                    if (i >= max(1, jj - K)) Bv[i - 1] = Bv[i - 1] - temp * cb[u];
-                }
-            }
-            __syncwarp();
-        }
-    } else if (tid < 32) {
+    if (tid < 32) {
         for (int jj = 1; jj <= n - 1; jj++) {
             const int LM = min(kl, n - jj);
             const int Lr = __ldg(ipiv + jj - 1);
@@ -1338,19 +1482,39 @@ __global__ void __launch_bounds__(256) k_coarse_solve(Lay L, const double* __res
     }
     pdl_done();
 }
-void launch_coarse_solve(cudaStream_t s, const Level& lv, const double* band, const int* ipiv, const double* rowb,
-                         int n, int kl, int ku, double* err, int Vbc) {
+template <typename TR>
+static void coarse_solve(cudaStream_t s, const Lay& L, const double* band, const int* ipiv, const double* rowb,
+                         const TR* rhs, int n, int kl, int ku, TR* err, int Vbc, int* timeout_flag) {
     const size_t sm = sizeof(double) * (size_t)n;
-    cudaFuncSetAttribute(k_coarse_solve<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    launch_pdl(k_coarse_solve<double>, 1, 256, sm, s, lv.L, band, ipiv, rowb, (const double*)lv.rhs, n, kl, ku, err,
-               Vbc); tc_note_launch();
+    auto go = [&](auto kernel, int ctas, auto... more) {
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(ctas, 1, 1);
+        cfg.blockDim = dim3(CS_THREADS, 1, 1);
+        cfg.dynamicSmemBytes = sm;
+        cfg.stream = s;
+        cudaLaunchAttribute at[2];
+        at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[0].val.programmaticStreamSerializationAllowed = 1;
+        at[1].id = cudaLaunchAttributeClusterDimension;
+        at[1].val.clusterDim.x = ctas;
+        at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = ctas > 1 ? 2 : 1;
+        cudaLaunchKernelEx(&cfg, kernel, L, band, ipiv, rowb, rhs, n, kl, ku, err, Vbc, more...); tc_note_launch();
+    };
+    // two rows per thread above kl = 240: the 16 steps between re-basings reach kl + 16 rows
+    if (kl > CS_MAXKL || sm > 226 * 1024) go(k_coarse_solve_wide<TR>, 1);
+    else if (kl <= 240) go(k_coarse_solve<TR, 1>, CS_CL, timeout_flag);
+    else go(k_coarse_solve<TR, 2>, CS_CL, timeout_flag);
+}
+void launch_coarse_solve(cudaStream_t s, const Level& lv, const double* band, const int* ipiv, const double* rowb,
+                         int n, int kl, int ku, double* err, int Vbc, int* timeout_flag) {
+    coarse_solve(s, lv.L, band, ipiv, rowb, (const double*)lv.rhs, n, kl, ku, err, Vbc, timeout_flag);
 }
 void launch_coarse_solve32(cudaStream_t s, const Level& lv, const double* band, const int* ipiv, const double* rowb,
-                           int n, int kl, int ku, float* err, int Vbc) {
-    const size_t sm = sizeof(double) * (size_t)n;
-    cudaFuncSetAttribute(k_coarse_solve<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    launch_pdl(k_coarse_solve<float>, 1, 256, sm, s, lv.L, band, ipiv, rowb, (const float*)lv.rhs32, n, kl, ku, err,
-               Vbc); tc_note_launch();
+                           int n, int kl, int ku, float* err, int Vbc, int* timeout_flag) {
+    coarse_solve(s, lv.L, band, ipiv, rowb, (const float*)lv.rhs32, n, kl, ku, err, Vbc, timeout_flag);
 }
 
 __global__ void k_copy(double* dst, const double* src, size_t n) {

@@ -42,6 +42,9 @@ __device__ __forceinline__ void mbar_arrive_expect(uint32_t a, int bytes) {
     asm volatile("{ .reg .b64 st; mbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1; }" ::"r"(a), "r"(bytes)
                  : "memory");
 }
+__device__ __forceinline__ void mbar_arrive(uint32_t a) {
+    asm volatile("{ .reg .b64 st; mbarrier.arrive.shared::cta.b64 st, [%0]; }" ::"r"(a) : "memory");
+}
 __device__ __forceinline__ bool mbar_try_wait(uint32_t a, int parity) {
     uint32_t ok;
     asm volatile(
