@@ -398,12 +398,62 @@ void launch_strain(cudaStream_t s, const Lay& L, const Phys& P, const double* u,
 // [13] Nu denominator, [14] Nu_bot numerator, [15..18] q1..q4
 // ---------------------------------------------------------------------------
 #define NROWINT 7
-// The integrands are evaluated in parallel into shared memory, CH columns at
-// a time; one thread per running sum then adds them serially with the
-// reference's expression, so every sum takes the same operations in the same
-// order as the serial loop (the values are the same doubles).
-constexpr int kStatCH = 512;
+// The integrands and then the trapezoids are evaluated in parallel into shared
+// memory, kStatCH at a time; one lane per running sum adds them serially, so every sum
+// takes the same operations in the same order as the serial loop (the values are the
+// same doubles).
+//
+// What bounds it: the serial additions, 68 cycles each (an FP64 operation of a warp takes
+// its scheduler 64).  The adding warp therefore does nothing else, the six warps of the
+// other schedulers evaluate the next trapezoids meanwhile, and the sums along the top and
+// bottom rows run in a block of their own beside the rows'.  With the whole expression in
+// the serial loop and those sums after the rows', the two kernels took 44 + 57 us on a
+// 256x64 grid (cold caches), now 19 + 8.
+constexpr int kStatCH = 128;
 constexpr int kStatThreads = 256;
+constexpr int kStatEval = kStatThreads / 32 * 24;  // threads that evaluate: warps 1-3 and 5-7
+
+// Trapezoid sums of NQ functions f(q, i), i = 0..n, with weights wt(i) and spacing h, left
+// to right: returns to lane l of warp 0 the sum of function l, and to lane NQ + l that
+// from i = from on.  Uses the whole block; f and wt only where on(q).
+template <int NQ, typename On, typename F, typename W>
+__device__ __forceinline__ double trapezoid_sums(int n, int from, double h, On on, F f, W wt) {
+    __shared__ double fv[NQ][kStatCH + 1], term[2][NQ][kStatCH];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, chunks = (n + kStatCH - 1) / kStatCH;
+    const int q0 = lane < NQ ? lane : lane - NQ, start = lane < NQ ? 0 : from;
+    const bool adds = warp == 0 && lane < 2 * NQ && on(q0);
+    double sum = 0.0;
+    for (int c = 0; c <= chunks; c++) {
+        const int e0 = threadIdx.x - 32 * (1 + (warp > 4));
+        if ((warp & 3) != 0 && c < chunks) {
+            const int i0 = c * kStatCH, m = min(kStatCH, n - i0);
+            for (int e = e0; e < NQ * (kStatCH + 1); e += kStatEval) {
+                const int q = e / (kStatCH + 1), j = e % (kStatCH + 1);
+                if (j <= m && on(q)) fv[q][j] = f(q, i0 + j) * wt(i0 + j);
+            }
+            asm volatile("bar.sync 1, %0;" ::"n"(kStatEval) : "memory");
+            for (int e = e0; e < NQ * kStatCH; e += kStatEval) {
+                const int q = e / kStatCH, j = e % kStatCH;
+                if (j < m && on(q)) term[c & 1][q][j] = 0.5 * (fv[q][j] + fv[q][j + 1]) * h;
+            }
+        }
+        if (adds && c > 0) {
+            const int i0 = (c - 1) * kStatCH, m = min(kStatCH, n - i0);
+            const double* t = term[(c - 1) & 1][q0];
+            int j = max(0, start - i0);
+            for (; j + 8 <= m; j += 8) {
+                double v[8];
+#pragma unroll
+                for (int u = 0; u < 8; u++) v[u] = t[j + u];
+#pragma unroll
+                for (int u = 0; u < 8; u++) sum = sum + v[u];
+            }
+            for (; j < m; j++) sum = sum + t[j];
+        }
+        __syncthreads();
+    }
+    return sum;
+}
 
 // integrand q at (i, k): 0..3 C by type, 4 u^2+w^2, 5 T, 6 RaT/conduct/vis
 __device__ __forceinline__ double stat_integrand(const Lay& L, const Phys& P, const double* __restrict__ T,
@@ -422,133 +472,49 @@ __device__ __forceinline__ bool stat_row_active(const Phys& P, int q) {
     return true;
 }
 
-// integrate1Dx of every row k (basics.f90 trapezoid, left to right): one
-// block per row
+// integrate1Dx of every row k (basics.f90 trapezoid, left to right): one block per
+// row; the last block: the top-row and Nusselt integrals along x, the corner fluxes
+// and the top-row strain maximum
 __global__ void __launch_bounds__(kStatThreads) k_stats_rows(Lay L, Phys P, const double* __restrict__ T,
                                                              const double* __restrict__ u,
                                                              const double* __restrict__ w,
                                                              const double* __restrict__ cd,
                                                              const double* __restrict__ vis, CPtrs Cn,
-                                                             double* __restrict__ rows) {
-    __shared__ double fv[NROWINT][kStatCH + 1];
-    const int k = blockIdx.x;
-    const int nx = L.a, nz = L.b;
-    const int t = threadIdx.x;
-    double fint = 0.0;
-    for (int c0 = 0; c0 < nx; c0 += kStatCH) {
-        const int n = min(kStatCH, nx - c0);  // sums over i = c0..c0+n-1 use f(c0..c0+n)
-        for (int e = t; e < NROWINT * (n + 1); e += blockDim.x) {
-            const int q = e / (n + 1), j = e % (n + 1);
-            fv[q][j] = stat_row_active(P, q) ? stat_integrand(L, P, T, u, w, cd, vis, Cn, q, c0 + j, k) : 0.0;
-        }
-        __syncthreads();
-        if (t < NROWINT && stat_row_active(P, t)) {
-            double fprev = fv[t][0];
-            double xprev = P.M.on ? mt(P.M.xr, c0) : 1.0;
-            for (int j = 0; j < n; j++) {
-                const double fn = fv[t][j + 1];
-                const double xn = P.M.on ? mt(P.M.xr, c0 + j + 1) : 1.0;
-                fint = fint + 0.5 * (fprev * xprev + fn * xn) * P.dr;
-                fprev = fn;
-                xprev = xn;
-            }
-        }
-        __syncthreads();
+                                                             const double* __restrict__ st,
+                                                             double* __restrict__ rows, DevScalars* ds) {
+    const int k = blockIdx.x, nx = L.a, nz = L.b, t = threadIdx.x;
+    auto wt = [&](int i) { return P.M.on ? mt(P.M.xr, i) : 1.0; };
+    if (k <= nz) {
+        auto on = [&](int q) { return stat_row_active(P, q); };
+        auto f = [&](int q, int i) { return stat_integrand(L, P, T, u, w, cd, vis, Cn, q, i, k); };
+        const double sum = trapezoid_sums<NROWINT>(nx, 0, P.dr, on, f, wt);
+        if (t < NROWINT) rows[(size_t)t * (nz + 1) + k] = on(t) ? sum : 0.0;
+        return;
     }
-    if (t < NROWINT) rows[(size_t)t * (nz + 1) + k] = stat_row_active(P, t) ? fint : 0.0;
-}
-
-// integrate1Dz of the row integrals (from k = 0, and from kent for the C
-// types), the top-row and Nusselt integrals along x, the corner fluxes and
-// the top-row strain maximum.  One block.
-__global__ void __launch_bounds__(kStatThreads) k_stats_final(Lay L, Phys P, int kent,
-                                                              const double* __restrict__ rows,
-                                                              const double* __restrict__ T,
-                                                              const double* __restrict__ u,
-                                                              const double* __restrict__ w,
-                                                              const double* __restrict__ cd,
-                                                              const double* __restrict__ st, DevScalars* ds) {
-    __shared__ double fv[NROWINT][kStatCH + 1];
-    __shared__ double red[kStatThreads / 32];
-    const int nx = L.a, nz = L.b;
-    const int t = threadIdx.x;
+    // the mobility integrand and the Nusselt integrands: values 0 top(i), 1 -cd*dT/dz at
+    // the top, 2 T at the bottom, 3 -cd*dT/dz at the bottom
+    const bool rat = (P.RaT != 0.0);
     const size_t ld = (size_t)L.ld;
-    // z-integrals: thread t < NROWINT sums row t from k = 0; thread
-    // NROWINT + q (q < 4) sums C type q from kent
-    {
-        const int q = (t < NROWINT) ? t : t - NROWINT;
-        const int k0 = (t < NROWINT) ? 0 : kent;
-        bool active = (t < NROWINT + 4);
-        if (q < 4 && q >= P.ntype) active = false;
-        if (t >= NROWINT && q >= 4) active = false;
-        double fint = 0.0;
-        for (int c0 = 0; c0 < nz; c0 += kStatCH) {
-            const int n = min(kStatCH, nz - c0);
-            for (int e = t; e < NROWINT * (n + 1); e += blockDim.x) {
-                const int qq = e / (n + 1), j = e % (n + 1);
-                fv[qq][j] = rows[(size_t)qq * (nz + 1) + c0 + j];
-            }
-            __syncthreads();
-            if (active) {
-                for (int j = 0; j < n; j++) {
-                    if (c0 + j < k0) continue;
-                    const double za = P.M.on ? mt(P.M.zs, c0 + j) : 1.0, zb = P.M.on ? mt(P.M.zs, c0 + j + 1) : 1.0;
-                    fint = fint + 0.5 * (fv[q][j] * za + fv[q][j + 1] * zb) * P.ds;
-                }
-            }
-            __syncthreads();
-        }
-        if (active) {
-            const int slot = (t < NROWINT) ? ((q < 4) ? q : (q - 4 + 8)) : (4 + q);
-            ds->integ[slot] = fint;
+    const double zs_top = P.M.on ? mt(P.M.zs, nz) : 1.0, zs_bot = P.M.on ? mt(P.M.zs, 0) : 1.0;
+    auto dz = [&](size_t x) { return -0.5 * T[x - ld] + 0.5 * T[x + ld]; };
+    auto on = [&](int q) { return q == 0 || rat; };
+    auto f = [&](int q, int i) {
+        const size_t x = IX(L, i, q < 2 ? nz : 0);
+        if (q == 0) return u[x] * u[x] + w[x] * w[x];
+        if (q == 2) return T[x];
+        return -cd[x] * (dz(x) / P.ds / (q == 1 ? zs_top : zs_bot));
+    };
+    const double sum = trapezoid_sums<4>(nx, 0, P.dr, on, f, wt);
+    if (t < 4) {
+        ds->integ[11 + t] = on(t) ? sum : 0.0;
+        if (rat) {
+            // corners (0, nz), (nx, nz), (nx, 0), (0, 0)
+            const size_t x = IX(L, t == 0 || t == 3 ? 0 : nx, t < 2 ? nz : 0);
+            ds->integ[15 + t] = -(cd[x] * dz(x)) / P.ds / (t < 2 ? zs_top : zs_bot);
         }
     }
-    // top-row mobility integrand and the Nusselt integrands: values 0 top(i),
-    // 1 -cd*dT/dz at the top, 2 T at the bottom, 3 -cd*dT/dz at the bottom;
-    // thread j < 4 keeps sum j
-    {
-        const bool rat = (P.RaT != 0.0);
-        const double zs_top = P.M.on ? mt(P.M.zs, nz) : 1.0, zs_bot = P.M.on ? mt(P.M.zs, 0) : 1.0;
-        double acc = 0.0;
-        for (int c0 = 0; c0 < nx; c0 += kStatCH) {
-            const int n = min(kStatCH, nx - c0);
-            for (int e = t; e < 4 * (n + 1); e += blockDim.x) {
-                const int q = e / (n + 1), i = c0 + e % (n + 1);
-                double v = 0.0;
-                if (q == 0) {
-                    const size_t x = IX(L, i, nz);
-                    v = u[x] * u[x] + w[x] * w[x];
-                } else if (rat && q == 1) {
-                    const size_t x = IX(L, i, nz);
-                    v = -cd[x] * ((-0.5 * T[x - ld] + 0.5 * T[x + ld]) / P.ds / zs_top);
-                } else if (rat && q == 2) {
-                    v = T[IX(L, i, 0)];
-                } else if (rat && q == 3) {
-                    const size_t x = IX(L, i, 0);
-                    v = -cd[x] * ((-0.5 * T[x - ld] + 0.5 * T[x + ld]) / P.ds / zs_bot);
-                }
-                fv[q][e % (n + 1)] = v;
-            }
-            __syncthreads();
-            if (t < 4 && (t == 0 || rat)) {
-                for (int j = 0; j < n; j++) {
-                    const double xa = P.M.on ? mt(P.M.xr, c0 + j) : 1.0, xb = P.M.on ? mt(P.M.xr, c0 + j + 1) : 1.0;
-                    acc = acc + 0.5 * (fv[t][j] * xa + fv[t][j + 1] * xb) * P.dr;
-                }
-            }
-            __syncthreads();
-        }
-        if (t < 4) ds->integ[11 + t] = acc;
-    }
-    if (t == 0 && P.RaT != 0.0) {
-        auto dz = [&](int i, int kk) { size_t x = IX(L, i, kk); return -0.5 * T[x - ld] + 0.5 * T[x + ld]; };
-        const double zt = P.M.on ? mt(P.M.zs, nz) : 1.0, zb = P.M.on ? mt(P.M.zs, 0) : 1.0;
-        ds->integ[15] = -(cd[IX(L, 0, nz)] * dz(0, nz)) / P.ds / zt;
-        ds->integ[16] = -(cd[IX(L, nx, nz)] * dz(nx, nz)) / P.ds / zt;
-        ds->integ[17] = -(cd[IX(L, nx, 0)] * dz(nx, 0)) / P.ds / zb;
-        ds->integ[18] = -(cd[IX(L, 0, 0)] * dz(0, 0)) / P.ds / zb;
-    }
-    // top-row strain maximum (fmax is exact and order-free)
+    // (fmax is exact and order-free)
+    __shared__ double red[kStatThreads / 32];
     double smax = -INFINITY;
     for (int i = t; i <= nx; i += blockDim.x) smax = fmax(smax, st[IX(L, i, nz)]);
     for (int o = 16; o > 0; o >>= 1) smax = fmax(smax, __shfl_down_sync(0xffffffffu, smax, o));
@@ -558,6 +524,26 @@ __global__ void __launch_bounds__(kStatThreads) k_stats_final(Lay L, Phys P, int
         double m = -INFINITY;
         for (int j = 0; j < (int)(blockDim.x >> 5); j++) m = fmax(m, red[j]);
         ds->strain_max = m;
+    }
+}
+
+// integrate1Dz of the row integrals: from k = 0, and from kent for the C types.  One
+// block; it also clears what k_nempty_stats counts.
+__global__ void __launch_bounds__(kStatThreads) k_stats_final(Lay L, Phys P, int kent,
+                                                              const double* __restrict__ rows, DevScalars* ds) {
+    const int nz = L.b, t = threadIdx.x;
+    auto on = [&](int q) { return q >= 4 || q < P.ntype; };
+    auto f = [&](int q, int k) { return rows[(size_t)q * (nz + 1) + k]; };
+    auto wt = [&](int k) { return P.M.on ? mt(P.M.zs, k) : 1.0; };
+    const double sum = trapezoid_sums<NROWINT>(nz, kent, P.ds, on, f, wt);
+    if (t < NROWINT) {
+        if (on(t)) ds->integ[t < 4 ? t : t - 4 + 8] = sum;
+    } else if (t < NROWINT + 4) {
+        if (on(t - NROWINT)) ds->integ[4 + t - NROWINT] = sum;
+    } else if (t == 31) {
+        ds->nempty_min = 0x7fffffff;
+        ds->nempty_max = -0x7fffffff;
+        ds->empty_cells = 0;
     }
 }
 __global__ void k_nempty_stats(Lay L, Range2 r, const int* __restrict__ ne, DevScalars* ds) {
@@ -579,21 +565,15 @@ __global__ void k_nempty_stats(Lay L, Range2 r, const int* __restrict__ ne, DevS
         atomicAdd(&ds->empty_cells, szero);
     }
 }
-__global__ void k_nempty_init(DevScalars* ds) {
-    ds->nempty_min = 0x7fffffff;
-    ds->nempty_max = -0x7fffffff;
-    ds->empty_cells = 0;
-}
 void launch_stats(cudaStream_t s, const Lay& L, const Phys& P, int kent, const double* T, const double* u,
                   const double* w, const double* conduct, const double* vis, const double* strain,
                   const double* const* Cnew, const int* nempty, double* rows, DevScalars* ds) {
     CPtrs C{};
     for (int j = 0; j < P.ntype && j < TC_MAX_TYPES; j++) C.p[j] = Cnew[j];
-    k_stats_rows<<<L.b + 1, kStatThreads, 0, s>>>(L, P, T, u, w, conduct, vis, C, rows); tc_note_launch();
-    k_stats_final<<<1, kStatThreads, 0, s>>>(L, P, kent, rows, T, u, w, conduct, strain, ds); tc_note_launch();
+    k_stats_rows<<<L.b + 2, kStatThreads, 0, s>>>(L, P, T, u, w, conduct, vis, C, strain, rows, ds); tc_note_launch();
+    k_stats_final<<<1, kStatThreads, 0, s>>>(L, P, kent, rows, ds); tc_note_launch();
     if (P.comp == 1 || P.tracer == 1) {
         Range2 r{0, L.a, 0, L.b};
-        k_nempty_init<<<1, 1, 0, s>>>(ds); tc_note_launch();
         k_nempty_stats<<<grid_for(r), dim3(BX, BY), 0, s>>>(L, r, nempty, ds); tc_note_launch();
     }
 }
