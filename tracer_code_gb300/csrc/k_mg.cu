@@ -1113,65 +1113,143 @@ void launch_coarse_lu(cudaStream_t s, double* band, int* ipiv, int n, int kl, in
     k_coarse_lu_global<<<1, 512, 0, s>>>(band, ipiv, n, kl, ku, &ds->lu_info); tc_note_launch();
 }
 
+// RN(x / d) from y + y2 = 1 / d to twice the precision: a quotient within one ulp, and
+// Markstein's correction with its exact remainder (IBM J. Res. Dev. 34, 1990).  y = 0: d
+// is near the ends of the range.
+__device__ __forceinline__ double solve_quot(double x, double d, double y, double y2) {
+    const double q0 = fma(x, y, x * y2);
+    double q = fma(fma(-q0, d, x), y, q0);
+    const unsigned hi = (unsigned)__double2hiint(x);
+    if ((hi >> 20 & 0x7ff) - 600u > 846u || __double2hiint(y) == 0) {
+        if (((hi << 1) | (unsigned)__double2loint(x)) != 0) q = x / d;  // 0 where x is
+    }
+    return q;
+}
+__device__ __forceinline__ void solve_recip(double d, double& y, double& y2) {
+    const unsigned ed = (unsigned)__double2hiint(d) >> 20 & 0x7ff;
+    y = ed - 600u > 846u ? 0.0 : 1.0 / d;
+    y2 = fma(-y, d, 1.0) * y;
+}
+
 // Explicit inverse of the factored coarse matrix: column j of A^-1 is the
 // DGBTRS solve (row interchanges + L solve, then dtbsv) of the unit vector
-// e_j.  One warp per column; the band is staged in shared memory when it
-// fits.  Stored row-major (Ainv[p*n + q]) for the coalesced products below.
-__global__ void k_coarse_inverse(const double* __restrict__ ABg, const int* __restrict__ ipiv_g, int n, int kl,
-                                 int ku, int in_smem, double* __restrict__ Ainv, double* __restrict__ Bscratch) {
+// e_j.  One warp per column, the vector in shared memory.  Stored row-major
+// (Ainv[p*n + q]) for the coalesced products below.
+//
+// What bounds it: the chain of FP64 operations of a column, 64 cycles each, so each
+// warp has a scheduler of its own (four per CTA) and the pivots' reciprocals, formed
+// once, replace most of each division.  The band comes from L1/L2, FW rows per lane below
+// the diagonal and 2 FW above, loaded four steps ahead.  286 -> 180 us at n = 297,
+// kl = 20 (before: eight warps per CTA, divisions, the band staged in shared memory where
+// it fits); n = 289, kl = 34: 346 us without the loads ahead, 239 with them.
+#define CI_WARPS 4
+template <int FW>
+__global__ void __launch_bounds__(32 * CI_WARPS) k_coarse_inverse(const double* __restrict__ ABg,
+                                                                  const int* __restrict__ ipiv, int n, int kl, int ku,
+                                                                  double* __restrict__ Ainv) {
+    constexpr int D = 4;  // steps loaded ahead
     extern __shared__ double sm[];
     const int ldab = 2 * kl + ku + 1, KD = ku + kl + 1, K = kl + ku;
-    const size_t tot = (size_t)ldab * n;
-    const int tid = threadIdx.x, nth = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nth >> 5;
-    const double* AB = in_smem ? sm : ABg;
-    int* ipv = (int*)(sm + (in_smem ? tot : 0));
-    double* Bw = in_smem ? (double*)(ipv + ((n + 1) & ~1)) + (size_t)warp * n : Bscratch + ((size_t)blockIdx.x * nw + warp) * n;
-    if (in_smem) {
-        for (size_t t = tid; t < tot; t += nth) sm[t] = ABg[t];
-        for (int t = tid; t < n; t += nth) ipv[t] = ipiv_g[t];
+    const int tid = threadIdx.x, nth = 32 * CI_WARPS, lane = tid & 31, warp = tid >> 5;
+    double *sd = sm, *sy = sd + n, *sy2 = sy + n, *Bw = sy2 + n + (size_t)warp * n;
+#define A_(rw, cl) ABg[(size_t)((rw) - 1) + (size_t)((cl) - 1) * ldab]
+    for (int t = tid; t < n; t += nth) {
+        sd[t] = __ldg(&A_(K + 1, t + 1));
+        solve_recip(sd[t], sy[t], sy2[t]);
     }
     __syncthreads();
-    const int* piv = in_smem ? ipv : ipiv_g;
-    const int j = blockIdx.x * nw + warp + 1;  // column of A^-1 (1-based)
+    const int j = blockIdx.x * CI_WARPS + warp + 1;  // column of A^-1 (1-based)
     if (j > n) return;
-#define A_(rw, cl) AB[(size_t)((rw) - 1) + (size_t)((cl) - 1) * ldab]
+    auto nonzero = [](double x) { return (unsigned long long)(__double_as_longlong(x) << 1) != 0ull; };
     for (int t = lane; t < n; t += 32) Bw[t] = (t == j - 1) ? 1.0 : 0.0;
     __syncwarp();
-    for (int jj = 1; jj <= n - 1; jj++) {
-        const int LM = min(kl, n - jj);
-        const int Lr = piv[jj - 1];
-        if (Lr != jj) {
-            if (lane == 0) { double t0 = Bw[Lr - 1]; Bw[Lr - 1] = Bw[jj - 1]; Bw[jj - 1] = t0; }
-            __syncwarp();
+    {
+        double f[D][FW];
+        int pv[D];
+        auto fetch = [&](int jj, int q) {
+            if (jj > n - 1) return;
+            pv[q] = __ldg(ipiv + jj - 1);
+#pragma unroll
+            for (int u = 0; u < FW; u++) {
+                const int t = 1 + lane + 32 * u;
+                f[q][u] = t <= min(kl, n - jj) ? __ldg(&A_(KD + t, jj)) : 0.0;
+            }
+        };
+        const int first = max(1, j - kl);  // earlier steps interchange and add zeros
+#pragma unroll
+        for (int q = 0; q < D; q++) fetch(first + q, q);
+        for (int j0 = first; j0 <= n - 1; j0 += D) {
+#pragma unroll
+            for (int q = 0; q < D; q++) {
+                const int jj = j0 + q;
+                if (jj > n - 1) break;
+                const int LM = min(kl, n - jj), Lr = pv[q];
+                const double top = Bw[Lr - 1];
+                if (Lr != jj) {
+                    __syncwarp();
+                    if (lane == 0) { Bw[Lr - 1] = Bw[jj - 1]; Bw[jj - 1] = top; }
+                    __syncwarp();
+                }
+                const double temp = -top;
+                if (nonzero(temp)) {
+#pragma unroll
+                    for (int u = 0; u < FW; u++) {
+                        const int t = 1 + lane + 32 * u;
+                        if (t <= LM) Bw[jj + t - 1] = Bw[jj + t - 1] + f[q][u] * temp;
+                    }
+                    for (int t = 1 + lane + 32 * FW; t <= LM; t += 32)
+                        Bw[jj + t - 1] = Bw[jj + t - 1] + __ldg(&A_(KD + t, jj)) * temp;
+                }
+                __syncwarp();
+                fetch(jj + D, q);
+            }
         }
-        const double temp = -Bw[jj - 1];
-        if (temp != 0.0)
-            for (int t = 1 + lane; t <= LM; t += 32) Bw[jj + t - 1] = Bw[jj + t - 1] + A_(KD + t, jj) * temp;
-        __syncwarp();
     }
-    for (int jj = n; jj >= 1; jj--) {
-        const double bj = Bw[jj - 1];
-        if (bj != 0.0) {
-            const int Lc = K + 1 - jj;
-            const double temp = bj / A_(K + 1, jj);
-            __syncwarp();
-            if (lane == 0) Bw[jj - 1] = temp;
-            for (int i = jj - 1 - lane; i >= max(1, jj - K); i -= 32) Bw[i - 1] = Bw[i - 1] - temp * A_(Lc + i, jj);
+    double g[D][2 * FW];
+    auto fetch = [&](int jj, int q) {
+        if (jj < 1) return;
+#pragma unroll
+        for (int u = 0; u < 2 * FW; u++) {
+            const int i = jj - 1 - lane - 32 * u;
+            g[q][u] = i >= max(1, jj - K) ? __ldg(&A_(K + 1 - jj + i, jj)) : 0.0;
         }
-        __syncwarp();
+    };
+#pragma unroll
+    for (int q = 0; q < D; q++) fetch(n - q, q);
+    for (int j0 = n; j0 >= 1; j0 -= D) {
+#pragma unroll
+        for (int q = 0; q < D; q++) {
+            const int jj = j0 - q;
+            if (jj < 1) break;
+            const double bj = Bw[jj - 1];
+            if (nonzero(bj)) {
+                const double temp = solve_quot(bj, sd[jj - 1], sy[jj - 1], sy2[jj - 1]);
+                __syncwarp();
+                if (lane == 0) Bw[jj - 1] = temp;
+#pragma unroll
+                for (int u = 0; u < 2 * FW; u++) {
+                    const int i = jj - 1 - lane - 32 * u;
+                    if (i >= max(1, jj - K)) Bw[i - 1] = Bw[i - 1] - temp * g[q][u];
+                }
+                for (int i = jj - 1 - lane - 64 * FW; i >= max(1, jj - K); i -= 32)
+                    Bw[i - 1] = Bw[i - 1] - temp * __ldg(&A_(K + 1 - jj + i, jj));
+            }
+            __syncwarp();
+            fetch(jj - D, q);
+        }
     }
 #undef A_
     for (int p = lane; p < n; p += 32) Ainv[(size_t)p * n + (j - 1)] = Bw[p];
 }
-void launch_coarse_inverse(cudaStream_t s, const double* band, const int* ipiv, int n, int kl, int ku, double* Ainv,
-                           double* bscratch) {
-    const int nw = 8;
-    const size_t band_bytes = sizeof(double) * (size_t)(2 * kl + ku + 1) * n;
-    const size_t smem = band_bytes + sizeof(int) * (size_t)((n + 1) & ~1) + sizeof(double) * (size_t)nw * n;
-    const int in_smem = smem <= 200 * 1024 ? 1 : 0;
-    const size_t sm = in_smem ? smem : 0;
-    if (in_smem) cudaFuncSetAttribute(k_coarse_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    k_coarse_inverse<<<(n + nw - 1) / nw, 32 * nw, sm, s>>>(band, ipiv, n, kl, ku, in_smem, Ainv, bscratch); tc_note_launch();
+void launch_coarse_inverse(cudaStream_t s, const double* band, const int* ipiv, int n, int kl, int ku, double* Ainv) {
+    const size_t sm = sizeof(double) * (3 + CI_WARPS) * (size_t)n;
+    auto go = [&](auto kernel) {
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        kernel<<<(n + CI_WARPS - 1) / CI_WARPS, 32 * CI_WARPS, sm, s>>>(band, ipiv, n, kl, ku, Ainv); tc_note_launch();
+    };
+    if (kl <= 32) go(k_coarse_inverse<1>);
+    else if (kl <= 64) go(k_coarse_inverse<2>);
+    else go(k_coarse_inverse<4>);
 }
 
 // Coarsest-level solve as x = A^-1 (RowB .* RHS) (Compute_coarse_vector,
@@ -1224,18 +1302,6 @@ void launch_coarse_apply(cudaStream_t s, const Level& lv, const double* Ainv, co
 #define CS_CL 8
 #define CS_MAXKL 496
 #define CS_WAIT (1 << 20)  // polls of a wait for four solved rows
-// RN(x / d) from y + y2 = 1 / d to twice the precision: a quotient within one ulp, and
-// Markstein's correction with its exact remainder (IBM J. Res. Dev. 34, 1990).  y = 0: d
-// is near the ends of the range.
-__device__ __forceinline__ double solve_quot(double x, double d, double y, double y2) {
-    const double q0 = fma(x, y, x * y2);
-    double q = fma(fma(-q0, d, x), y, q0);
-    const unsigned hi = (unsigned)__double2hiint(x);
-    if ((hi >> 20 & 0x7ff) - 600u > 846u || __double2hiint(y) == 0) {
-        if (((hi << 1) | (unsigned)__double2loint(x)) != 0) q = x / d;  // 0 where x is
-    }
-    return q;
-}
 template <typename TR, int RR>
 __global__ void __launch_bounds__(CS_THREADS) k_coarse_solve(Lay L, const double* __restrict__ ABg,
                                                              const int* __restrict__ ipiv,
@@ -1352,11 +1418,8 @@ __global__ void __launch_bounds__(CS_THREADS) k_coarse_solve(Lay L, const double
     for (int e = n, it = 0; e >= 1; e -= 32, it++) {
         const int i = e - lane, i2 = i - 32;
         if (rank == 0 && warp == (it & 1)) {
-            const unsigned ed = (unsigned)__double2hiint(pivot) >> 20 & 0x7ff;
-            const double y = ed - 600u > 846u ? 0.0 : 1.0 / pivot;
             s_d[lane] = pivot;
-            s_y[lane] = y;
-            s_y2[lane] = fma(-y, pivot, 1.0) * y;
+            solve_recip(pivot, s_y[lane], s_y2[lane]);
             __syncwarp();
             // the block's columns, four steps ahead: column e - l at row i
             double a[4];

@@ -102,7 +102,7 @@ struct Handle {
     double Cinit[TC_MAX_TYPES] = {};
     long long nequalize = 0;
     std::vector<int64_t> eq_row;
-    double *band = nullptr, *rowb = nullptr, *bvec = nullptr, *ainv = nullptr;
+    double *band = nullptr, *rowb = nullptr, *ainv = nullptr;
     // coarse grids above kCoarseInverseMax unknowns are solved by banded
     // substitution each visit instead of an explicit inverse
     bool coarse_banded = false;
@@ -1337,7 +1337,7 @@ tc_status multigrid(Handle* h) {
         launch_coarse_build(h->st, h->lev[G], h->band, h->rowb, h->kl, h->ku, h->p.Vbc);
         launch_coarse_lu(h->st, h->band, h->ipiv, h->ngrid_coarse, h->kl, h->ku, h->ds);
         if (!h->coarse_banded)
-            launch_coarse_inverse(h->st, h->band, h->ipiv, h->ngrid_coarse, h->kl, h->ku, h->ainv, h->bvec);
+            launch_coarse_inverse(h->st, h->band, h->ipiv, h->ngrid_coarse, h->kl, h->ku, h->ainv);
         h->lu_valid = true;
     };
     // SF = error(1); compute_velocities; compute_strain_rate_invariant
@@ -1999,7 +1999,6 @@ tc_status create(Handle* h, const tc_params* in) {
     h->coarse_banded = h->ngrid_coarse > kCoarseInverseMax;
     if (!h->coarse_banded) {
         TRY(dalloc_t(h, &h->ainv, (size_t)h->ngrid_coarse * h->ngrid_coarse));
-        TRY(dalloc_t(h, &h->bvec, (size_t)(h->ngrid_coarse + 8) * h->ngrid_coarse));
         // interior unknowns p = i*(nzc+1) + k in increasing order, with their offsets
         const Lay Lc = make_lay(nx >> (G - 1), nz >> (G - 1));
         std::vector<int> cq, cx;

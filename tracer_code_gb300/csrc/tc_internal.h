@@ -234,8 +234,7 @@ void launch_prolong(cudaStream_t s, const Level& coarse, const Level& fine, cons
 void launch_stream_bcs(cudaStream_t s, const Level& lv, double* S, int Vbc);
 void launch_coarse_build(cudaStream_t s, const Level& lv, double* band, double* rowb, int kl, int ku, int Vbc);
 void launch_coarse_lu(cudaStream_t s, double* band, int* ipiv, int n, int kl, int ku, DevScalars* ds);
-void launch_coarse_inverse(cudaStream_t s, const double* band, const int* ipiv, int n, int kl, int ku, double* Ainv,
-                           double* bscratch);
+void launch_coarse_inverse(cudaStream_t s, const double* band, const int* ipiv, int n, int kl, int ku, double* Ainv);
 void launch_coarse_solve(cudaStream_t s, const Level& lv, const double* band, const int* ipiv, const double* rowb,
                          int n, int kl, int ku, double* err, int Vbc, int* timeout_flag);
 void launch_coarse_solve32(cudaStream_t s, const Level& lv, const double* band, const int* ipiv, const double* rowb,
