@@ -256,15 +256,20 @@ __global__ void __launch_bounds__(BuildShape<T>::threads, 1) k_subcycle_build(Su
     }
 }
 
-// ---- FP32 build, four columns per CTA --------------------------------------------
-// The mixed solve's build (k_subcycle_build<float>'s arithmetic per column)
-// on four unit vectors at once: every shared-memory plane holds the four
-// columns' values of a point in one float4, so a sweep's 13 tap loads serve
-// four columns, and the coefficients, ghost targets and factors are shared.
-// The coarsest solve uses the compact FP32 inverse Ac (Ac[e][e2] = A^-1 at
-// the interior unknowns cq[e], cq[e2], times the row scale rowb[cq[e2]]):
-// the matrix is stored in FP32 anyway, and an FP64 solve of 945 x 2
+// ---- FP32 build, four or eight columns per CTA ------------------------------------
+// The mixed solve's build (k_subcycle_build<float>'s arithmetic per column) on 4 GR unit
+// vectors at once: a shared-memory plane holds four columns' values of a point in one
+// float4, so a sweep's loads serve four columns, and the coefficients, ghost targets and
+// factors are shared by all.  The coarsest solve uses the compact FP32 inverse Ac
+// (Ac[e][e2] = A^-1 at the interior unknowns cq[e], cq[e2], times the row scale
+// rowb[cq[e2]]): the matrix is stored in FP32 anyway, and an FP64 solve of 945 x 2
 // right-hand sides costs about 150 us of the FP64 pipe per build.
+//
+// What bounds it is the shared-memory reads.  A thread takes a strip of P points of a
+// column: 5 P + 8 reads instead of 13 P; with two points on 512 threads and eight columns
+// per CTA, 945 columns make one wave.  Against one point per thread and four columns
+// (1.6 waves): 568 -> 456 us for a 64x16 level (280 sweeps); three and four points (454 and
+// 477 us) leave too few warps to use the fewer reads.
 __device__ __forceinline__ float4 f4_fma(float c, float4 v, float4 a) {
     return make_float4(fmaf(c, v.x, a.x), fmaf(c, v.y, a.y), fmaf(c, v.z, a.z), fmaf(c, v.w, a.w));
 }
@@ -304,67 +309,139 @@ __device__ __forceinline__ void store_stream4(const Lay& L, float4* S, int i, in
     for (int g = 0; g < n; g++) S[idx[g]] = f4_scale(sg[g], v);
 }
 
-__global__ void __launch_bounds__(1024, 1) k_subcycle_build4(SubArgs<float> A, const float* __restrict__ Ac) {
-    constexpr int kThreads = 1024;
+template <int P, int GR, int NT, int MB>
+__global__ void __launch_bounds__(NT, MB) k_subcycle_build4(SubArgs<float> A, const float* __restrict__ Ac) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    float4* P0 = reinterpret_cast<float4*>(smem_raw);
-    float4* P1 = P0 + A.LS.plane;
-    float4* P2 = P1 + A.LS.plane;
-    float4* RG = P2 + A.LS.plane;
-    float4* EG = RG + A.LG.plane;
+    // planes without the global layout's row padding
+    Lay LS = A.LS, LG = A.LG;
+    LS.ld = LS.a + 1 + 2 * SP;
+    LG.ld = LG.a + 1 + 2 * SP;
+    LS.plane = (size_t)LS.ld * LS.nk;
+    LG.plane = (size_t)LG.ld * LG.nk;
+    const int pl = (int)LS.plane, gl = (int)LG.plane, ld = LS.ld;
+    float4* P0 = reinterpret_cast<float4*>(smem_raw);  // [GR] planes each
+    float4* P1 = P0 + GR * pl;
+    float4* P2 = P1 + GR * pl;
+    float4* RG = P2 + GR * pl;
+    float4* EG = RG + GR * gl;
     const int tid = threadIdx.x;
     const int nS = A.nS;
-    const int a1 = A.LS.a - 1, b1 = A.LS.b - 1;
-    const int j0 = blockIdx.x * 4;  // columns j0 .. j0 + 3 (those below nS)
-    const size_t total = 3 * A.LS.plane + 2 * A.LG.plane;
-    for (size_t t = tid; t < total; t += blockDim.x) P0[t] = make_float4(0.f, 0.f, 0.f, 0.f);
-    const int rpad = (((a1 + 31) & ~31) * b1 <= kThreads) ? ((a1 + 31) & ~31) : a1;
+    const int a1 = LS.a - 1, b1 = LS.b - 1;
+    const int j0 = blockIdx.x * 4 * GR;  // columns j0 .. j0 + 4 GR - 1 (those below nS)
+    for (int t = tid; t < GR * (3 * pl + 2 * gl); t += NT) P0[t] = make_float4(0.f, 0.f, 0.f, 0.f);
+    const int strips = (b1 + P - 1) / P;
+    const int rpad = (((a1 + 31) & ~31) * strips <= NT) ? ((a1 + 31) & ~31) : a1;
     const int si = tid % rpad, sk = tid / rpad;
-    const bool pa = si < a1 && sk < b1;
-    const int pi = pa ? 1 + si : 1, pk = pa ? 1 + sk : 1;
-    const int pidx = pa ? sk * a1 + si : 0;
-    const size_t px = IX(A.LS, pi, pk);
-    float cf[TC_NCOEF], dt;
+    const bool pa = si < a1 && sk < strips;
+    // a strip that would pass the last row ends there: it shares points with the one before
+    // (both write the same values)
+    const int pi = pa ? 1 + si : 1, pk = pa ? 1 + min(sk * P, max(b1 - P, 0)) : 1;
+    const int pn = pa ? min(P, b1) : 0;  // points of the strip
+    const int px = (int)IX(LS, pi, pk);
+    float cf[P][TC_NCOEF], dt[P];
+    // the ghost copies of ghost_targets: offset of the column's mirror (0: none), rows by row
+    const int side = pi <= SP ? -2 * pi : (pi >= LS.a - SP ? 2 * (LS.a - pi) : 0);
+    const bool rows = pk <= SP || pk + P - 1 >= LS.b - SP;
+    const float zsgn = (A.Vbc == 1) ? 1.f : -1.f;
 #pragma unroll
-    for (int d = 0; d < TC_NCOEF; d++) cf[d] = pa ? __ldg(A.coef + px + d * A.LS.plane) : 0.f;
-    dt = pa ? __ldg(A.dts + px) : 0.f;
-    const float4 rq = make_float4(pa && pidx == j0 ? 1.f : 0.f, pa && pidx == j0 + 1 ? 1.f : 0.f,
-                                  pa && pidx == j0 + 2 ? 1.f : 0.f, pa && pidx == j0 + 3 ? 1.f : 0.f);
-    int gidx[3];
-    float gsg[3];
-    const int gn = pa ? ghost_targets<float>(A.LS, pi, pk, A.Vbc, gidx, gsg) : 0;
+    for (int p = 0; p < P; p++) {
+        const bool on = p < pn;
+        const size_t xg = IX(A.LS, pi, on ? pk + p : pk);
+#pragma unroll
+        for (int d = 0; d < TC_NCOEF; d++) cf[p][d] = on ? -__ldg(A.coef + xg + d * A.LS.plane) : 0.f;
+        dt[p] = on ? __ldg(A.dts + xg) : 0.f;
+    }
+    auto unit = [&](int p, int g) {
+        const int e = (pk + p - 1) * a1 + pi - 1 - j0 - 4 * g;
+        return make_float4(e == 0 ? 1.f : 0.f, e == 1 ? 1.f : 0.f, e == 2 ? 1.f : 0.f, e == 3 ? 1.f : 0.f);
+    };
     __syncthreads();
-    auto put = [&](float4* S, float4 v) {
-        S[px] = v;
-        for (int g = 0; g < gn; g++) S[gidx[g]] = f4_scale(gsg[g], v);
+    auto put = [&](float4* S, int p, float4 v) {
+        S[px + p * ld] = v;
+        if (side != 0) S[px + p * ld + side] = f4_scale(-1.f, v);
+        if (rows) {
+            const int k = pk + p;
+            const int m = k <= SP ? -2 * k : (k >= LS.b - SP ? 2 * (LS.b - k) : 0);
+            if (m != 0) {
+                S[px + (p + m) * ld] = f4_scale(zsgn, v);
+                if (side != 0) S[px + (p + m) * ld + side] = f4_scale(-zsgn, v);
+            }
+        }
     };
-    const ptrdiff_t ld = (ptrdiff_t)A.LS.ld;
-    const ptrdiff_t off[TC_NCOEF] = {0, -1, 1, -2, 2, -ld, ld, -2 * ld, 2 * ld, -1 - ld, 1 - ld, -1 + ld, 1 + ld};
-    // rhs - L S at this thread's point, per column (sm_apply's order)
-    auto apply = [&](const float4* S, float4 rhs) {
-        float4 acc = rhs;
+    // rhs - L S at this thread's points, per column (sm_apply's order)
+    auto apply = [&](const float4* S, float4 (&acc)[P], float4 (&own)[P]) {
+        const float4* c = S + px;
+        if constexpr (P == 1) {
+            const int off[TC_NCOEF] = {0, -1, 1, -2, 2, -ld, ld, -2 * ld, 2 * ld, -1 - ld, 1 - ld, -1 + ld, 1 + ld};
+            own[0] = c[0];
 #pragma unroll
-        for (int d = 0; d < TC_NCOEF; d++) acc = f4_fma(-cf[d], S[(ptrdiff_t)px + off[d]], acc);
-        return acc;
+            for (int d = 0; d < TC_NCOEF; d++) acc[0] = f4_fma(cf[0][d], c[off[d]], acc[0]);
+            return;
+        }
+        float4 v[P + 4];
+#pragma unroll
+        for (int q = 0; q < P + 4; q++) v[q] = c[(min(q, pn + 3) - 2) * ld];
+        float4 l[P + 2], r[P + 2];
+#pragma unroll
+        for (int q = 0; q < P + 2; q++) {
+            l[q] = c[(min(q, pn + 1) - 1) * ld - 1];
+            r[q] = c[(min(q, pn + 1) - 1) * ld + 1];
+        }
+#pragma unroll
+        for (int p = 0; p < P; p++) {
+            const float4* e = c + min(p, max(pn - 1, 0)) * ld;
+            own[p] = v[p + 2];
+            acc[p] = f4_fma(cf[p][0], v[p + 2], acc[p]);
+            acc[p] = f4_fma(cf[p][1], l[p + 1], acc[p]);
+            acc[p] = f4_fma(cf[p][2], r[p + 1], acc[p]);
+            acc[p] = f4_fma(cf[p][3], e[-2], acc[p]);
+            acc[p] = f4_fma(cf[p][4], e[2], acc[p]);
+            acc[p] = f4_fma(cf[p][5], v[p + 1], acc[p]);
+            acc[p] = f4_fma(cf[p][6], v[p + 3], acc[p]);
+            acc[p] = f4_fma(cf[p][7], v[p], acc[p]);
+            acc[p] = f4_fma(cf[p][8], v[p + 4], acc[p]);
+        }
+#pragma unroll
+        for (int p = 0; p < P; p++) {
+            acc[p] = f4_fma(cf[p][9], l[p], acc[p]);
+            acc[p] = f4_fma(cf[p][10], r[p], acc[p]);
+            acc[p] = f4_fma(cf[p][11], l[p + 2], acc[p]);
+            acc[p] = f4_fma(cf[p][12], r[p + 2], acc[p]);
+        }
     };
+    const int pidx = (pk - 1) * a1 + pi - 1;
     auto visit = [&](float4* Sa, float4* Sb, int up) -> float4* {
         const float* cv = A.tab + (up ? 2 : 0) * A.nsweeps;
         const bool pp = !up && A.per_point_down;
         float cunext = __ldg(cv);
-        float cnext = (pp && pa) ? __ldg(A.ctab + pidx) : 0.f;
+        float cnext[P];
+#pragma unroll
+        for (int p = 0; p < P; p++) cnext[p] = (pp && p < pn) ? __ldg(A.ctab + pidx + p * a1) : 0.f;
         for (int n = 0; n < A.nsweeps; n++) {
-            const float cu = cunext, cpp = cnext;
+            float cd[P];
+#pragma unroll
+            for (int p = 0; p < P; p++) cd[p] = (pp ? cnext[p] : cunext) * dt[p];
             if (n + 1 < A.nsweeps) {
                 cunext = __ldg(cv + n + 1);
-                if (pp && pa) cnext = __ldg(A.ctab + (size_t)(n + 1) * nS + pidx);
+                if (pp)
+#pragma unroll
+                    for (int p = 0; p < P; p++)
+                        if (p < pn) cnext[p] = __ldg(A.ctab + (size_t)(n + 1) * nS + pidx + p * a1);
             }
             if (pa) {
-                const float4 res = apply(Sa, rq);
-                const float c = pp ? cpp : cu;
-                const float cd = c * dt;
-                const float4 s0 = Sa[px];
-                put(Sb, make_float4(fmaf(cd, res.x, s0.x), fmaf(cd, res.y, s0.y), fmaf(cd, res.z, s0.z),
-                                    fmaf(cd, res.w, s0.w)));
+#pragma unroll
+                for (int g = 0; g < GR; g++) {
+                    float4 acc[P], own[P];
+#pragma unroll
+                    for (int p = 0; p < P; p++) acc[p] = unit(p, g);
+                    apply(Sa + g * pl, acc, own);
+#pragma unroll
+                    for (int p = 0; p < P; p++)
+                        if (p < pn)
+                            put(Sb + g * pl, p, make_float4(fmaf(cd[p], acc[p].x, own[p].x), fmaf(cd[p], acc[p].y, own[p].y),
+                                                            fmaf(cd[p], acc[p].z, own[p].z),
+                                                            fmaf(cd[p], acc[p].w, own[p].w)));
+                }
             }
             __syncthreads();
             float4* t = Sa;
@@ -373,50 +450,82 @@ __global__ void __launch_bounds__(1024, 1) k_subcycle_build4(SubArgs<float> A, c
         }
         return Sa;
     };
-    const int lane = tid & 31, warp = tid >> 5, nwarps = kThreads / 32;
-    const int NG = A.LG.b + 1;
+    const int lane = tid & 31, warp = tid >> 5, nwarps = NT / 32;
+    const int NG = LG.b + 1, mG = (LG.a - 1) * (LG.b - 1);
     for (int blk = 1; blk <= A.kmax; blk++) {
         float4* e = visit(P0, P1, 0);
         if (e != P0) {
-            for (size_t t = tid; t < A.LS.plane; t += blockDim.x) P0[t] = e[t];
+            for (int t = tid; t < GR * pl; t += NT) P0[t] = e[t];
             __syncthreads();
         }
-        if (pa) P1[px] = apply(P0, rq);
+        if (pa) {
+#pragma unroll
+            for (int g = 0; g < GR; g++) {
+                float4 acc[P], own[P];
+#pragma unroll
+                for (int p = 0; p < P; p++) acc[p] = unit(p, g);
+                apply(P0 + g * pl, acc, own);
+#pragma unroll
+                for (int p = 0; p < P; p++)
+                    if (p < pn) P1[g * pl + px + p * ld] = acc[p];
+            }
+        }
         __syncthreads();
-        for (int c = tid; c < (A.LG.a - 1) * (A.LG.b - 1); c += blockDim.x) {
-            const int ic = 1 + c % (A.LG.a - 1), kc = 1 + c / (A.LG.a - 1);
-            RG[IX(A.LG, ic, kc)] = sm_restrict9_4(P1, A.LS, 2 * ic, 2 * kc);
+        for (int t = tid; t < GR * mG; t += NT) {
+            const int g = t / mG, c = t % mG, ic = 1 + c % (LG.a - 1), kc = 1 + c / (LG.a - 1);
+            RG[g * gl + (int)IX(LG, ic, kc)] = sm_restrict9_4(P1 + g * pl, LS, 2 * ic, 2 * kc);
         }
         __syncthreads();
         // coarsest solve x = Ac RG (one warp per unknown, lane-strided, shuffle tree)
         for (int w = warp; w < A.m; w += nwarps) {
             const int pw = __ldg(A.cq + w);
             const float* row = Ac + (size_t)w * A.m;
-            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (int e2 = lane; e2 < A.m; e2 += 32) acc = f4_fma(__ldg(row + e2), RG[__ldg(A.cx + e2)], acc);
-            for (int o = 16; o > 0; o >>= 1) {
-                acc.x += __shfl_down_sync(0xffffffffu, acc.x, o);
-                acc.y += __shfl_down_sync(0xffffffffu, acc.y, o);
-                acc.z += __shfl_down_sync(0xffffffffu, acc.z, o);
-                acc.w += __shfl_down_sync(0xffffffffu, acc.w, o);
+            float4 acc[GR];
+#pragma unroll
+            for (int g = 0; g < GR; g++) acc[g] = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int e2 = lane; e2 < A.m; e2 += 32) {
+                const int q = __ldg(A.cq + e2), x = (int)IX(LG, q / NG, q % NG);
+                const float f = __ldg(row + e2);
+#pragma unroll
+                for (int g = 0; g < GR; g++) acc[g] = f4_fma(f, RG[g * gl + x], acc[g]);
             }
-            if (lane == 0) store_stream4(A.LG, EG, pw / NG, pw % NG, acc, A.Vbc);
+#pragma unroll
+            for (int g = 0; g < GR; g++) {
+                for (int o = 16; o > 0; o >>= 1) {
+                    acc[g].x += __shfl_down_sync(0xffffffffu, acc[g].x, o);
+                    acc[g].y += __shfl_down_sync(0xffffffffu, acc[g].y, o);
+                    acc[g].z += __shfl_down_sync(0xffffffffu, acc[g].z, o);
+                    acc[g].w += __shfl_down_sync(0xffffffffu, acc[g].w, o);
+                }
+                if (lane == 0) store_stream4(LG, EG + g * gl, pw / NG, pw % NG, acc[g], A.Vbc);
+            }
         }
         __syncthreads();
-        if (pa) put(P0, f4_add(P0[px], sm_prolong4(A.LG, EG, pi, pk)));
+        if (pa) {
+            // a strip that shares points with the one before must not add to them twice
+            const int p0 = 1 + sk * P - pk;
+#pragma unroll
+            for (int g = 0; g < GR; g++)
+#pragma unroll
+                for (int p = 0; p < P; p++)
+                    if (p >= p0 && p < pn)
+                        put(P0 + g * pl, p,
+                            f4_add(P0[g * pl + px + p * ld], sm_prolong4(LG, EG + g * gl, pi, pk + p)));
+        }
         __syncthreads();
         float* out = A.M[blk - 1];
         if (out != nullptr) {
-            for (size_t t = tid; t < A.LS.plane; t += blockDim.x) P1[t] = P0[t];
+            for (int t = tid; t < GR * pl; t += NT) P1[t] = P0[t];
             __syncthreads();
             const float4* f = visit(P1, P2, 1);
-            for (int p = tid; p < nS; p += blockDim.x) {
-                const float4 v = f[IX(A.LS, 1 + p % a1, 1 + p / a1)];
-                float* o = out + (size_t)p * nS + j0;
-                o[0] = v.x;
-                if (j0 + 1 < nS) o[1] = v.y;
-                if (j0 + 2 < nS) o[2] = v.z;
-                if (j0 + 3 < nS) o[3] = v.w;
+            for (int t = tid; t < GR * nS; t += NT) {
+                const int g = t % GR, p = t / GR, j = j0 + 4 * g;
+                const float4 v = f[g * pl + (int)IX(LS, 1 + p % a1, 1 + p / a1)];
+                float* o = out + (size_t)p * nS + j;
+                if (j < nS) o[0] = v.x;
+                if (j + 1 < nS) o[1] = v.y;
+                if (j + 2 < nS) o[2] = v.z;
+                if (j + 3 < nS) o[3] = v.w;
             }
             __syncthreads();
         }
@@ -485,18 +594,28 @@ size_t build_smem(const Lay& LS, const Lay& LG) {
     return sizeof(T) * (4 * LS.plane + 2 * LG.plane);
 }
 
+template <int P, int GR, int NT, int MB>
+int launch_build4_as(cudaStream_t s, const SubArgs<float>& A, float* Ac, size_t smem) {
+    if (cudaFuncSetAttribute(k_subcycle_build4<P, GR, NT, MB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+        cudaSuccess)
+        return -1;
+    k_subcycle_build4<P, GR, NT, MB><<<(A.nS + 4 * GR - 1) / (4 * GR), NT, smem, s>>>(A, Ac);
+    tc_note_launch();
+    return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
+}
 int launch_build4(cudaStream_t s, const SubArgs<float>& A, float* Ac) {
-    const size_t smem = sizeof(float4) * (3 * A.LS.plane + 2 * A.LG.plane);
+    auto plane = [](const Lay& L) { return (size_t)(L.a + 1 + 2 * SP) * L.nk; };
+    const size_t smem = sizeof(float4) * (3 * plane(A.LS) + 2 * plane(A.LG));
     if (A.nS > kMaxS || smem > 200 * 1024 || Ac == nullptr) return -1;
     const int mm = A.m * A.m;
     k_coarse_compact32<<<(mm + 255) / 256, 256, 0, s>>>(A.Ainv, A.rowb, A.cq, A.m, A.n, Ac);
     tc_note_launch();
-    if (cudaFuncSetAttribute(k_subcycle_build4, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-        cudaSuccess)
-        return -1;
-    k_subcycle_build4<<<(A.nS + 3) / 4, 1024, smem, s>>>(A, Ac);
-    tc_note_launch();
-    return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
+    // two points a thread where 512 threads cover the level and eight columns' planes fit;
+    // else one (a 93x11 level, 606 us)
+    const int strips = A.LS.b / 2;
+    if ((A.LS.a - 1) * strips <= 512 && 2 * smem <= 200 * 1024)
+        return launch_build4_as<2, 2, 512, 1>(s, A, Ac, 2 * smem);
+    return launch_build4_as<1, 1, 1024, 1>(s, A, Ac, smem);
 }
 
 template <typename T>
