@@ -179,6 +179,7 @@ __global__ void __launch_bounds__(NT, 1) k_visit_cluster(VisitParams<T> Q, T* Sg
     const size_t bsz = (size_t)R * W;
     const int tid = threadIdx.x;
     const T zsgn = (Q.Vbc == 1) ? T(1) : T(-1);
+    const bool flip_z = Q.Vbc != 1;
     // this thread's strip
     const int cols = a - 1;
     const int i = 1 + tid % cols, strip = tid / cols;
@@ -285,30 +286,35 @@ __global__ void __launch_bounds__(NT, 1) k_visit_cluster(VisitParams<T> Q, T* Sg
         pre0[p] = (ld && Q.nsweeps > 0) ? __ldg(ctab + tab_base + (size_t)p * cols) : T(0);
         pre1[p] = (ld && Q.nsweeps > 1) ? __ldg(ctab + (size_t)npl + tab_base + (size_t)p * cols) : T(0);
     }
+    // c(n) * dt; FP64 forms the next sweep's before it waits for that sweep's halo
+    T cd[P];
+    auto factors = [&](int n) {
+        if (Q.per_point && kDivide) {
+            const T tn = Q.temp[n];
+#pragma unroll
+            for (int p = 0; p < P; p++) cd[p] = (T(2) / (ca[p] + cbv[p] * tn)) * dt[p];
+        } else if (Q.per_point) {
+#pragma unroll
+            for (int p = 0; p < P; p++) {
+                cd[p] = pre0[p] * dt[p];
+                pre0[p] = pre1[p];
+                pre1[p] = (act[p] && n + 2 < Q.nsweeps)
+                              ? __ldg(ctab + (size_t)(n + 2) * npl + tab_base + (size_t)p * cols)
+                              : T(0);
+            }
+        } else {
+            const T c = Q.c[n];
+#pragma unroll
+            for (int p = 0; p < P; p++) cd[p] = c * dt[p];
+        }
+    };
+    if (!kDivide && Q.nsweeps > 0) factors(0);
     for (int n = 0; n < Q.nsweeps && !timed_out; n++) {
         const int nxt_b = (cur_b + 1 == nbuf) ? 0 : cur_b + 1;
         const T* cur = buf + (size_t)cur_b * bsz;
         T* nxt = buf + (size_t)nxt_b * bsz;
         if (act[0]) {
-            T cp[P];
-            if (Q.per_point && kDivide) {
-                const T tn = Q.temp[n];
-#pragma unroll
-                for (int p = 0; p < P; p++) cp[p] = T(2) / (ca[p] + cbv[p] * tn);
-            } else if (Q.per_point) {
-#pragma unroll
-                for (int p = 0; p < P; p++) {
-                    cp[p] = pre0[p];
-                    pre0[p] = pre1[p];
-                    pre1[p] = (act[p] && n + 2 < Q.nsweeps)
-                                  ? __ldg(ctab + (size_t)(n + 2) * npl + tab_base + (size_t)p * cols)
-                                  : T(0);
-                }
-            } else {
-                const T c = Q.c[n];
-#pragma unroll
-                for (int p = 0; p < P; p++) cp[p] = c;
-            }
+            if (kDivide) factors(n);
             // strip values: centre column rows r0-2..r0+P+1, columns i+-1 rows
             // r0-1..r0+P, columns i+-2 rows r0..r0+P-1 (rows past the band are
             // inside the padded buffer; their results are not stored)
@@ -358,23 +364,24 @@ __global__ void __launch_bounds__(NT, 1) k_visit_cluster(VisitParams<T> Q, T* Sg
             for (int p = 0; p < P; p++) acc[p] = fma(cf[p][12], vp1[p + 2], acc[p]);
             T v[P];
 #pragma unroll
-            for (int p = 0; p < P; p++) v[p] = fma(cp[p] * dt[p], acc[p], v0[p + 2]);
+            for (int p = 0; p < P; p++) v[p] = fma(cd[p], acc[p], v0[p + 2]);
             T* nb = nxt + (size_t)r0 * W + cc;
 #pragma unroll
             for (int p = 0; p < P; p++)
                 if (act[p]) nb[p * W] = v[p];
+            // (signs changed as bits: the FP64 pipe is the bound)
             if (has_side) {
                 T* ns = nxt + (size_t)r0 * W + side;
 #pragma unroll
                 for (int p = 0; p < P; p++)
-                    if (act[p]) ns[p * W] = -v[p];
+                    if (act[p]) ns[p * W] = flip_sign(v[p], true);
             }
             if (has_grow) {
 #pragma unroll
                 for (int p = 0; p < P; p++) {
                     if (!act[p]) continue;
-                    if (kr + p == 1) nb[(p - 2) * W] = zsgn * v[p];
-                    if (kr + p == b - 1) nb[(p + 2) * W] = zsgn * v[p];
+                    if (kr + p == 1) nb[(p - 2) * W] = flip_sign(v[p], flip_z);
+                    if (kr + p == b - 1) nb[(p + 2) * W] = flip_sign(v[p], flip_z);
                 }
             }
             if (remote) {
@@ -400,6 +407,7 @@ __global__ void __launch_bounds__(NT, 1) k_visit_cluster(VisitParams<T> Q, T* Sg
             __syncwarp();
             if (tid == 0) mbar_arrive_expect(nb, expect);
             else if ((tid & 31) == 0) mbar_arrive(nb);
+            if (!kDivide && n + 1 < Q.nsweeps) factors(n + 1);
             int it = 0;
             bool to = false;
             while (!mbar_try_wait(nb, (phase >> nxt_b) & 1)) {
@@ -408,6 +416,7 @@ __global__ void __launch_bounds__(NT, 1) k_visit_cluster(VisitParams<T> Q, T* Sg
             phase ^= 1 << nxt_b;
             if (to) { timed_out = true; break; }
         } else {
+            if (!kDivide && n + 1 < Q.nsweeps) factors(n + 1);
             __syncthreads();
         }
         cur_b = nxt_b;
@@ -611,10 +620,14 @@ static bool visit_shape(const Lay& L, int nsweeps, bool fp32, int cfg, VisitShap
         s->C = (rows + s->rpc - 1) / s->rpc;
     } else {
         // one point per thread over up to 16 CTAs: more SMs issue the sweep
-        // (measured faster than fewer, fuller CTAs for levels of <= 4K points)
+        // (measured faster than fewer, fuller CTAs for levels of <= 4K points).
+        // FP64: not fewer than a warp per scheduler, whose operations take the same
+        // 64 cycles for one warp each; fewer CTAs then exchange less (70 sweeps on
+        // 8x8: one CTA 57 us, seven 66; 16x16: two 65, fifteen 66; 256 points a
+        // CTA: 79)
         s->p = 1;
         s->nt = 256;
-        s->rpc = spread_rpc;
+        s->rpc = fp32 ? spread_rpc : std::max(spread_rpc, std::min(rows, 128 / cols));
         s->C = (rows + s->rpc - 1) / s->rpc;
         if (s->rpc * cols > s->nt) return false;
     }

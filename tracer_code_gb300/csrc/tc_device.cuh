@@ -251,24 +251,33 @@ __device__ __forceinline__ void fold_from_fields(const FoldG32& F, const float* 
     }
 }
 
+// v or -v, as bits: signs change without the FP64 pipe
+__device__ __forceinline__ float flip_sign(float v, bool flip) { return flip ? -v : v; }
+__device__ __forceinline__ double flip_sign(double v, bool flip) {
+    return __hiloint2double(__double2hiint(v) ^ (flip ? 0x80000000 : 0), __double2loint(v));
+}
+
 // writes v at interior (i,k) and the ghost/mirror copies enforceBCs_stream
 // derives from it (Vbc=0: antisymmetric rows; Vbc=1: symmetric rows)
 template <typename T>
 __device__ __forceinline__ void store_stream(const Lay& L, T* S, int i, int k, T v, int Vbc) {
     const int a = L.a, b = L.b;
-    int gi[3] = {i, 0, 0};
-    T si[3] = {T(1), T(-1), T(-1)};
-    int ng = 1;
-    if (i <= SP) gi[ng++] = -i;
-    if (i >= a - SP) gi[ng++] = 2 * a - i;
-    int gk[3] = {k, 0, 0};
-    const T zsgn = (Vbc == 1) ? T(1) : T(-1);
-    T sk[3] = {T(1), zsgn, zsgn};
-    int nk = 1;
-    if (k <= SP) gk[nk++] = -k;
-    if (k >= b - SP) gk[nk++] = 2 * b - k;
-    for (int u = 0; u < nk; u++)
-        for (int t = 0; t < ng; t++) S[IX(L, gi[t], gk[u])] = (si[t] * sk[u]) * v;
+    const ptrdiff_t ld = (ptrdiff_t)L.ld;
+    T* s = S + IX(L, i, k);
+    *s = v;
+    const bool xl = i <= SP, xr = i >= a - SP, zl = k <= SP, zr = k >= b - SP;
+    if (!(xl || xr || zl || zr)) return;
+    const T side = flip_sign(v, true), row = flip_sign(v, Vbc != 1), corner = flip_sign(v, Vbc == 1);
+    if (xl) s[-2 * i] = side;
+    if (xr) s[2 * (a - i)] = side;
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+        if (!(u == 0 ? zl : zr)) continue;
+        T* g = s + (u == 0 ? -2 * k : 2 * (b - k)) * ld;
+        *g = row;
+        if (xl) g[-2 * i] = corner;
+        if (xr) g[2 * (a - i)] = corner;
+    }
 }
 
 // ---------------------------------------------------------------------------

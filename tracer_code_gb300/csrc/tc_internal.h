@@ -183,7 +183,7 @@ struct Level {
     FoldG32 gw;
     int use_g32;  // 1: the level's per-sweep FP32 smoother reads g32
     // launch configuration of this level's smoother, set by tc_autotune
-    // (defaults: 32x8 blocks; fused visits wherever they fit)
+    // (defaults: 32x8 blocks, 64x2 on small FP64 levels; fused visits wherever they fit)
     int sweep_bx, sweep_by;
     int fuse;       // 1 = one cluster launch per visit when the level fits, 0 = one launch per sweep
     int visit_cfg;  // shape of the fused visit: 0 = default, else 100*points per strip + CTAs
