@@ -74,11 +74,11 @@ __device__ __forceinline__ void eig_pair(const LevConst& c, double v, double vx,
                                          double vxz, double& eR, double& eI) {
     double t1 = (vxx - vzz) * c.eK1;
     double t2 = v * c.eK2;
-    double t3 = 2.0 * v * c.eTrrss;
-    double t4 = 4.0 * vxz * c.eTrs;
+    double t3 = v * (2.0 * c.eTrrss);
+    double t4 = vxz * (4.0 * c.eTrs);
     eR = -(t1 + t2 + t3 + t4);
-    double t5 = 2.0 * vx * c.eK5;
-    double t6 = 2.0 * vz * c.eK6;
+    double t5 = vx * (2.0 * c.eK5);
+    double t6 = vz * (2.0 * c.eK6);
     eI = fabs(t5) + fabs(t6);
 }
 
@@ -127,6 +127,70 @@ __device__ void eig_pair_metric(const LevConst& c, int i, int k, double v, doubl
     }
 }
 
+// x / h for a spacing h > 0 with hinv = RN(1 / h): a product where the spacings are
+// powers of two, else two Newton corrections (Markstein, as quot_round in k_tracer.cu)
+__device__ __forceinline__ double spacing_quot(double x, double h, double hinv, int recip) {
+    if (recip) return x * hinv;
+    const unsigned hi = (unsigned)__double2hiint(x), ex = hi >> 20 & 0x7ff;
+    if (ex - 200u > 1600u) return ((hi << 1) | (unsigned)__double2loint(x)) != 0 ? x / h : x;
+    double q = x * hinv;
+    q = fma(fma(-q, h, x), hinv, q);
+    return fma(fma(-q, h, x), hinv, q);
+}
+// viscosity_gradients' differences, -0.5 vm + 0.5 vp over dr and so on.  The factors that
+// are powers of two are exact, so they go into the spacing; half the FP64 operations.
+struct VisDiff {
+    double r, rr, s, ss, rs;
+};
+__device__ __forceinline__ double second_diff(double m, double c, double p) { return fma(-2.0, c, m) + p; }
+__device__ __forceinline__ VisDiff vis_diff(const LevConst& c, double v0, double vm, double vp, double vzm, double vzp,
+                                            double mm, double pm, double mp, double pp) {
+    VisDiff d;
+    d.r = spacing_quot(vp - vm, 2.0 * c.dr, 0.5 * c.rdr, c.recip);
+    d.rr = spacing_quot(second_diff(vm, v0, vp), c.dr2, c.rdr2, c.recip);
+    d.s = spacing_quot(vzp - vzm, 2.0 * c.ds, 0.5 * c.rds, c.recip);
+    d.ss = spacing_quot(second_diff(vzm, v0, vzp), c.ds2, c.rds2, c.recip);
+    d.rs = spacing_quot(((mm - pm) - mp) + pp, 4.0 * c.drds, 0.25 * c.rdrds, c.recip);
+    return d;
+}
+
+// viscosity_gradients at node (i, k) (in d) and, if asked, |eigR / eigI|
+template <bool METRIC>
+__device__ __forceinline__ double vis_point(const LevConst& c, int i, int k, bool eig, double v0, double vm, double vp,
+                                            double vzm, double vzp, double mm, double pm, double mp, double pp,
+                                            VisDiff& d) {
+    d = vis_diff(c, v0, vm, vp, vzm, vzp, mm, pm, mp, pp);
+    double eR = 0.0, eI = 1.0;
+    if (METRIC) {
+        // viscosity_gradients on a stretched grid (iterative_solver.f90:320-324)
+        const int ii = i * c.mf, kk = k * c.mf;
+        const double x1 = mt(c.M.xr, ii), x2 = mt(c.M.xrr, ii), z1 = mt(c.M.zs, kk), z2 = mt(c.M.zss, kk);
+        const double ax = d.r / x1, az = d.s / z1;
+        const double axx = (d.rr - ax * x2) / (x1 * x1), azz = (d.ss - az * z2) / (z1 * z1);
+        d.rs = d.rs / x1 / z1;
+        d.r = ax; d.s = az; d.rr = axx; d.ss = azz;
+        if (eig) eig_pair_metric(c, i, k, v0, d.r, d.s, d.rr, d.ss, d.rs, eR, eI);
+    } else if (eig) {
+        eig_pair(c, v0, d.r, d.s, d.rr, d.ss, d.rs, eR, eI);
+    }
+    return eig ? fabs(eR / eI) : 0.0;
+}
+// vis_space (smoother.f90:142-164): the Laplacian that smooths the viscosity
+template <bool METRIC>
+__device__ __forceinline__ double vis_laplacian(const LevConst& c, int i, int k, double v0, double vm, double vp,
+                                                double vzm, double vzp) {
+    const double Trr = spacing_quot(second_diff(vm, v0, vp), c.dr2, c.rdr2, c.recip);
+    const double Tss = spacing_quot(second_diff(vzm, v0, vzp), c.ds2, c.rds2, c.recip);
+    if (!METRIC) return Trr + Tss;
+    const double Tr = spacing_quot(vp - vm, 2.0 * c.dr, 0.5 * c.rdr, c.recip);
+    const double Ts = spacing_quot(vzp - vzm, 2.0 * c.ds, 0.5 * c.rds, c.recip);
+    const int i1 = i * c.mf, k1 = k * c.mf;
+    const double x1 = mt(c.M.xr, i1), x2 = mt(c.M.xrr, i1), z1 = mt(c.M.zs, k1), z2 = mt(c.M.zss, k1);
+    const double Tx = Tr / x1, Tz = Ts / z1;
+    const double Txx = (Trr - Tx * x2) / (x1 * x1), Tzz = (Tss - Tz * z2) / (z1 * z1);
+    return Txx + Tzz;
+}
+
 __global__ void k_vis_grad(Lay L, LevConst c, Range2 r, const double* __restrict__ V, double* __restrict__ vx,
                            double* __restrict__ vz, double* __restrict__ vxx, double* __restrict__ vzz,
                            double* __restrict__ vxz, double* __restrict__ ratio, int do_eig, int ivis,
@@ -139,42 +203,13 @@ __global__ void k_vis_grad(Lay L, LevConst c, Range2 r, const double* __restrict
             vx[x] = 0.0; vz[x] = 0.0; vxx[x] = 0.0; vzz[x] = 0.0; vxz[x] = 0.0;
         } else {
             const size_t ld = (size_t)L.ld;
-            double v0 = V[x], vm = V[x - 1], vp = V[x + 1], vzm = V[x - ld], vzp = V[x + ld];
-            const double nr = -0.5 * vm + 0.5 * vp, nrr = vm + -2.0 * v0 + vp;
-            const double ns = -0.5 * vzm + 0.5 * vzp, nss = vzm + -2.0 * v0 + vzp;
-            const double nrs =
-                0.25 * V[x - 1 - ld] + -0.25 * V[x + 1 - ld] + -0.25 * V[x - 1 + ld] + 0.25 * V[x + 1 + ld];
-            // power-of-two spacings: the products equal the quotients exactly
-            double vis_r, vis_rr, vis_s, vis_ss, vis_rs;
-            if (c.recip) {
-                vis_r = nr * c.rdr; vis_rr = nrr * c.rdr2; vis_s = ns * c.rds; vis_ss = nss * c.rds2;
-                vis_rs = nrs * c.rdrds;
-            } else {
-                vis_r = nr / c.dr; vis_rr = nrr / c.dr2; vis_s = ns / c.ds; vis_ss = nss / c.ds2; vis_rs = nrs / c.drds;
-            }
-            if (c.M.on) {
-                // viscosity_gradients on a stretched grid (iterative_solver.f90:320-324)
-                const int ii = i * c.mf, kk = k * c.mf;
-                const double x1 = mt(c.M.xr, ii), x2 = mt(c.M.xrr, ii), z1 = mt(c.M.zs, kk), z2 = mt(c.M.zss, kk);
-                const double ax = vis_r / x1, az = vis_s / z1;
-                const double axx = (vis_rr - ax * x2) / (x1 * x1), azz = (vis_ss - az * z2) / (z1 * z1);
-                const double axz = vis_rs / x1 / z1;
-                vx[x] = ax; vz[x] = az; vxx[x] = axx; vzz[x] = azz; vxz[x] = axz;
-                if (do_eig) {
-                    double eR, eI;
-                    eig_pair_metric(c, i, k, v0, ax, az, axx, azz, axz, eR, eI);
-                    rat = fabs(eR / eI);
-                    ratio[x] = rat;
-                }
-            } else {
-                vx[x] = vis_r; vz[x] = vis_s; vxx[x] = vis_rr; vzz[x] = vis_ss; vxz[x] = vis_rs;
-                if (do_eig) {
-                    double eR, eI;
-                    eig_pair(c, v0, vis_r, vis_s, vis_rr, vis_ss, vis_rs, eR, eI);
-                    rat = fabs(eR / eI);
-                    ratio[x] = rat;
-                }
-            }
+            const double v0 = V[x], vm = V[x - 1], vp = V[x + 1], vzm = V[x - ld], vzp = V[x + ld];
+            const double mm = V[x - 1 - ld], pm = V[x + 1 - ld], mp = V[x - 1 + ld], pp = V[x + 1 + ld];
+            VisDiff d;
+            rat = c.M.on ? vis_point<true>(c, i, k, do_eig != 0, v0, vm, vp, vzm, vzp, mm, pm, mp, pp, d)
+                         : vis_point<false>(c, i, k, do_eig != 0, v0, vm, vp, vzm, vzp, mm, pm, mp, pp, d);
+            vx[x] = d.r; vz[x] = d.s; vxx[x] = d.rr; vzz[x] = d.ss; vxz[x] = d.rs;
+            if (do_eig) ratio[x] = rat;
         }
     }
     if (do_eig && ivis != 0) reduce_to(RED_MIN, rat, rs.part, rs.count, out_min);
@@ -189,6 +224,20 @@ void launch_vis_grad(cudaStream_t s, const Level& lv, const double* vis, int do_
 // ---------------------------------------------------------------------------
 // one Chebyshev step of smoother_vis with viscosityBCs fused
 // ---------------------------------------------------------------------------
+// v at (i, k) and its side ghosts (rows 0..b): V(-i,k)=V(i,k), V(a+i,k)=V(a-i,k)
+__device__ __forceinline__ void store_with_sides(const Lay& L, double* row, int i, double v) {
+    const int a = L.a;
+    row[i] = v;
+    if (i >= 1 && i <= SP) row[-i] = v;
+    if (i >= a - SP && i <= a - 1) row[2 * a - i] = v;
+}
+// the top/bottom ghosts that mirror (i, k), of this column and of its side-ghost columns
+__device__ __forceinline__ void store_mirror_rows(const Lay& L, double* Vout, int i, int k, double v, int RaTnz,
+                                                  double visT2) {
+    const int b = L.b;
+    if (k >= 1 && k <= SP) store_with_sides(L, Vout + IX(L, 0, -k), i, RaTnz ? (1.0 / v / visT2) : v);
+    if (k >= b - SP && k <= b - 1) store_with_sides(L, Vout + IX(L, 0, 2 * b - k), i, RaTnz ? (1.0 / v) : v);
+}
 __global__ void k_vis_smooth(Lay L, LevConst cc, Range2 r, const double* __restrict__ Vin, double* __restrict__ Vout,
                              const double* __restrict__ dtv, double c, const double* cdev, int RaTnz, double visT2) {
     RANGE_IK(r);
@@ -196,43 +245,13 @@ __global__ void k_vis_smooth(Lay L, LevConst cc, Range2 r, const double* __restr
     if (cdev) c = *cdev;  // the factor the device-side filter loop chose
     const size_t ld = (size_t)L.ld;
     size_t x = IX(L, i, k);
-    double v0 = Vin[x];
-    const double nrr = Vin[x - 1] + -2.0 * v0 + Vin[x + 1], nss = Vin[x - ld] + -2.0 * v0 + Vin[x + ld];
-    // power-of-two spacings: the products equal the quotients exactly
-    const double Trr = cc.recip ? nrr * cc.rdr2 : nrr / cc.dr2;
-    const double Tss = cc.recip ? nss * cc.rds2 : nss / cc.ds2;
-    double temp;
-    if (cc.M.on) {
-        // vis_space on a stretched grid (smoother.f90:142-164)
-        const double nr = -0.5 * Vin[x - 1] + 0.5 * Vin[x + 1], ns = -0.5 * Vin[x - ld] + 0.5 * Vin[x + ld];
-        const double Tr = cc.recip ? nr * cc.rdr : nr / cc.dr, Ts = cc.recip ? ns * cc.rds : ns / cc.ds;
-        const int i1 = i * cc.mf, k1 = k * cc.mf;
-        const double x1 = mt(cc.M.xr, i1), x2 = mt(cc.M.xrr, i1), z1 = mt(cc.M.zs, k1), z2 = mt(cc.M.zss, k1);
-        const double Tx = Tr / x1, Tz = Ts / z1;
-        const double Txx = (Trr - Tx * x2) / (x1 * x1), Tzz = (Tss - Tz * z2) / (z1 * z1);
-        temp = Txx + Tzz;
-    } else {
-        temp = Trr + Tss;
-    }
+    const double v0 = Vin[x], vm = Vin[x - 1], vp = Vin[x + 1], vzm = Vin[x - ld], vzp = Vin[x + ld];
+    const double temp = cc.M.on ? vis_laplacian<true>(cc, i, k, v0, vm, vp, vzm, vzp)
+                                : vis_laplacian<false>(cc, i, k, v0, vm, vp, vzm, vzp);
     double dts = dtv[x] * 0.99;
     double v = v0 + c * dts * temp;
-    Vout[x] = v;
-    const int a = L.a, b = L.b;
-    // side ghosts (rows 0..b): V(-i,k)=V(i,k), V(a+i,k)=V(a-i,k)
-    int gi[3] = {i, 0, 0};
-    int ng = 1;
-    if (i >= 1 && i <= SP) gi[ng++] = -i;
-    if (i >= a - SP && i <= a - 1) gi[ng++] = 2 * a - i;
-    for (int t = 1; t < ng; t++) Vout[IX(L, gi[t], k)] = v;
-    // top/bottom ghosts of this column and of its side-ghost columns
-    if (k >= 1 && k <= SP) {
-        double g = RaTnz ? (1.0 / v / visT2) : v;
-        for (int t = 0; t < ng; t++) Vout[IX(L, gi[t], -k)] = g;
-    }
-    if (k >= b - SP && k <= b - 1) {
-        double g = RaTnz ? (1.0 / v) : v;
-        for (int t = 0; t < ng; t++) Vout[IX(L, gi[t], 2 * b - k)] = g;
-    }
+    store_with_sides(L, Vout + IX(L, 0, k), i, v);
+    store_mirror_rows(L, Vout, i, k, v, RaTnz, visT2);
 }
 void launch_vis_smooth(cudaStream_t s, const Level& lv, const double* vin, double* vout, double c, int kmin,
                        int kmax, int RaT_nonzero, double visT2, const double* cdev) {
@@ -240,6 +259,200 @@ void launch_vis_smooth(cudaStream_t s, const Level& lv, const double* vin, doubl
     k_vis_smooth<<<grid_for(r), dim3(BX, BY), 0, s>>>(lv.L, lv.c, r, vin, vout, lv.dt_vis, c, cdev, RaT_nonzero,
                                                        visT2);
     tc_note_launch();
+}
+
+// ---------------------------------------------------------------------------
+// smoother_vis (smoother.f90:166-263) of a small level in one launch of a cluster: the loop
+// of k_loop.cu's filter graphs, test and step in one pass with one cluster barrier.  A pass
+// takes the smallest eigenvalue ratio of the current viscosity and already writes the next
+// step into the other plane (the factor does not depend on the ratio); when the test then
+// ends the loop that plane is dropped.  The derivative fields are written once, after the
+// loop; where no test reads the ratio (interpolate) the passes only smooth.  vx null: the
+// level's own viscosity (src) and derivatives stay, the result is left in A.
+//
+// What bounds it: the FP64 pipe, about 45 operations of 64 cycles a point and pass for 128
+// points per SM at a time, and L2 latency.  The graph's loop took four nodes a step, 20 to
+// 25 us whatever the level, and twelve copies around an interpolation: the viscosities of
+// levels 2 to 4 of a 256x64 grid 330 + 320 + 131 us, now 116 + 65 + 35.  Larger levels keep
+// the graphs: with the ratio one cluster's FP64 pipes cost as much as the nodes at 16,700
+// points (151 us against 145); stretched grids take some 30 divisions a point.
+// ---------------------------------------------------------------------------
+#define VF_THREADS 512
+#define VF_CL 16
+#define VF_MAX_SMOOTH 17000  // points, without and with the ratio in each pass
+#define VF_MAX_RATIO 12000
+#define VF_MAX_RATIO_METRIC 4500
+template <bool METRIC>
+__global__ void __launch_bounds__(VF_THREADS) k_vis_filter(Lay L, LevConst c, VisFltArgs q, int reset,
+                                                           const double* src, double* A, double* B,
+                                                           const double* __restrict__ dtv, int kmin,
+                                                           int kmax, int RaTnz, double visT2, double* __restrict__ vx,
+                                                           double* __restrict__ vz, double* __restrict__ vxx,
+                                                           double* __restrict__ vzz, double* __restrict__ vxz,
+                                                           double* __restrict__ ratio, DevScalars* ds) {
+    cg::cluster_group cl = cg::this_cluster();
+    const int C = (int)cl.num_blocks(), rank = (int)cl.block_rank(), nt = (int)blockDim.x;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int gt = rank * nt + tid, gn = C * nt;
+    __shared__ unsigned long long s_warp[VF_THREADS / 32], s_all[2][VF_CL];
+    const ptrdiff_t ld = (ptrdiff_t)L.ld;
+    const int a = L.a, b = L.b, w = a + 1, npts = w * (kmax - kmin + 1);
+    for (size_t x = gt; x < L.plane; x += gn) {
+        const double v = ld_state(src + x);
+        B[x] = v;
+        if (A != src) A[x] = v;
+    }
+    // the smallest ratio of the level, from each thread's (as bits: none is negative, a NaN is never the smallest)
+    auto level_min = [&](unsigned long long m, int par) {
+        unsigned hi = __reduce_min_sync(0xffffffffu, (unsigned)(m >> 32));
+        unsigned lo = __reduce_min_sync(0xffffffffu, (unsigned)(m >> 32) == hi ? (unsigned)m : 0xffffffffu);
+        if (lane == 0) s_warp[warp] = (unsigned long long)hi << 32 | lo;
+        __syncthreads();
+        if (warp == 0) {
+            m = lane < nt / 32 ? s_warp[lane] : ~0ull;
+            hi = __reduce_min_sync(0xffffffffu, (unsigned)(m >> 32));
+            lo = __reduce_min_sync(0xffffffffu, (unsigned)(m >> 32) == hi ? (unsigned)m : 0xffffffffu);
+            if (lane < C) cl.map_shared_rank(&s_all[0][0], lane)[par * VF_CL + rank] = (unsigned long long)hi << 32 | lo;
+        }
+        cl.sync();
+        m = ~0ull;
+        for (int r = 0; r < C; r++) m = min(m, s_all[par][r]);
+        return __longlong_as_double((long long)m);
+    };
+    auto point_ratio = [&](const double* V, size_t x, int i, int k, double v0, double vm, double vp, double vzm,
+                           double vzp, VisDiff& d) {
+        return vis_point<METRIC>(c, i, k, true, v0, vm, vp, vzm, vzp, ld_state(V + x - 1 - ld),
+                                 ld_state(V + x + 1 - ld), ld_state(V + x - 1 + ld), ld_state(V + x + 1 + ld), d);
+    };
+    constexpr unsigned long long kInf = 0x7ffull << 52;
+    // the loop's state, the same on every thread (k_vflt_init)
+    int nvis = reset ? 0 : ds->vis_nvis_store, nstore = reset ? 1 : ds->vis_nn_store;
+    int phase = 0, n = 0, nn = nstore, niter = q.niter0, status = 0, n_eta = 0;
+    long long guard = 0;
+    bool more = true, fine = false;
+    auto next_outer = [&] {
+        nvis += 1;
+        nstore = 1;
+        if (q.option == 1) {
+            niter = 6;
+            phase = 1;
+        }
+        n += 1;
+        nn = 1;
+        if (++guard > q.cap) {
+            status = TC_ERR_LOOP_CAP;
+            more = false;
+        }
+    };
+    if (nn > niter) next_outer();
+    more = true;
+    cl.sync();  // both planes are the level's viscosity
+    double rmin = 0.0;
+    int it = 0;
+    for (;; it++) {
+        const double* V = (it & 1) ? B : A;
+        double* W = (it & 1) ? A : B;
+        const double f = phase == 0 ? __ldg(q.tabA + nn - 1) : __ldg(q.tabB + nn - 1);
+        unsigned long long m = kInf;
+        for (int p = gt; p < npts; p += gn) {
+            const int i = p % w, k = kmin + p / w;
+            const size_t x = IX(L, i, k);
+            const double v0 = ld_state(V + x), vm = ld_state(V + x - 1), vp = ld_state(V + x + 1);
+            const double vzm = ld_state(V + x - ld), vzp = ld_state(V + x + ld);
+            const double dts = __ldg(dtv + x) * 0.99;
+            const double v = v0 + f * dts * vis_laplacian<METRIC>(c, i, k, v0, vm, vp, vzm, vzp);
+            store_with_sides(L, W + IX(L, 0, k), i, v);
+            // (the reciprocals of rows beyond walls at RaT != 0 are not read by the passes)
+            if (!RaTnz) store_mirror_rows(L, W, i, k, v, 0, visT2);
+            if (!q.interpolate && i >= 1 && i <= a - 1 && k >= 1 && k <= b - 1) {
+                VisDiff d;
+                const double rat = point_ratio(V, x, i, k, v0, vm, vp, vzm, vzp, d);
+                m = min(m, (unsigned long long)__double_as_longlong(rat));
+            }
+        }
+        if (q.interpolate) cl.sync();
+        else rmin = level_min(m, it & 1);
+        // k_vflt_check
+        bool stop;
+        if (q.option == 1) {
+            stop = (nvis >= 1 && rmin > q.eig_ratio_min) || n > 20;
+            if (stop) {
+                fine = true;
+                n_eta = n;
+            }
+        } else if (q.interpolate == 0) {
+            stop = rmin > q.eig_ratio;
+            if (stop) nstore = nn;
+        } else {
+            stop = nvis >= 1;
+        }
+        if (stop) break;
+        if (++guard > q.cap) {
+            status = TC_ERR_LOOP_CAP;
+            more = false;
+        }
+        if (++nn > niter) next_outer();
+        if (!more) break;
+    }
+    const double* V = (it & 1) ? B : A;
+    unsigned long long m = kInf;
+    for (int p = gt; p < (a - 1) * (b - 1); p += gn) {
+        const int i = 1 + p % (a - 1), k = 1 + p / (a - 1);
+        const size_t x = IX(L, i, k);
+        VisDiff d;
+        const double rat = point_ratio(V, x, i, k, ld_state(V + x), ld_state(V + x - 1), ld_state(V + x + 1),
+                                       ld_state(V + x - ld), ld_state(V + x + ld), d);
+        if (vx != nullptr) {
+            vx[x] = d.r; vz[x] = d.s; vxx[x] = d.rr; vzz[x] = d.ss; vxz[x] = d.rs;
+        }
+        ratio[x] = rat;
+        m = min(m, (unsigned long long)__double_as_longlong(rat));
+    }
+    rmin = level_min(m, (it + 1) & 1);
+    if (it & 1)
+        for (int p = gt; p < (a + 1 + 2 * SP) * (b + 1); p += gn) {
+            const size_t x = IX(L, p % (a + 1 + 2 * SP) - SP, p / (a + 1 + 2 * SP));
+            A[x] = ld_state(B + x);
+        }
+    if (it > 0)
+        for (int p = gt; p < npts; p += gn) {
+            const int i = p % w, k = kmin + p / w;
+            if (k <= SP || k >= b - SP) store_mirror_rows(L, A, i, k, ld_state(V + IX(L, i, k)), RaTnz, visT2);
+        }
+    if (gt == 0) {
+        ds->ratio_min = rmin;
+        ds->vis_nvis_store = nvis;
+        ds->vis_nn_store = nstore;
+        if (fine) {
+            ds->eig_fine = rmin;
+            ds->n_eta = n_eta;
+        }
+        if (status != 0) ds->flt_status = status;
+    }
+}
+bool vis_filter_fits(const Level& lv, int interpolate) {
+    const int points = (lv.L.a + 1) * (lv.L.b + 1);
+    return points <= (interpolate ? VF_MAX_SMOOTH : lv.c.M.on ? VF_MAX_RATIO_METRIC : VF_MAX_RATIO);
+}
+void launch_vis_filter(cudaStream_t s, const Level& lv, const VisFltArgs& q, int reset, const double* src, double* A,
+                       double* B, int derivatives, int kmin, int kmax, int RaT_nonzero, double visT2,
+                       DevScalars* ds) {
+    const int npts = (lv.L.a + 1) * (kmax - kmin + 1);
+    const int nt = std::min(VF_THREADS, (npts + 128 * VF_CL - 1) / (128 * VF_CL) * 128);
+    auto kernel = lv.c.M.on ? k_vis_filter<true> : k_vis_filter<false>;
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)std::min(VF_CL, (npts + nt - 1) / nt), 1, 1);
+    cfg.blockDim = dim3(nt, 1, 1);
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = cfg.gridDim.x;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, lv.L, lv.c, q, reset, src, A, B, (const double*)lv.dt_vis, kmin, kmax,
+                       RaT_nonzero, visT2, derivatives ? lv.vx : nullptr, lv.vz, lv.vxx, lv.vzz, lv.vxz, lv.ratio, ds); tc_note_launch();
 }
 
 // ---------------------------------------------------------------------------

@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(BuildShape<T>::threads, 1) k_subcycle_build(Su
     bool pa[kPPT];
     T cf[kPPT][TC_NCOEF], dt[kPPT], rq[kPPT];
     int gn[kPPT], gidx[kPPT][3];
-    T gsg[kPPT][3];
+    bool neg[kPPT][3];  // the ghosts' signs
     // threads in rows of rpad slots (a1 rounded up to whole warps) when
     // that many fit, so that no warp's taps straddle two rows (which puts
     // two lanes on one shared-memory bank); else a1 slots per row
@@ -159,7 +159,9 @@ __global__ void __launch_bounds__(BuildShape<T>::threads, 1) k_subcycle_build(Su
         for (int d = 0; d < TC_NCOEF; d++) cf[q][d] = pa[q] ? __ldg(A.coef + px[q] + d * A.LS.plane) : T(0);
         dt[q] = pa[q] ? __ldg(A.dts + px[q]) : T(0);
         rq[q] = (pa[q] && p == j) ? T(1) : T(0);
-        gn[q] = pa[q] ? ghost_targets<T>(A.LS, pi[q], pk[q], A.Vbc, gidx[q], gsg[q]) : 0;
+        T sg[3] = {T(1), T(1), T(1)};
+        gn[q] = pa[q] ? ghost_targets<T>(A.LS, pi[q], pk[q], A.Vbc, gidx[q], sg) : 0;
+        for (int g = 0; g < 3; g++) neg[q][g] = sg[g] < T(0);
     }
     __syncthreads();
     if (tid == 0) R[IX(A.LS, 1 + j % a1, 1 + j / a1)] = T(1);
@@ -167,7 +169,7 @@ __global__ void __launch_bounds__(BuildShape<T>::threads, 1) k_subcycle_build(Su
     // store_stream of v at this thread's point q into S
     auto put = [&](T* S, int q, T v) {
         S[px[q]] = v;
-        for (int g = 0; g < gn[q]; g++) S[gidx[q][g]] = gsg[q][g] * v;
+        for (int g = 0; g < gn[q]; g++) S[gidx[q][g]] = flip_sign(v, neg[q][g]);
     };
     // one visit of Nmulti sweeps from Sa (ping-pong with Sb); returns the plane holding the result
     auto visit = [&](T* Sa, T* Sb, int up) -> T* {

@@ -457,9 +457,8 @@ tc_status filter_state_to_host(Handle* h) {
     return TC_OK;
 }
 
-// Launches a filter graph (n_pre kernels before its WHILE node), first
-// handing the module scalars over to the device.
-tc_status launch_filter_graph(Handle* h, cudaGraphExec_t ge, int n_pre) {
+// Hands the module scalars over to the device (before a device loop runs).
+tc_status filter_state_to_device(Handle* h) {
     if (!h->flt_dev_state) {
         DevScalars init{};
         init.vis_nvis_store = h->Nvis_store;
@@ -475,6 +474,12 @@ tc_status launch_filter_graph(Handle* h, cudaGraphExec_t ge, int n_pre) {
         CK(cudaStreamSynchronize(h->st));
         h->flt_dev_state = true;
     }
+    return TC_OK;
+}
+
+// Launches a filter graph (n_pre kernels before its WHILE node).
+tc_status launch_filter_graph(Handle* h, cudaGraphExec_t ge, int n_pre) {
+    TRY(filter_state_to_device(h));
     CK(cudaGraphLaunch(ge, h->st));
     tc_note_launch(n_pre);
     return TC_OK;
@@ -691,8 +696,15 @@ void grad_eig(Handle* h, int level, bool eig) {
     if (eig) h->ratio_level = (h->p.ivis != 0) ? level : 0;
 }
 
-// smoother_vis (smoother.f90:166-263)
-tc_status smoother_vis(Handle* h, int level, int interpolate) {
+// the whole loop of smoother_vis in one launch (k_mg.cu)
+bool vis_filter_runs(const Handle* h, int level, int interpolate) {
+    const bool device = h->capturing || !(h->flt_failed || h->no_graphs || h->no_device_loop);
+    return h->fuse_visits && h->p.ivis != 0 && device && vis_filter_fits(h->lev[level], interpolate);
+}
+
+// smoother_vis (smoother.f90:166-263); work: smooth a copy of the viscosity there and leave
+// the level's own viscosity and derivatives (where vis_filter_runs)
+tc_status smoother_vis(Handle* h, int level, int interpolate, double* work = nullptr) {
     Level& lv = h->lev[level];
     int option, Niter;
     double lb, la;
@@ -723,31 +735,45 @@ tc_status smoother_vis(Handle* h, int level, int interpolate) {
         double* cur = lv.vis[lv.vcur];
         double* oth = lv.vis[1 - lv.vcur];
         const size_t by = sizeof(double) * lv.L.plane;
+        if (vis_filter_runs(h, level, interpolate)) {
+            if (!h->capturing) TRY(filter_state_to_device(h));
+            launch_vis_filter(h->st, lv, fa, reset, cur, work ? work : cur, oth, work ? 0 : 1, kmin, kmax, RaTnz,
+                              visT2, h->ds);
+            h->ratio_level = level;
+            return TC_OK;
+        }
+        // the test reads no eigenvalue ratio where it interpolates: one gradient after the loop
+        const int nk = interpolate ? 2 : 3;
         auto pre = [&](cudaGraphConditionalHandle c) {
             if (cudaMemcpyAsync(oth, cur, by, cudaMemcpyDeviceToDevice, h->st) != cudaSuccess)
                 h->enq_err = cudaErrorUnknown;
             launch_vflt_init(h->st, h->ds, reset, fa);
-            launch_vis_grad(h->st, lv, cur, 1, h->p.ivis, h->rs, h->ds);
-            launch_vflt_check(h->st, h->ds, fa, 3, c);
+            if (!interpolate) launch_vis_grad(h->st, lv, cur, 1, h->p.ivis, h->rs, h->ds);
+            launch_vflt_check(h->st, h->ds, fa, nk, c);
         };
         auto body = [&](cudaGraphConditionalHandle c) {
             launch_vis_smooth(h->st, lv, cur, oth, 0.0, kmin, kmax, RaTnz, visT2, &h->ds->flt_c);
             if (cudaMemcpyAsync(cur, oth, by, cudaMemcpyDeviceToDevice, h->st) != cudaSuccess)
                 h->enq_err = cudaErrorUnknown;
-            launch_vis_grad(h->st, lv, cur, 1, h->p.ivis, h->rs, h->ds);
-            launch_vflt_check(h->st, h->ds, fa, 3, c);
+            if (!interpolate) launch_vis_grad(h->st, lv, cur, 1, h->p.ivis, h->rs, h->ds);
+            launch_vflt_check(h->st, h->ds, fa, nk, c);
+        };
+        auto done = [&]() {
+            if (interpolate) launch_vis_grad(h->st, lv, cur, 1, h->p.ivis, h->rs, h->ds);
+            h->ratio_level = (h->p.ivis != 0) ? level : 0;  // grad_eig's, run at least once
         };
         if (h->capturing) {
             long long nb;
             emit_while(h, pre, body, &nb);
-            h->ratio_level = (h->p.ivis != 0) ? level : 0;
+            done();
             return TC_OK;
         }
         cudaGraphExec_t ge = filter_graph(h, kFltVis * 1000 + level * 10 + interpolate,
                                           [&](cudaGraphExec_t* out) { return build_while_graph(h, pre, body, out); });
         if (ge) {
-            h->ratio_level = (h->p.ivis != 0) ? level : 0;  // grad_eig's, run at least once
-            return launch_filter_graph(h, ge, 3);
+            TRY(launch_filter_graph(h, ge, nk));
+            done();
+            return TC_OK;
         }
         TRY(filter_state_to_host(h));
     }
@@ -812,15 +838,16 @@ tc_status compute_viscosity(Handle* h, int level) {
     Level& f = h->lev[l1];
     Level& c = h->lev[level];
     const size_t by = sizeof(double) * f.L.plane;
+    const bool copy = !vis_filter_runs(h, l1, 1);  // else the filter works on a copy itself
     double* src[6] = {cur_vis(h, l1), f.vx, f.vz, f.vxx, f.vzz, f.vxz};
-    for (int q = 0; q < 6; q++) CK(cudaMemcpyAsync(f.bak[q], src[q], by, cudaMemcpyDeviceToDevice, h->st));
-    TRY(smoother_vis(h, l1, 1));
-    launch_restrict_vis(h->st, c, f, cur_vis(h, l1), cur_vis(h, level));
+    for (int q = 0; copy && q < 6; q++) CK(cudaMemcpyAsync(f.bak[q], src[q], by, cudaMemcpyDeviceToDevice, h->st));
+    TRY(smoother_vis(h, l1, 1, copy ? nullptr : f.bak[0]));
+    launch_restrict_vis(h->st, c, f, copy ? cur_vis(h, l1) : f.bak[0], cur_vis(h, level));
     launch_vis_bcs_init(h->st, c, cur_vis(h, level), h->p.RaT != 0.0 ? 1 : 0, h->p.visT * h->p.visT);
     if (level < h->grids) TRY(smoother_vis(h, level, 0));
     else grad_eig(h, level, false);
     double* dst[6] = {cur_vis(h, l1), f.vx, f.vz, f.vxx, f.vzz, f.vxz};
-    for (int q = 0; q < 6; q++) CK(cudaMemcpyAsync(dst[q], f.bak[q], by, cudaMemcpyDeviceToDevice, h->st));
+    for (int q = 0; copy && q < 6; q++) CK(cudaMemcpyAsync(dst[q], f.bak[q], by, cudaMemcpyDeviceToDevice, h->st));
     return TC_OK;
 }
 

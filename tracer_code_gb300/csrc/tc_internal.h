@@ -221,6 +221,10 @@ void launch_vis_grad(cudaStream_t s, const Level& lv, const double* vis, int do_
 void launch_vis_smooth(cudaStream_t s, const Level& lv, const double* vin, double* vout, double c, int kmin,
                        int kmax, int RaT_nonzero, double visT2, const double* cdev = nullptr);
 void launch_restrict_vis(cudaStream_t s, const Level& coarse, const Level& fine, const double* vfine, double* vcoarse);
+bool vis_filter_fits(const Level& lv, int interpolate);
+void launch_vis_filter(cudaStream_t s, const Level& lv, const VisFltArgs& q, int reset, const double* src, double* A,
+                       double* B, int derivatives, int kmin, int kmax, int RaT_nonzero, double visT2,
+                       DevScalars* ds);
 void launch_vis_bcs_init(cudaStream_t s, const Level& coarse, double* v, int RaT_nonzero, double visT2);
 void launch_level_coefs(cudaStream_t s, const Level& lv, const double* vis, int ivis, double courant_stream,
                         int cheb_level, bool with_dt = true);
