@@ -208,6 +208,38 @@ __global__ void k_win_init(Lay L, Range2 r, const double* __restrict__ coef, con
     if (adnn) adnn[x] = an;
 }
 
+// One step of warp_sums: of N values of which this lane has to finish cnt, the lanes with
+// bit OFF take the second half and the others the first, each adding the other's.
+template <int N, int OFF>
+__device__ __forceinline__ void sum_step(double* s, int& base, int& cnt) {
+    constexpr int H = (N + 1) / 2;
+    const bool up = (threadIdx.x & OFF) != 0;
+#pragma unroll
+    for (int t = 0; t < H; t++) {
+        const double second = H + t < N ? s[H + t] : 0.0;
+        const double keep = up ? second : s[t], give = up ? s[t] : second;
+        s[t] = keep + __shfl_xor_sync(0xffffffffu, give, OFF);
+    }
+    base += up ? H : 0;
+    cnt = up ? max(cnt - H, 0) : min(cnt, H);
+}
+// The warp's sums of N values per lane, each by the tree of shuffles over 16, 8, 4, 2 and 1
+// lanes, in N + 1 additions (of 64 cycles each) instead of 5 N: every lane ends with at
+// most one sum, s[0] of value `base` where it returns true.
+template <int N>
+__device__ __forceinline__ bool warp_sums(double* s, int& base) {
+    constexpr int N1 = (N + 1) / 2, N2 = (N1 + 1) / 2, N3 = (N2 + 1) / 2, N4 = (N3 + 1) / 2;
+    static_assert((N4 + 1) / 2 == 1, "more sums than lanes");
+    base = 0;
+    int cnt = N;
+    sum_step<N, 16>(s, base, cnt);
+    sum_step<N1, 8>(s, base, cnt);
+    sum_step<N2, 4>(s, base, cnt);
+    sum_step<N3, 2>(s, base, cnt);
+    sum_step<N4, 1>(s, base, cnt);
+    return cnt > 0;
+}
+
 // the grid-stride sums for ND directions
 template <int ND>
 __device__ __forceinline__ void win_sums(const Lay& L, const double* __restrict__ coef, const double* rhs,
@@ -281,25 +313,27 @@ __global__ void __launch_bounds__(256) k_win_dots(Lay L, const double* __restric
         case 4: win_sums<4>(L, coef, rhs, psi, prev, rp, P, AP, rn, adnn, snew, nold, s); break;
         default: win_sums<kWD>(L, coef, rhs, psi, prev, rp, P, AP, rn, adnn, snew, nold, s); break;
     }
-    // block sums (warp shuffle, then one warp over the warps' partials)
-    __shared__ double sh[kWS][16];
+    // block sums: each warp's, then a lane per sum over the eight warps in the order of a
+    // warp's tree
+    __shared__ double sh[8][kWS];
     __shared__ bool last;
     const int tid = threadIdx.x, bid = blockIdx.x, nb = gridDim.x;
-#pragma unroll
-    for (int q = 0; q < kWS; q++) {
-        double v = s[q];
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-        if ((tid & 31) == 0) sh[q][tid >> 5] = v;
+    {
+        int q;
+        if (warp_sums<kWS>(s, q)) sh[tid >> 5][q] = s[0];
     }
     __syncthreads();
     if (tid < 32) {
-        for (int q = 0; q < kWS; q++) {
-            double v = (tid < (int)(blockDim.x >> 5)) ? sh[q][tid] : 0.0;
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-            if (tid == 0) rs.part[(size_t)q * nb + bid] = v;
-        }
-        if (tid == 0) {
+        if (tid < kWS) {
+            double v[8];
+#pragma unroll
+            for (int w = 0; w < 8; w++) v[w] = sh[w][tid];
+            rs.part[(size_t)tid * nb + bid] =
+                ((v[0] + v[4]) + (v[2] + v[6])) + ((v[1] + v[5]) + (v[3] + v[7]));
             __threadfence();
+        }
+        __syncwarp();
+        if (tid == 0) {
             const unsigned int t = atomicAdd(rs.count, 1u);
             last = (t == (unsigned int)(nb - 1));
         }
@@ -331,56 +365,65 @@ __global__ void __launch_bounds__(256) k_win_dots(Lay L, const double* __restric
         }
     }
     __syncthreads();
-    if (tid == 0) {
+    if (tid < 32) {
         // LDL^T of G in direction order, dropping a direction whose pivot
         // falls below 1e-10 of its diagonal (nearly in the span of the kept
         // ones) or whose diagonal is not positive; then G beta = b on the
-        // kept directions
-        double G[kWD][kWD], Lm[kWD][kWD], D[kWD], y[kWD], beta[kWD];
+        // kept directions.  Lane i has row i: an FP64 operation takes a warp as
+        // long as a thread.
+        const int i = min(tid, kWD - 1);
+        double g[kWD], l[kWD], D[kWD], beta[kWD];
         bool keep[kWD];
-        int t = 0;
-        for (int i = 0; i < kWD; i++)
-            for (int j = i; j < kWD; j++) {
-                G[i][j] = tot[t];
-                G[j][i] = tot[t];
-                t++;
-            }
-        for (int i = 0; i < kWD; i++) {
-            keep[i] = false;
-            D[i] = 0.0;
-            beta[i] = 0.0;
-            y[i] = 0.0;
-            for (int j = 0; j < kWD; j++) Lm[i][j] = 0.0;
+        __shared__ double sl[kWD][kWD], sz[kWD];
+#pragma unroll
+        for (int j = 0; j < kWD; j++) {
+            const int lo = min(i, j), hi = max(i, j);
+            g[j] = tot[lo * kWD - lo * (lo - 1) / 2 + hi - lo];
+            l[j] = D[j] = beta[j] = 0.0;
+            keep[j] = false;
         }
-        for (int j = 0; j < nd; j++) {
-            double dj = G[j][j];
+#pragma unroll
+        for (int j = 0; j < kWD; j++) {
+            if (j >= nd) break;
+            double v = g[j];
+#pragma unroll
             for (int k = 0; k < j; k++)
-                if (keep[k]) dj -= Lm[j][k] * Lm[j][k] * D[k];
-            if (!(G[j][j] > 0.0) || !(dj > 1e-10 * G[j][j])) continue;
+                if (keep[k]) v -= l[k] * __shfl_sync(0xffffffffu, l[k], j) * D[k];
+            const double dj = __shfl_sync(0xffffffffu, v, j), gj = __shfl_sync(0xffffffffu, g[j], j);
+            if (!(gj > 0.0) || !(dj > 1e-10 * gj)) continue;
             keep[j] = true;
             D[j] = dj;
-            Lm[j][j] = 1.0;
-            for (int i = j + 1; i < nd; i++) {
-                double v = G[i][j];
-                for (int k = 0; k < j; k++)
-                    if (keep[k]) v -= Lm[i][k] * Lm[j][k] * D[k];
-                Lm[i][j] = v / dj;
+            if (i > j) l[j] = v / dj;
+            else if (i == j) l[j] = 1.0;
+        }
+        double y = tot[kWT + i];
+#pragma unroll
+        for (int k = 0; k < kWD; k++)
+            if (keep[k]) {
+                const double yk = __shfl_sync(0xffffffffu, y, k);
+                if (i > k) y -= l[k] * yk;
             }
+        double di = 1.0;
+#pragma unroll
+        for (int k = 0; k < kWD; k++)
+            if (k == i && keep[k]) di = D[k];
+        const double z = y / di;
+        if (tid < kWD) {
+            sz[tid] = z;
+#pragma unroll
+            for (int k = 0; k < kWD; k++) sl[tid][k] = l[k];
         }
-        for (int i = 0; i < nd; i++) {
-            if (!keep[i]) continue;
-            double v = tot[kWT + i];
-            for (int k = 0; k < i; k++)
-                if (keep[k]) v -= Lm[i][k] * y[k];
-            y[i] = v;
+        __syncwarp();
+#pragma unroll
+        for (int r = kWD - 1; r >= 0; r--) {
+            if (!keep[r]) continue;
+            double v = sz[r];
+#pragma unroll
+            for (int k = r + 1; k < kWD; k++)
+                if (keep[k]) v -= sl[k][r] * beta[k];
+            beta[r] = v;
         }
-        for (int i = nd - 1; i >= 0; i--) {
-            if (!keep[i]) continue;
-            double v = y[i] / D[i];
-            for (int k = i + 1; k < nd; k++)
-                if (keep[k]) v -= Lm[k][i] * beta[k];
-            beta[i] = v;
-        }
+        if (tid != 0) return;
         for (int i = 0; i < kWD; i++) ds->win_beta[i] = beta[i];
         ds->win_nd = nd;
         ds->win_dnn = dnn_now;
