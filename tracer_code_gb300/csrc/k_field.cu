@@ -91,19 +91,26 @@ void launch_smoothness(cudaStream_t s, const Lay& L, const double* f, RedScratch
     k_smoothness<<<grid_for(r), dim3(BX, BY), 0, s>>>(L, r, f, rs, &ds->diff); tc_note_launch();
 }
 
-__device__ __forceinline__ double lap5(const double* __restrict__ T, size_t x, size_t ld, double dr2, double ds2) {
-    double c = T[x];
-    double Trr = (T[x - 1] + -2.0 * c + T[x + 1]) / dr2;
-    double Tss = (T[x - ld] + -2.0 * c + T[x + ld]) / ds2;
-    return Trr + Tss;
+// second differences over dr2 and ds2
+__device__ __forceinline__ double diff_rr(const Phys& P, const double* __restrict__ T, size_t x) {
+    return spacing_quot(second_diff(T[x - 1], T[x], T[x + 1]), P.dr2, P.rdr2, P.dr_pow2);
+}
+__device__ __forceinline__ double diff_ss(const Phys& P, const double* __restrict__ T, size_t x, size_t ld) {
+    return spacing_quot(second_diff(T[x - ld], T[x], T[x + ld]), P.ds2, P.rds2, P.ds_pow2);
+}
+// first differences over dr and ds
+__device__ __forceinline__ double diff_r(const Phys& P, const double* __restrict__ T, size_t x) {
+    return first_diff(T[x - 1], T[x + 1], P.dr, P.rdr, P.dr_pow2);
+}
+__device__ __forceinline__ double diff_s(const Phys& P, const double* __restrict__ T, size_t x, size_t ld) {
+    return first_diff(T[x - ld], T[x + ld], P.ds, P.rds, P.ds_pow2);
 }
 // smoother_space (smoother.f90:122-140) at node (i, k), stretched or uniform
 __device__ __forceinline__ double smoother_space(const Phys& P, const double* __restrict__ T, size_t x, size_t ld,
                                                  int i, int k) {
-    if (!P.M.on) return lap5(T, x, ld, P.dr2, P.ds2);
-    const double c = T[x];
-    const double Tr = (-0.5 * T[x - 1] + 0.5 * T[x + 1]) / P.dr, Ts = (-0.5 * T[x - ld] + 0.5 * T[x + ld]) / P.ds;
-    const double Trr = (T[x - 1] + -2.0 * c + T[x + 1]) / P.dr2, Tss = (T[x - ld] + -2.0 * c + T[x + ld]) / P.ds2;
+    const double Trr = diff_rr(P, T, x), Tss = diff_ss(P, T, x, ld);
+    if (!P.M.on) return Trr + Tss;
+    const double Tr = diff_r(P, T, x), Ts = diff_s(P, T, x, ld);
     const double x1 = mt(P.M.xr, i), z1 = mt(P.M.zs, k);
     const double Tx = Tr / x1, Tz = Ts / z1;
     const double Txx = (Trr - Tx * mt(P.M.xrr, i)) / (x1 * x1);
@@ -165,8 +172,8 @@ __global__ void k_conduct_grad(Lay L, Phys P, Range2 r, const double* __restrict
     if (!inr) return;
     const size_t ld = (size_t)L.ld;
     size_t x = IX(L, i, k);
-    cr[x] = (-0.5 * cd[x - 1] + 0.5 * cd[x + 1]) / P.dr;
-    cs[x] = (-0.5 * cd[x - ld] + 0.5 * cd[x + ld]) / P.ds;
+    cr[x] = diff_r(P, cd, x);
+    cs[x] = diff_s(P, cd, x, ld);
 }
 void launch_conductivity(cudaStream_t s, const Lay& L, const Phys& P, const double* const* Cvis, double* conduct,
                          double* conduct_r, double* conduct_s) {
@@ -183,12 +190,12 @@ void launch_conductivity(cudaStream_t s, const Lay& L, const Phys& P, const doub
 __device__ __forceinline__ double uf_(const Lay& L, const Phys& P, const double* SF, int i, int k) {
     const size_t ld = (size_t)L.ld;
     size_t x = IX(L, i, k);
-    const double SFs = (-0.5 * SF[x - ld] + 0.5 * SF[x + ld]) / P.ds;
+    const double SFs = diff_s(P, SF, x, ld);
     return P.M.on ? SFs / mt(P.M.zs, k) : SFs;
 }
 __device__ __forceinline__ double wf_(const Lay& L, const Phys& P, const double* SF, int i, int k) {
     size_t x = IX(L, i, k);
-    const double SFr = (-0.5 * SF[x - 1] + 0.5 * SF[x + 1]) / P.dr;
+    const double SFr = diff_r(P, SF, x);
     return -(P.M.on ? SFr / mt(P.M.xr, i) : SFr);
 }
 __global__ void k_velocities(Lay L, Phys P, Range2 r, const double* __restrict__ SF, double* __restrict__ u,
@@ -235,7 +242,7 @@ __global__ void k_derivatives(Lay L, Phys P, Range2 r, const double* __restrict_
     RANGE_IK(r);
     if (!inr) return;
     size_t x = IX(L, i, k);
-    der[x] = (-0.5 * f[x - 1] + 0.5 * f[x + 1]) / P.dr;
+    der[x] = diff_r(P, f, x);
 }
 void launch_derivatives(cudaStream_t s, const Lay& L, const Phys& P, const double* f, double* der) {
     Range2 r{0, L.a, -1, L.b + 1};
@@ -313,11 +320,8 @@ __global__ void k_energy(Lay L, Phys P, Range2 r, int stage, const double* __res
     if (!inr) return;
     const size_t ld = (size_t)L.ld;
     size_t x = IX(L, i, k);
-    double Tr = (-0.5 * Tin[x - 1] + 0.5 * Tin[x + 1]) / P.dr;
-    double Ts = (-0.5 * Tin[x - ld] + 0.5 * Tin[x + ld]) / P.ds;
-    double c = Tin[x];
-    double Trr = (Tin[x - 1] + -2.0 * c + Tin[x + 1]) / P.dr2;
-    double Tss = (Tin[x - ld] + -2.0 * c + Tin[x + ld]) / P.ds2;
+    const double Tr = diff_r(P, Tin, x), Ts = diff_s(P, Tin, x, ld);
+    const double Trr = diff_rr(P, Tin, x), Tss = diff_ss(P, Tin, x, ld);
     double kx = cr[x], kz = cs[x];
     double heat;
     if (P.comp == 0) heat = P.H;
@@ -372,10 +376,8 @@ __global__ void k_strain(Lay L, Phys P, Range2 r, const double* __restrict__ u, 
     if (!inr) return;
     const size_t ld = (size_t)L.ld;
     size_t x = IX(L, i, k);
-    double ur = (-0.5 * u[x - 1] + 0.5 * u[x + 1]) / P.dr;
-    double us = (-0.5 * u[x - ld] + 0.5 * u[x + ld]) / P.ds;
-    double wr = (-0.5 * w[x - 1] + 0.5 * w[x + 1]) / P.dr;
-    double ws = (-0.5 * w[x - ld] + 0.5 * w[x + ld]) / P.ds;
+    double ur = diff_r(P, u, x), us = diff_s(P, u, x, ld);
+    double wr = diff_r(P, w, x), ws = diff_s(P, w, x, ld);
     if (P.M.on) {
         // ux = ur / xr, uz = us / zs, wx = wr / xr, wz = ws / zs (momentum.f90:45-48)
         const double x1 = mt(P.M.xr, i), z1 = mt(P.M.zs, k);

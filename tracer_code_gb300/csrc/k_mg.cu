@@ -127,28 +127,17 @@ __device__ void eig_pair_metric(const LevConst& c, int i, int k, double v, doubl
     }
 }
 
-// x / h for a spacing h > 0 with hinv = RN(1 / h): a product where the spacings are
-// powers of two, else two Newton corrections (Markstein, as quot_round in k_tracer.cu)
-__device__ __forceinline__ double spacing_quot(double x, double h, double hinv, int recip) {
-    if (recip) return x * hinv;
-    const unsigned hi = (unsigned)__double2hiint(x), ex = hi >> 20 & 0x7ff;
-    if (ex - 200u > 1600u) return ((hi << 1) | (unsigned)__double2loint(x)) != 0 ? x / h : x;
-    double q = x * hinv;
-    q = fma(fma(-q, h, x), hinv, q);
-    return fma(fma(-q, h, x), hinv, q);
-}
 // viscosity_gradients' differences, -0.5 vm + 0.5 vp over dr and so on.  The factors that
 // are powers of two are exact, so they go into the spacing; half the FP64 operations.
 struct VisDiff {
     double r, rr, s, ss, rs;
 };
-__device__ __forceinline__ double second_diff(double m, double c, double p) { return fma(-2.0, c, m) + p; }
 __device__ __forceinline__ VisDiff vis_diff(const LevConst& c, double v0, double vm, double vp, double vzm, double vzp,
                                             double mm, double pm, double mp, double pp) {
     VisDiff d;
-    d.r = spacing_quot(vp - vm, 2.0 * c.dr, 0.5 * c.rdr, c.recip);
+    d.r = first_diff(vm, vp, c.dr, c.rdr, c.recip);
     d.rr = spacing_quot(second_diff(vm, v0, vp), c.dr2, c.rdr2, c.recip);
-    d.s = spacing_quot(vzp - vzm, 2.0 * c.ds, 0.5 * c.rds, c.recip);
+    d.s = first_diff(vzm, vzp, c.ds, c.rds, c.recip);
     d.ss = spacing_quot(second_diff(vzm, v0, vzp), c.ds2, c.rds2, c.recip);
     d.rs = spacing_quot(((mm - pm) - mp) + pp, 4.0 * c.drds, 0.25 * c.rdrds, c.recip);
     return d;
@@ -182,8 +171,7 @@ __device__ __forceinline__ double vis_laplacian(const LevConst& c, int i, int k,
     const double Trr = spacing_quot(second_diff(vm, v0, vp), c.dr2, c.rdr2, c.recip);
     const double Tss = spacing_quot(second_diff(vzm, v0, vzp), c.ds2, c.rds2, c.recip);
     if (!METRIC) return Trr + Tss;
-    const double Tr = spacing_quot(vp - vm, 2.0 * c.dr, 0.5 * c.rdr, c.recip);
-    const double Ts = spacing_quot(vzp - vzm, 2.0 * c.ds, 0.5 * c.rds, c.recip);
+    const double Tr = first_diff(vm, vp, c.dr, c.rdr, c.recip), Ts = first_diff(vzm, vzp, c.ds, c.rds, c.recip);
     const int i1 = i * c.mf, k1 = k * c.mf;
     const double x1 = mt(c.M.xr, i1), x2 = mt(c.M.xrr, i1), z1 = mt(c.M.zs, k1), z2 = mt(c.M.zss, k1);
     const double Tx = Tr / x1, Tz = Ts / z1;
@@ -1815,13 +1803,13 @@ __global__ void k_rhs1(Lay L, Phys P, Range2 r, const double* __restrict__ Tb, C
         // dx/dr at node i (1 on a uniform grid, where the division is skipped)
         const double x1 = P.M.on ? mt(P.M.xr, i) : 1.0;
         if (P.RaT != 0.0) {
-            double Tr = (-0.5 * Tb[x - 1] + 0.5 * Tb[x + 1]) / P.dr;
+            double Tr = first_diff(Tb[x - 1], Tb[x + 1], P.dr, P.rdr, P.dr_pow2);
             if (P.M.on) Tr = Tr / x1;
             R = P.RaT * Tr;
         }
         if (P.comp == 1)
             for (int j = 0; j < P.ntype; j++) {
-                double Cr = (-0.5 * Cb.p[j][x - 1] + 0.5 * Cb.p[j][x + 1]) / P.dr;
+                double Cr = first_diff(Cb.p[j][x - 1], Cb.p[j][x + 1], P.dr, P.rdr, P.dr_pow2);
                 if (P.M.on) Cr = Cr / x1;
                 R = R - P.RaC[j] * Cr;
             }

@@ -1958,7 +1958,10 @@ tc_status create(Handle* h, const tc_params* in) {
         P.xn = dx;
         P.zn = dz;
         int e = 0;
-        P.ds_pow2 = (std::frexp(P.ds, &e) == 0.5) ? 1 : 0;
+        auto pow2 = [&](double x) { return std::frexp(x, &e) == 0.5; };
+        P.dr_pow2 = (pow2(P.dr) && pow2(P.dr2)) ? 1 : 0;
+        P.ds_pow2 = (pow2(P.ds) && pow2(P.ds2)) ? 1 : 0;
+        P.rdr2 = 1.0 / P.dr2; P.rds2 = 1.0 / P.ds2;
     }
     const size_t pl = h->L1.plane;
     double** fine[] = {&h->T, &h->T0, &h->T1, &h->T2, &h->SF, &h->Tvis, &h->Tvis2, &h->Tbuoy, &h->u, &h->w,

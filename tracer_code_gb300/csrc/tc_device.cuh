@@ -251,6 +251,24 @@ __device__ __forceinline__ void fold_from_fields(const FoldG32& F, const float* 
     }
 }
 
+// x / h for a spacing h > 0 with hinv = RN(1 / h): a product where the spacings are
+// powers of two, else two Newton corrections (Markstein, as quot_round in k_tracer.cu)
+__device__ __forceinline__ double spacing_quot(double x, double h, double hinv, int recip) {
+    if (recip) return x * hinv;
+    const unsigned hi = (unsigned)__double2hiint(x), ex = hi >> 20 & 0x7ff;
+    if (ex - 200u > 1600u) return ((hi << 1) | (unsigned)__double2loint(x)) != 0 ? x / h : x;
+    double q = x * hinv;
+    q = fma(fma(-q, h, x), hinv, q);
+    return fma(fma(-q, h, x), hinv, q);
+}
+// central differences over a spacing: (-0.5 m + 0.5 p) / h and m - 2 c + p, the factors that
+// are powers of two taken into the spacing or a multiply-add (exact; an FP64 operation of a
+// warp takes 64 cycles of its scheduler, a division ten)
+__device__ __forceinline__ double first_diff(double m, double p, double h, double hinv, int recip) {
+    return spacing_quot(p - m, 2.0 * h, 0.5 * hinv, recip);
+}
+__device__ __forceinline__ double second_diff(double m, double c, double p) { return fma(-2.0, c, m) + p; }
+
 // v or -v, as bits: signs change without the FP64 pipe
 __device__ __forceinline__ float flip_sign(float v, bool flip) { return flip ? -v : v; }
 __device__ __forceinline__ double flip_sign(double v, bool flip) {

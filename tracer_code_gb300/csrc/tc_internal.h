@@ -201,7 +201,8 @@ struct Phys {
     double aspect, dr, ds, dr2, ds2, dro2, dso2;
     double rdr, rds;             // 1/dr, 1/ds rounded (tracer cell indices: quot_trunc, quot_nint)
     const double *xn, *zn;       // i * dr for i = 0..nx+1, k * ds for k = 0..nz+1 (tracer offsets)
-    int ds_pow2;                 // ds is a power of two: x / ds = x * rds exactly
+    double rdr2, rds2;           // 1/dr2, 1/ds2
+    int dr_pow2, ds_pow2;        // dr (ds) is a power of two: x / dr = x * rdr exactly, and over dr2
     double RaT, RaC[TC_MAX_TYPES], lnvisT, lnvisP, lnvisC[TC_MAX_TYPES], visT2, H, Htype[TC_MAX_TYPES];
     double lncf[TC_MAX_TYPES];   // log(1/conduct_factor)
     double courantT, courantC;
