@@ -513,8 +513,9 @@ void launch_accel_window(cudaStream_t s, const Level& l1, double* psi, double* p
     // kernel's launch bounds), so that the block sums and their fold stay few
     // one CTA of 256 threads per SM, grid-stride over the points: the block
     // sums of the up to 20 FP64 products cost per thread, so few threads with
-    // several points each are fastest (measured at 1024x256: 1 x SMs 306 us per
-    // level-1 visit, 2 x 317, 3 x 326, 6 x 358; 512 threads 317)
+    // several points each are fastest (measured at 1024x256 with one smoother launch
+    // per sweep: 1 x SMs 306 us per level-1 visit, 2 x 317, 3 x 326, 6 x 358; 512 threads
+    // 317)
     int nb = (npts + 255) / 256;
     if (nb > nsm) nb = nsm;
     launch_pdl(k_win_dots, dim3((unsigned)nb), dim3(256), 0, s, l1.L, (const double*)l1.coef,
