@@ -980,7 +980,7 @@ __global__ void k_coarse_lu_global(double* __restrict__ AB, int* __restrict__ ip
 // cycle), search 600, reciprocal 620, message 400.  Everything else is kept off it.
 // Before, one cluster of 8 CTAs with the whole window in its shared memory, every
 // column's update on the chain: n = 10201, kl = 202 (a 200x200 grid halved once) 73 ms,
-// now 14.1; one CTA for n = 400, kl = 63: 2.36 ms, now 0.46.
+// now 12.7; one CTA for n = 400, kl = 63: 2.36 ms, now 0.46.
 #define LUP_NB 16
 #define LUP_CL 16              // CTAs of the panel's cluster: one per column
 #define LUP_WAIT (1 << 20)     // polls of a wait for a column's multipliers
@@ -1259,8 +1259,11 @@ bool launch_lu_panels(cudaStream_t s, double* band, int* ipiv, int n, int kl, in
     const size_t smem = sizeof(double) * 2 * LUP_NB * T;
     cudaFuncSetAttribute(k_lu_panel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     cudaFuncSetAttribute(k_lu_panel<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    // two to four columns behind the panel per SM, on up to eight clusters with the panel's
-    const int clusters = 1 + std::min(7, (kl + ku + 31) / 32);
+    // the columns behind the panel two to four per SM, on up to seven clusters with the
+    // panel's: an eighth of the chip stays free for the next launch's panel, whose CTAs then
+    // share no SM with this launch's (n = 2600, kl = 202: 3.23 ms; with eight clusters 3.62,
+    // with six 3.47)
+    const int clusters = 1 + std::min(6, (kl + ku + 31) / 32);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(LUP_CL * clusters, 1, 1);
     cfg.blockDim = dim3(2 * T, 1, 1);
