@@ -556,7 +556,7 @@ void launch_level_coefs(cudaStream_t s, const Level& lv, const double* vis, int 
 
 // One FP64 sweep, a point per thread.  What bounds it is the FP64 pipe, 14 operations a
 // point after the wait (c * dt is formed before it, ghost signs change as bits): 1024x256
-// points 8.6 -> 8.4 us a sweep with 17 before (floor 6.1), 512x128 3.5 -> 3.3.
+// points 8.6 -> 8.4 us a sweep with 17 before (now 8.2, floor 6.1), 512x128 3.5 -> 3.3.
 __global__ void __launch_bounds__(256, 1) k_sweep(Lay L, Range2 r, const double* Sin, double* Sout,
                         const double* __restrict__ coef, const double* rhs,
                         const double* __restrict__ dts, const double* __restrict__ cA, const double* __restrict__ cB,
@@ -571,11 +571,13 @@ __global__ void __launch_bounds__(256, 1) k_sweep(Lay L, Range2 r, const double*
         cd = c * __ldg(dts + x);
     }
     pdl_entry();
+    // the next sweep's blocks come in as this one's leave, their coefficients loaded meanwhile
+    // (released at the end: 590 -> 572 us for 70 sweeps of 1024x256, 264 -> 241 of 200x200)
+    pdl_done();
     if (!inr) return;
     double res = fold_apply(L, Sin, x, cf, ld_state(rhs + x));
     double v = fma(cd, res, ld_state(Sin + x));
     store_stream(L, Sout, i, k, v, Vbc);
-    pdl_done();
 }
 // one point per thread: the two-point kernel (k_sweep_x2<double>, 120 registers)
 // measured 18.3 against 8.5 us per level-1 sweep (half the resident warps)
