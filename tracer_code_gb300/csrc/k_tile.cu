@@ -331,13 +331,16 @@ __device__ __forceinline__ void load_tile(float* buf, int bsz, int R, const Lay&
 // signal arrive together and no fence is needed.  An inbox has two sides used in
 // turn; a side is written again only after its owner has sent the edge of the
 // exchange between, i.e. after it has read the side.  Numbers go on from visit
-// to visit (each CTA keeps its own count in global memory).
+// to visit: a level has one count per tile of its largest tiling, all of them
+// equal between visits (the uniform and the per-point factor may take different
+// tilings, so a visit also moves on the counts of tiles that it does not have).
 //
 // Waits are bounded: past the limit the CTA waits no more, finishes its loop
 // and reports the timeout.
 struct Exchange {
     unsigned long long* inbox;  // per tile 2 sides of W * R words (grid)
-    unsigned* count;            // per tile: exchanges so far (grid)
+    unsigned* count;            // per tile of the level's largest tiling: exchanges so far (grid)
+    int counts;                 // how many
 };
 __device__ __forceinline__ void st_words(unsigned long long* p, unsigned long long a, unsigned long long b) {
     asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"(a), "l"(b) : "memory");
@@ -532,8 +535,10 @@ __global__ void __launch_bounds__(NT, 1) k_tile_visit(const __grid_constant__ Ti
     }
     dead = __syncthreads_or(dead ? 1 : 0) != 0;
     if (GRID) {
-        // every CTA counts the same exchanges, whether its waits ran out or not
-        if (tid == 0) X.count[me] = count0 + (unsigned)((Q.nsweeps + S - 1) / S);
+        // every CTA counts the same exchanges, whether its waits ran out or not, and those
+        // of the tiles beyond this visit's tiling
+        for (int t = me + tid * (int)gridDim.x; t < X.counts; t += nth * (int)gridDim.x)
+            X.count[t] = count0 + (unsigned)((Q.nsweeps + S - 1) / S);
     } else {
         cluster_arrive();  // this CTA's halos have landed: it needs no other CTA any more
     }
@@ -749,7 +754,7 @@ int launch_visit(cudaStream_t s, const VisitCall& c) {
     }
     cfg.attrs = attr;
     const Level& lv = *c.lv;
-    const Exchange X{lv.tile_inbox, lv.tile_count};
+    const Exchange X{lv.tile_inbox, lv.tile_count, lv.tile_counts};
     return cudaLaunchKernelEx(&cfg, k, *c.Q, c.S, (const float*)lv.coef32, (const float*)lv.g32,
                               (const float*)lv.rhs32, (const float*)lv.dts32, (const float*)lv.cA32,
                               (const float*)lv.cB32, c.res, c.flag, X) == cudaSuccess

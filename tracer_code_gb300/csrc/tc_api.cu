@@ -2122,12 +2122,14 @@ tc_status create(Handle* h, const tc_params* in) {
         }
         lv.tile_inbox = nullptr;
         lv.tile_count = nullptr;
+        lv.tile_counts = 0;
         if (p.solver_precision == 1 && h->fuse_visits && l < G && !tile_visit_fits(lv.L, p.Nmulti, 0)) {
             size_t words = 0;
             const int tiles = tile_grid_tiles(lv.L, p.Nmulti, &words);
             if (tiles > 0) {
                 TRY(dalloc_t(h, &lv.tile_inbox, words));
                 TRY(dalloc_t(h, &lv.tile_count, (size_t)tiles));
+                lv.tile_counts = tiles;
             }
         }
         tcs::LevSpacing s;

@@ -191,6 +191,7 @@ struct Level {
     // their exchange counts (null: the level does not use it)
     unsigned long long* tile_inbox;
     unsigned* tile_count;
+    int tile_counts;
     int blk;        // when not fused: 0 = one k_sweep / k_sweep32 launch per sweep, n = n sweeps per k_sweep_blk launch
     MetricFold mfold;  // stretched grids: the tap weights of the computational derivatives
 };
