@@ -986,8 +986,10 @@ __global__ void k_coarse_lu_global(double* __restrict__ AB, int* __restrict__ ip
 #define LUP_NB 16
 #define LUP_CL 16              // CTAs of the panel's cluster: one per column
 #define LUP_WAIT (1 << 20)     // polls of a wait for a column's multipliers
+#define LUP_TEST_WAIT (1 << 14)  // polls of the timeout-path test's word
 template <int T>
-__global__ void __launch_bounds__(2 * T) k_lu_panel(double* ABg, int* ipiv, int n, int kl, int ku, int p, DevScalars* ds) {
+__global__ void __launch_bounds__(2 * T) k_lu_panel(double* ABg, int* ipiv, int n, int kl, int ku, int p, DevScalars* ds,
+                                                    const int* test_flag) {
     constexpr int NB = LUP_NB, NW = T / 32, R = T / 32;  // NW: warps of a column
     extern __shared__ __align__(16) double smd[];  // [2][NB][T]: multipliers of panel p-1, unscaled columns of this one
     double* msg = smd + NB * T;
@@ -1063,18 +1065,41 @@ __global__ void __launch_bounds__(2 * T) k_lu_panel(double* ABg, int* ipiv, int 
         __syncthreads();
         publish();
         bool dead = false;
+        if (test_flag != nullptr) {
+            if (o == 0)
+                for (int it = 0; *(volatile const int*)test_flag == 0 && it < LUP_TEST_WAIT; it++) {
+                }
+            dead = true;
+        }
         // the step of column i of this panel, once it is here; its JU and info.  Every thread passes the
-        // same barriers, also if a wait gave up
+        // same barriers, also if a wait gave up (it then takes no step and keeps its JU and info)
         auto arrived = [&](int i, int& ju, int& info) {
             int it = 0;
-            while (!mbar_try_wait(smem_addr(&bar[i]), 0))
+            bool here;
+            while (!(here = mbar_try_wait(smem_addr(&bar[i]), 0)))
                 if (dead || ++it > LUP_WAIT) { dead = true; break; }
-            const unsigned long long code = head[i][0];
+            const unsigned long long code = here ? head[i][0] : (unsigned long long)info << 36 | (unsigned long long)ju << 12;
             const double rcp = __longlong_as_double((long long)head[i][1]);
             const int ok = NB + i, op = (int)(code >> 1) & (T - 1);
             ju = (int)(code >> 12) & 0xffffff;
             info = (int)(code >> 36);
             step((code & 1) && jc <= ju, ok, op, [&] { return rcp * msg[i * T + (o == op ? ok : o)]; });
+        };
+        // The end of a panel's CTA: no CTA leaves while another still reads or writes its
+        // shared memory.  A thread that gave up reports it and waits, within the same bound,
+        // for the columns still on their way here, before the barrier and, when all are sent, after it.
+        auto leave = [&] {
+            auto landed = [&] {
+                for (int i = 0; dead && live && i <= last; i++)
+                    for (int it = 0; it < LUP_WAIT && !mbar_try_wait(smem_addr(&bar[i]), 0); it++) {
+                    }
+            };
+            if (dead) atomicExch(&ds->visit_timeout, 1);
+            landed();
+            __syncwarp();
+            cluster_arrive_relaxed();
+            cluster_wait();
+            landed();
         };
         if (ahead) {
             // The FP64 pipe is the panel's while this CTA holds the pivot chain: these
@@ -1082,7 +1107,7 @@ __global__ void __launch_bounds__(2 * T) k_lu_panel(double* ABg, int* ipiv, int 
             // done, or just before it comes, by the time they have until then.
             auto chain_passed = [] { asm volatile("bar.sync 3, %0;" ::"n"(2 * T) : "memory"); };
             const int pause = c < 6 ? -1 : c < 10 ? 0 : c - 1;
-            int ju, info;
+            int ju = 0, info = 0;
             if (live && pause < 0) chain_passed();
             if (p > 0) {
 #pragma unroll
@@ -1104,9 +1129,7 @@ __global__ void __launch_bounds__(2 * T) k_lu_panel(double* ABg, int* ipiv, int 
                 publish();
             }
             if (valid) *at(r, jc) = v;
-            if (o == 0 && dead) atomicExch(&ds->visit_timeout, 1);
-            cluster_arrive_relaxed();
-            cluster_wait();
+            leave();
             return;
         }
         cluster_wait();
@@ -1198,11 +1221,9 @@ __global__ void __launch_bounds__(2 * T) k_lu_panel(double* ABg, int* ipiv, int 
                     ds->lu_run = ju;
                     ds->lu_info = info;
                 }
-                if (dead) atomicExch(&ds->visit_timeout, 1);
             }
         }
-        cluster_arrive_relaxed();
-        cluster_wait();  // no CTA leaves while another still reads or writes its shared memory
+        leave();
         return;
     }
     // columns behind these two panels: steps of panel p-1
@@ -1257,7 +1278,8 @@ __global__ void __launch_bounds__(2 * T) k_lu_panel(double* ABg, int* ipiv, int 
 }
 // false where the device does not hold a cluster of LUP_CL such CTAs
 template <int T>
-bool launch_lu_panels(cudaStream_t s, double* band, int* ipiv, int n, int kl, int ku, DevScalars* ds) {
+bool launch_lu_panels(cudaStream_t s, double* band, int* ipiv, int n, int kl, int ku, DevScalars* ds,
+                      const int* test_flag) {
     const size_t smem = sizeof(double) * 2 * LUP_NB * T;
     cudaFuncSetAttribute(k_lu_panel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     cudaFuncSetAttribute(k_lu_panel<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
@@ -1289,12 +1311,13 @@ bool launch_lu_panels(cudaStream_t s, double* band, int* ipiv, int n, int kl, in
     for (int p = 0; p * LUP_NB < n; p++) {
         if (p == 0) cfg.gridDim.x = LUP_CL;
         else cfg.gridDim.x = LUP_CL * clusters;
-        cudaLaunchKernelEx(&cfg, k_lu_panel<T>, band, ipiv, n, kl, ku, p, ds); tc_note_launch();
+        cudaLaunchKernelEx(&cfg, k_lu_panel<T>, band, ipiv, n, kl, ku, p, ds, test_flag); tc_note_launch();
     }
     return true;
 }
 
-void launch_coarse_lu(cudaStream_t s, double* band, int* ipiv, int n, int kl, int ku, DevScalars* ds) {
+void launch_coarse_lu(cudaStream_t s, double* band, int* ipiv, int n, int kl, int ku, DevScalars* ds,
+                      const int* test_flag) {
     const int ldab = 2 * kl + ku + 1;
     const size_t ring = sizeof(double) * (size_t)ldab * (kl + ku + 1 + LU1_AHEAD);
     // one CTA for the narrowest bands: no messages and no launches between the columns
@@ -1306,10 +1329,10 @@ void launch_coarse_lu(cudaStream_t s, double* band, int* ipiv, int n, int kl, in
     }
     // one row per thread: the rows that two panels' steps reach
     const int rows = kl + 2 * LUP_NB;
-    if (rows <= 64 ? launch_lu_panels<64>(s, band, ipiv, n, kl, ku, ds)
-        : rows <= 128 ? launch_lu_panels<128>(s, band, ipiv, n, kl, ku, ds)
-        : rows <= 256 ? launch_lu_panels<256>(s, band, ipiv, n, kl, ku, ds)
-        : rows <= 512 && launch_lu_panels<512>(s, band, ipiv, n, kl, ku, ds)) return;
+    if (rows <= 64 ? launch_lu_panels<64>(s, band, ipiv, n, kl, ku, ds, test_flag)
+        : rows <= 128 ? launch_lu_panels<128>(s, band, ipiv, n, kl, ku, ds, test_flag)
+        : rows <= 256 ? launch_lu_panels<256>(s, band, ipiv, n, kl, ku, ds, test_flag)
+        : rows <= 512 && launch_lu_panels<512>(s, band, ipiv, n, kl, ku, ds, test_flag)) return;
     k_coarse_lu_global<<<1, 512, 0, s>>>(band, ipiv, n, kl, ku, &ds->lu_info); tc_note_launch();
 }
 

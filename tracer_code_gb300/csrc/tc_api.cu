@@ -1301,6 +1301,16 @@ void enqueue_rest(Handle* h, int) { enqueue_cycle_rest(h); }
 
 void compute_velocities(Handle* h);
 
+// A bounded wait of the solve gave up: the coarse factors and what is made
+// from them are built again by the next solve.
+const char* const kVisitGaveUp = "fused visit or coarse solve: a wait exceeded its bound";
+tc_status wait_gave_up(Handle* h, const char* what) {
+    h->lu_valid = false;
+    h->sub_valid = false;
+    h->err = what;
+    return TC_ERR_DEVICE_TIMEOUT;
+}
+
 // multigrid (iterative_solver.f90:79-173).  Newtonian rheology
 // (non_Newtonian = 0): viscosities, level operators and the coarse LU once
 // per solve.  non_Newtonian = 1: every cycle starts from the current
@@ -1319,10 +1329,7 @@ tc_status loop_result(Handle* h, long long n_pre, long long n_body) {
     const int st = h->hs->cyc_status;
     const long long bodies = (st == TC_ERR_MG_CYCLES) ? q - 2 : q - 1;
     tc_note_launch(n_pre + (bodies > 0 ? bodies : 0) * n_body);
-    if (h->hs->visit_timeout || st == TC_ERR_DEVICE_TIMEOUT) {
-        h->err = "fused smoother visit: neighbour wait exceeded its bound";
-        return TC_ERR_DEVICE_TIMEOUT;
-    }
+    if (h->hs->visit_timeout || st == TC_ERR_DEVICE_TIMEOUT) return wait_gave_up(h, kVisitGaveUp);
     if (st == TC_ERR_MG_RESIDUAL) return TC_ERR_MG_RESIDUAL;
     h->last_cycles = q;
     if (st == TC_ERR_MG_CYCLES) return TC_ERR_MG_CYCLES;
@@ -1362,10 +1369,11 @@ tc_status multigrid(Handle* h) {
     // Compute_Matrix_coarse + DGBTRF (and the explicit inverse the coarse visits apply)
     auto coarse_setup = [&]() {
         launch_coarse_build(h->st, h->lev[G], h->band, h->rowb, h->kl, h->ku, h->p.Vbc);
-        launch_coarse_lu(h->st, h->band, h->ipiv, h->ngrid_coarse, h->kl, h->ku, h->ds);
+        launch_coarse_lu(h->st, h->band, h->ipiv, h->ngrid_coarse, h->kl, h->ku, h->ds,
+                         h->wait_test ? &h->ds->never_set : nullptr);
         if (!h->coarse_banded)
             launch_coarse_inverse(h->st, h->band, h->ipiv, h->ngrid_coarse, h->kl, h->ku, h->ainv);
-        h->lu_valid = true;
+        h->lu_valid = false;  // until the factorisation's waits and pivots are read
     };
     // SF = error(1); compute_velocities; compute_strain_rate_invariant
     auto strain_from_correction = [&]() {
@@ -1420,13 +1428,16 @@ tc_status multigrid(Handle* h) {
     // cycle_correction = 2 / 4: d spans the correction with the cycles' own)
     h->acc_dnn_on = h->net != nullptr && !nonN && h->acc_dnn != nullptr &&
                     (h->p.learned_guess == 3 || h->p.cycle_correction == 2 || h->p.cycle_correction == 4);
+    // the word that every bounded wait of the solve reports to: cleared before the
+    // factorisation, whose waits are read with its pivot test
+    CK(cudaMemsetAsync(&h->ds->visit_timeout, 0, sizeof(int), h->st));
+    bool rebuild = false;
     if (!nonN) {
         TRY(level_setup());
-        const bool rebuild = (h->time == 0.0 || h->p.ivis > 0 || !h->lu_valid);
+        rebuild = (h->time == 0.0 || h->p.ivis > 0 || !h->lu_valid);
         if (rebuild) coarse_setup();
         if (h->sub_on && (rebuild || !h->sub_valid)) TRY(subcycle_setup());
     }
-    CK(cudaMemsetAsync(&h->ds->visit_timeout, 0, sizeof(int), h->st));
     const size_t img = (size_t)h->nx * h->nz;
     const bool rec = h->rec_raw && h->rec_count < h->rec_cap;
     if (rec)
@@ -1463,9 +1474,11 @@ tc_status multigrid(Handle* h) {
                          h->ds, h->p.Vbc);
     }
     // the start's read: the network's wait flag, the learned start's
-    // bookkeeping and the coarse LU's pivot test
+    // bookkeeping and the coarse LU's waits and pivot test
     const bool dnn_on = h->acc_dnn_on, lg3 = (h->p.learned_guess == 3);
-    TRY(sync_point(h, [h, dnn_on, lg3]() -> tc_status {
+    TRY(sync_point(h, [h, dnn_on, lg3, rebuild]() -> tc_status {
+        if (h->hs->visit_timeout) return wait_gave_up(h, "coarse LU: the wait for a column exceeded its bound");
+        if (rebuild) h->lu_valid = true;
         if (dnn_on) {
             if (h->hs->net_fail) {
                 h->err = "learned guess: a convolution's bounded wait gave up";
@@ -1582,10 +1595,7 @@ tc_status multigrid(Handle* h) {
         }
         TRY(sync_scalars(h));
         if (nonN && h->hs->lu_info != 0) return TC_ERR_SINGULAR;
-        if (h->hs->visit_timeout) {
-            h->err = "fused smoother visit: neighbour wait exceeded its bound";
-            return TC_ERR_DEVICE_TIMEOUT;
-        }
+        if (h->hs->visit_timeout) return wait_gave_up(h, kVisitGaveUp);
         const double rm = h->hs->res_mag[1];
         if (rm > 1.0e10 * res_ref1) return TC_ERR_MG_RESIDUAL;
         if (rm / res_ref1 <= h->p.tolerance) break;

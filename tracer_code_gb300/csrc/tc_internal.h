@@ -239,7 +239,9 @@ void launch_restrict_res(cudaStream_t s, const Level& coarse, const Level& fine,
 void launch_prolong(cudaStream_t s, const Level& coarse, const Level& fine, const double* ec, double* ef, int Vbc);
 void launch_stream_bcs(cudaStream_t s, const Level& lv, double* S, int Vbc);
 void launch_coarse_build(cudaStream_t s, const Level& lv, double* band, double* rowb, int kl, int ku, int Vbc);
-void launch_coarse_lu(cudaStream_t s, double* band, int* ipiv, int n, int kl, int ku, DevScalars* ds);
+// test_flag: the timeout-path test's word (or null), as the visits'
+void launch_coarse_lu(cudaStream_t s, double* band, int* ipiv, int n, int kl, int ku, DevScalars* ds,
+                      const int* test_flag = nullptr);
 void launch_coarse_inverse(cudaStream_t s, const double* band, const int* ipiv, int n, int kl, int ku, double* Ainv);
 void launch_coarse_solve(cudaStream_t s, const Level& lv, const double* band, const int* ipiv, const double* rowb,
                          int n, int kl, int ku, double* err, int Vbc, int* timeout_flag);
