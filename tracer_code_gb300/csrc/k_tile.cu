@@ -43,6 +43,7 @@ constexpr int kMaxSweeps = 128;
 constexpr int kMaxCluster = 16;
 constexpr int kWaitLimit = 1 << 20;      // polls of a halo wait
 constexpr int kTestWaitLimit = 1 << 14;  // polls of the timeout-path test's word
+constexpr long long kDrain = 200000;     // cycles; edges land within about 1000
 constexpr int PC = 2;                    // columns of a patch; its rows PR are a template parameter
 
 // A tile's shared buffer starts HX columns left of its owned points and 2S rows
@@ -336,7 +337,9 @@ __device__ __forceinline__ void load_tile(float* buf, int bsz, int R, const Lay&
 // tilings, so a visit also moves on the counts of tiles that it does not have).
 //
 // Waits are bounded: past the limit the CTA waits no more, finishes its loop
-// and reports the timeout.
+// and reports the timeout.  In a cluster it also arms its mbarriers no more (the
+// phase it gave up on is still open) and, after the last cluster barrier, when
+// every neighbour has sent its edges, stays for kDrain cycles while they land.
 struct Exchange {
     unsigned long long* inbox;  // per tile 2 sides of W * R words (grid)
     unsigned* count;            // per tile of the level's largest tiling: exchanges so far (grid)
@@ -519,7 +522,7 @@ __global__ void __launch_bounds__(NT, 1) k_tile_visit(const __grid_constant__ Ti
             } else {
                 const int par = (p + 1) & 1;
                 const uint32_t off = (uint32_t)(next * bsz) * 4u, boff = 8u * (uint32_t)par;
-                if (tid == 0) mbar_arrive_expect(smem_addr(&bar[par]), expect);
+                if (tid == 0 && !dead) mbar_arrive_expect(smem_addr(&bar[par]), expect);
                 for (int t = tid; t < np; t += nth) {
                     const uint3 e = push[t];
                     st_async4(e.y + off, ld4(edge + e.x), e.z + boff);
@@ -601,7 +604,12 @@ __global__ void __launch_bounds__(NT, 1) k_tile_visit(const __grid_constant__ Ti
             }
         }
     }
-    if (!GRID) cluster_wait();  // no CTA leaves while another may still write its shared memory
+    if (!GRID) {
+        cluster_wait();  // no CTA leaves while another may still write its shared memory
+        if (dead)
+            for (const long long t0 = clock64(); clock64() - t0 < kDrain;) {
+            }
+    }
 }
 
 // ---- host side ----------------------------------------------------------------------
