@@ -485,11 +485,12 @@ tc_status tc_time_visit(tc_handle* h, int32_t level, int32_t reps, double* ms_pe
  * TC_ERR_UNSUPPORTED if the handle has no such matrix. */
 tc_status tc_time_subcycle(tc_handle* h, int32_t k, int32_t reps, double* ms_per_apply);
 /* Timeout-path test (no counterpart in the reference).  With on != 0 every
- * fused cluster visit of the handle first waits, with a bounded poll, for a
- * device word that nothing sets, before it issues any sweep or write to
- * another CTA; the poll runs out, the visit takes its timeout exit and the
- * next tc_multigrid returns TC_ERR_DEVICE_TIMEOUT.  on = 0 restores normal
- * visits; the handle then solves as before. */
+ * fused visit of the handle first waits, with a bounded poll, for a device
+ * word that nothing sets, before it issues any sweep or write to another
+ * CTA; the poll runs out, the visit takes its timeout exit and the next
+ * tc_multigrid returns TC_ERR_DEVICE_TIMEOUT.  The coarse factorisation by
+ * panels and the banded coarse solve poll likewise and then wait for nothing.
+ * on = 0 restores normal solves; the handle then solves as before. */
 tc_status tc_debug_wait_test(tc_handle* h, int32_t on);
 /* Level-1 FP32 smoother of the mixed solve (no counterpart in the reference).
  * By default it forms the 13 folded coefficients from five FP32 viscosity

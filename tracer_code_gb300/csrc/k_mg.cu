@@ -1525,11 +1525,13 @@ void launch_coarse_apply(cudaStream_t s, const Level& lv, const double* Ainv, co
 #define CS_CL 8
 #define CS_MAXKL 496
 #define CS_WAIT (1 << 20)  // polls of a wait for four solved rows
+#define CS_TEST_WAIT (1 << 14)  // polls of the timeout-path test's word
 template <typename TR, int RR>
 __global__ void __launch_bounds__(CS_THREADS) k_coarse_solve(Lay L, const double* __restrict__ ABg,
                                                              const int* __restrict__ ipiv,
                                                              const double* __restrict__ rowb, const TR* rhs, int n,
-                                                             int kl, int ku, TR* err, int Vbc, int* timeout_flag) {
+                                                             int kl, int ku, TR* err, int Vbc, int* timeout_flag,
+                                                             const int* test_flag) {
     constexpr int NP = 16, D = 4;  // steps between re-basings, steps loaded ahead
     extern __shared__ double Bv[];
     __shared__ double s_d[32], s_y[32], s_y2[32];  // pivots of a block and their reciprocals
@@ -1631,6 +1633,12 @@ __global__ void __launch_bounds__(CS_THREADS) k_coarse_solve(Lay L, const double
     double v = 0.0;  // of the chain: lane l has row e - l
     double pivot = 1.0;
     bool dead = false;
+    if (test_flag != nullptr && rank == 0) {
+        if (lane == 0)
+            for (int it = 0; *(volatile const int*)test_flag == 0 && it < CS_TEST_WAIT; it++) {
+            }
+        dead = true;
+    }
     if (rank == 0 && warp == 0) {
         if (n - lane >= 1) {
             v = Bv[n - lane - 1];
@@ -1770,7 +1778,8 @@ __global__ void __launch_bounds__(256) k_coarse_solve_wide(Lay L, const double* 
 }
 template <typename TR>
 static void coarse_solve(cudaStream_t s, const Lay& L, const double* band, const int* ipiv, const double* rowb,
-                         const TR* rhs, int n, int kl, int ku, TR* err, int Vbc, int* timeout_flag) {
+                         const TR* rhs, int n, int kl, int ku, TR* err, int Vbc, int* timeout_flag,
+                         const int* test_flag) {
     const size_t sm = sizeof(double) * (size_t)n;
     auto go = [&](auto kernel, int ctas, auto... more) {
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
@@ -1791,16 +1800,16 @@ static void coarse_solve(cudaStream_t s, const Lay& L, const double* band, const
     };
     // two rows per thread above kl = 240: the 16 steps between re-basings reach kl + 16 rows
     if (kl > CS_MAXKL || sm > 226 * 1024) go(k_coarse_solve_wide<TR>, 1);
-    else if (kl <= 240) go(k_coarse_solve<TR, 1>, CS_CL, timeout_flag);
-    else go(k_coarse_solve<TR, 2>, CS_CL, timeout_flag);
+    else if (kl <= 240) go(k_coarse_solve<TR, 1>, CS_CL, timeout_flag, test_flag);
+    else go(k_coarse_solve<TR, 2>, CS_CL, timeout_flag, test_flag);
 }
 void launch_coarse_solve(cudaStream_t s, const Level& lv, const double* band, const int* ipiv, const double* rowb,
-                         int n, int kl, int ku, double* err, int Vbc, int* timeout_flag) {
-    coarse_solve(s, lv.L, band, ipiv, rowb, (const double*)lv.rhs, n, kl, ku, err, Vbc, timeout_flag);
+                         int n, int kl, int ku, double* err, int Vbc, int* timeout_flag, const int* test_flag) {
+    coarse_solve(s, lv.L, band, ipiv, rowb, (const double*)lv.rhs, n, kl, ku, err, Vbc, timeout_flag, test_flag);
 }
 void launch_coarse_solve32(cudaStream_t s, const Level& lv, const double* band, const int* ipiv, const double* rowb,
-                           int n, int kl, int ku, float* err, int Vbc, int* timeout_flag) {
-    coarse_solve(s, lv.L, band, ipiv, rowb, (const float*)lv.rhs32, n, kl, ku, err, Vbc, timeout_flag);
+                           int n, int kl, int ku, float* err, int Vbc, int* timeout_flag, const int* test_flag) {
+    coarse_solve(s, lv.L, band, ipiv, rowb, (const float*)lv.rhs32, n, kl, ku, err, Vbc, timeout_flag, test_flag);
 }
 
 __global__ void k_copy(double* dst, const double* src, size_t n) {

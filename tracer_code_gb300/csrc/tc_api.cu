@@ -1030,7 +1030,8 @@ void enqueue_cycle_rest(Handle* h) {
         } else {
             if (h->coarse_banded)
                 launch_coarse_solve(h->st, h->lev[G], h->band, h->ipiv, h->rowb, h->ngrid_coarse, h->kl, h->ku,
-                                    cur_err(h, G), h->p.Vbc, &h->ds->visit_timeout);
+                                    cur_err(h, G), h->p.Vbc, &h->ds->visit_timeout,
+                                    h->wait_test ? &h->ds->never_set : nullptr);
             else
                 launch_coarse_apply(h->st, h->lev[G], h->ainv, h->rowb, h->ngrid_coarse, h->coarse_q, h->coarse_x,
                                     h->coarse_m, cur_err(h, G), h->p.Vbc);
@@ -1165,7 +1166,8 @@ void enqueue_rest_mixed(Handle* h, int) {
         } else if (level < G) iterate_stream32(h, level, dir, pending_pro ? 1 : 0, f.rst, f.rst_zero);
         else if (h->coarse_banded)
             launch_coarse_solve32(h->st, h->lev[G], h->band, h->ipiv, h->rowb, h->ngrid_coarse, h->kl, h->ku,
-                                  cur_e32(h, G), h->p.Vbc, &h->ds->visit_timeout);
+                                  cur_e32(h, G), h->p.Vbc, &h->ds->visit_timeout,
+                                  h->wait_test ? &h->ds->never_set : nullptr);
         else launch_coarse_apply32(h->st, h->lev[G], h->ainv, h->rowb, h->ngrid_coarse, h->coarse_q, h->coarse_x,
                                    h->coarse_m, cur_e32(h, G), h->p.Vbc);
         restricted = f.rst != 0;

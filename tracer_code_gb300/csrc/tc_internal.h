@@ -244,9 +244,9 @@ void launch_coarse_lu(cudaStream_t s, double* band, int* ipiv, int n, int kl, in
                       const int* test_flag = nullptr);
 void launch_coarse_inverse(cudaStream_t s, const double* band, const int* ipiv, int n, int kl, int ku, double* Ainv);
 void launch_coarse_solve(cudaStream_t s, const Level& lv, const double* band, const int* ipiv, const double* rowb,
-                         int n, int kl, int ku, double* err, int Vbc, int* timeout_flag);
+                         int n, int kl, int ku, double* err, int Vbc, int* timeout_flag, const int* test_flag = nullptr);
 void launch_coarse_solve32(cudaStream_t s, const Level& lv, const double* band, const int* ipiv, const double* rowb,
-                           int n, int kl, int ku, float* err, int Vbc, int* timeout_flag);
+                           int n, int kl, int ku, float* err, int Vbc, int* timeout_flag, const int* test_flag = nullptr);
 void launch_coarse_apply(cudaStream_t s, const Level& lv, const double* Ainv, const double* rowb, int n,
                          const int* cq, const int* cx, int m, double* err, int Vbc);
 void launch_copy_plane(cudaStream_t s, double* dst, const double* src, size_t n);
