@@ -501,13 +501,7 @@ void launch_accel_window(cudaStream_t s, const Level& l1, double* psi, double* p
                          double* rn, double* rp, const double* dnn, const double* adnn, int use_dnn, RedScratch rs,
                          DevScalars* ds, int Vbc) {
     Range2 r{1, l1.L.a - 1, 1, l1.L.b - 1};
-    static int nsm = 0;
-    if (nsm == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-        if (nsm <= 0) nsm = 1;
-    }
+    const int nsm = tc_sm_count();
     const int npts = (l1.L.a - 1) * (l1.L.b - 1);
     // grid-stride over the points with one wave of CTAs (three per SM: the
     // kernel's launch bounds), so that the block sums and their fold stay few
@@ -530,13 +524,7 @@ void launch_accel_window(cudaStream_t s, const Level& l1, double* psi, double* p
 void launch_accel(cudaStream_t s, const Level& l1, double* psi, double* prev, const double* dnn, int k1, int k2,
                   int record_prev, RedScratch rs, DevScalars* ds, int Vbc) {
     Range2 r{1, l1.L.a - 1, 1, l1.L.b - 1};
-    static int nsm = 0;
-    if (nsm == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-        if (nsm <= 0) nsm = 1;
-    }
+    const int nsm = tc_sm_count();
     const int npts = (l1.L.a - 1) * (l1.L.b - 1);
     int nb = (npts + 255) / 256;
     if (nb > 2 * nsm) nb = 2 * nsm;

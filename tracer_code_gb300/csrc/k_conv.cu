@@ -212,27 +212,20 @@ static PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
 
 template <int N>
 static bool conv_attr() {
-    static bool done = false;
-    if (!done) {
+    static PerDevice set;
+    return set.get([] {
         const int smax = kStages * (64 * 256 + N * 64 * 2) + 1024;
-        if (cudaFuncSetAttribute(k_conv3x3p<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, smax) != cudaSuccess)
-            return false;
-        done = true;
-    }
-    return true;
+        return cudaFuncSetAttribute(k_conv3x3p<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, smax) == cudaSuccess
+                   ? 0
+                   : -1;
+    }) == 0;
 }
 
 // CTAs of the persistent convolution: two per SM while two double-buffered
 // accumulators fit the SM's 512 TMEM columns (one for N = 256)
 template <int N>
 static unsigned conv_grid(int ntiles) {
-    static int nsm = 0;
-    if (nsm == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-        if (nsm <= 0) nsm = 1;
-    }
+    const int nsm = tc_sm_count();
     const int per_sm = (4 * N <= 512) ? 2 : 1;
     const int g = nsm * per_sm;
     return (unsigned)(ntiles < g ? ntiles : g);
@@ -241,17 +234,6 @@ static unsigned conv_grid(int ntiles) {
 }  // namespace nn
 
 using namespace nn;
-
-int nn_sm_count() {
-    static int nsm = 0;
-    if (nsm == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-        if (nsm <= 0) nsm = 1;
-    }
-    return nsm;
-}
 
 // map of an NHWC BF16 tensor [nb][H][W][ctot] with boxes {c, bx, by, 1}; swizzle:
 // 0 or the bytes of a box row (32, 64 or 128)

@@ -1301,12 +1301,13 @@ bool launch_lu_panels(cudaStream_t s, double* band, int* ipiv, int n, int kl, in
     at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    static const int fits = [&] {
-        int c = 0;
-        if (cudaOccupancyMaxActiveClusters(&c, k_lu_panel<T>, &cfg) != cudaSuccess) { cudaGetLastError(); return 0; }
-        return c;
-    }();
-    if (fits < 1) return false;
+    static PerDevice fits;
+    if (fits.get([&] {
+            int c = 0;
+            if (cudaOccupancyMaxActiveClusters(&c, k_lu_panel<T>, &cfg) != cudaSuccess) { cudaGetLastError(); return 0; }
+            return c;
+        }) < 1)
+        return false;
     cfg.numAttrs = 2;
     for (int p = 0; p * LUP_NB < n; p++) {
         if (p == 0) cfg.gridDim.x = LUP_CL;

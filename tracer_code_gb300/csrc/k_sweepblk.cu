@@ -453,13 +453,14 @@ static bool gblk_launch(cudaStream_t s, const Level& lv, const float* Sin, float
     constexpr int SX = TX + 4 * NS;
     constexpr int SY = (NSTR * P + 4 > TY + 4 * NS) ? NSTR * P + 4 : TY + 4 * NS;
     constexpr size_t smem = sizeof(float) * ((size_t)2 * SY * SX + (size_t)TC_NCOEF * P * NT);
-    static bool attr = false;
-    if (!attr) {
-        if (cudaFuncSetAttribute(k_sweep_gblk<NS, P, TX, TY, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem) != cudaSuccess)
-            return false;
-        attr = true;
-    }
+    static PerDevice set;
+    if (set.get([&] {
+            return cudaFuncSetAttribute(k_sweep_gblk<NS, P, TX, TY, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)smem) == cudaSuccess
+                       ? 0
+                       : -1;
+        }) != 0)
+        return false;
     BlkParams<float, NS> Q;
     Q.L = lv.L;
     Q.per_point = per_point;

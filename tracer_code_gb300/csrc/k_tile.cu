@@ -649,17 +649,6 @@ int push_count(const TileGeom& G) {
     return ny * 2 * G.S * (G.TX / 4) + nx * (G.HX / 4) * G.TY + nx * ny * (G.HX / 4) * 2 * G.S;
 }
 
-int sm_count() {
-    static int nsm = 0;
-    if (nsm == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-        if (nsm <= 0) nsm = 1;
-    }
-    return nsm;
-}
-
 int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
 // Cycles of one sweep, a fit to measured visits (70 sweeps at 64x16..512x128):
@@ -734,13 +723,15 @@ struct VisitCall {
 template <int W, int PR, int NT, bool PP, bool GRID>
 int launch_visit(cudaStream_t s, const VisitCall& c) {
     auto k = k_tile_visit<W, PR, NT, PP, GRID>;
-    static bool ready = false;
-    if (!ready) {
-        if ((!GRID && cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) ||
-            cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess)
-            return 2;
-        ready = true;
-    }
+    static PerDevice set;
+    if (set.get([k] {
+            return (GRID || cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) &&
+                           cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) ==
+                               cudaSuccess
+                       ? 0
+                       : -1;
+        }) != 0)
+        return 2;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(c.p->G.NX * c.p->G.NY), 1, 1);
     cfg.blockDim = dim3((unsigned)c.p->threads, 1, 1);
@@ -801,7 +792,7 @@ int tile_grid_tiles(const Lay& L, int nsweeps, size_t* words) {
     *words = 0;
     for (int pp = 0; pp < 2; pp++) {
         VisitPlan p;
-        if (nsweeps > kMaxSweeps || nsweeps <= 5 || !visit_plan(L, sm_count(), true, pp != 0, &p)) continue;
+        if (nsweeps > kMaxSweeps || nsweeps <= 5 || !visit_plan(L, tc_sm_count(), true, pp != 0, &p)) continue;
         const size_t w = (size_t)p.G.NX * p.G.NY * 2 * p.G.W * p.G.R;
         if (w > *words) *words = w;
         if (p.G.NX * p.G.NY > most) most = p.G.NX * p.G.NY;
@@ -816,7 +807,7 @@ int launch_tile_visit(cudaStream_t s, const Level& lv, bool grid, float* S, cons
                       const int* test_flag) {
     VisitPlan p;
     if (nsweeps > kMaxSweeps || (grid && (nsweeps <= 5 || lv.tile_inbox == nullptr)) ||
-        !visit_plan(lv.L, grid ? sm_count() : kMaxCluster, grid, per_point != 0, &p))
+        !visit_plan(lv.L, grid ? tc_sm_count() : kMaxCluster, grid, per_point != 0, &p))
         return 1;
     TileParams Q;
     fill_params(&Q, lv, p.G, nsweeps, c, temp, per_point, Vbc);
@@ -831,5 +822,6 @@ int launch_tile_visit(cudaStream_t s, const Level& lv, bool grid, float* S, cons
     const VisitCall call{&p, &Q, &lv, S, res, timeout_flag};
     const int r = grid ? launch_visit_any<true>(s, call) : launch_visit_any<false>(s, call);
     if (r == 0) tc_note_launch();
+    else cudaGetLastError();  // the caller's other kernels run instead: leave no error behind
     return r;
 }

@@ -213,12 +213,14 @@ __global__ void __launch_bounds__(320, 1) k_wgrad(const __grid_constant__ CUtens
 template <int CC>
 static int launch_cc(cudaStream_t s, const CUtensorMap& zmap, const CUtensorMap& xmap, const WgradArgs& a, dim3 grid,
                      int smem) {
-    static bool ready = false;
-    if (!ready) {
-        if (cudaFuncSetAttribute(k_wgrad<CC>, cudaFuncAttributeMaxDynamicSharedMemorySize, 202 * 1024) != cudaSuccess)
-            return 4;
-        ready = true;
-    }
+    static PerDevice set;
+    if (set.get([] {
+            return cudaFuncSetAttribute(k_wgrad<CC>, cudaFuncAttributeMaxDynamicSharedMemorySize, 202 * 1024) ==
+                           cudaSuccess
+                       ? 0
+                       : -1;
+        }) != 0)
+        return 4;
     k_wgrad<CC><<<grid, 320, smem, s>>>(zmap, xmap, a);
     tc_note_launch();
     return cudaGetLastError() == cudaSuccess ? 0 : 5;
@@ -246,7 +248,7 @@ using namespace nn;
 int wgrad_splits(int nb, int H, int W, int cin) {
     const int cin_p = (cin + 15) / 16 * 16, chunks = cin_p / chunk_of(cin_p);
     int per, s;
-    split_of(nb * H * W / kWgTile, 3 * chunks, nn_sm_count(), &per, &s);
+    split_of(nb * H * W / kWgTile, 3 * chunks, tc_sm_count(), &per, &s);
     return s;
 }
 
@@ -268,7 +270,7 @@ int wgrad_launch(cudaStream_t s, const __nv_bfloat16* x, int x_tot, int x_off, i
     a.zn = cout / a.za;
     a.tiles = nb * H * W / kWgTile;
     int splits;
-    split_of(a.tiles, 3 * (cin_p / a.cc), nn_sm_count(), &a.per_split, &splits);
+    split_of(a.tiles, 3 * (cin_p / a.cc), tc_sm_count(), &a.per_split, &splits);
     const int st_bytes = kWgTile * 2 * (cout + 3 * a.cc);
     a.stages = (200 * 1024) / st_bytes;
     if (a.stages > 8) a.stages = 8;

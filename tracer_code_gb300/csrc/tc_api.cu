@@ -36,6 +36,21 @@ void tc_note_launch(long long n) {
     t_launches += n;
 }
 
+int tc_current_device() {
+    int dev = -1;
+    cudaGetDevice(&dev);
+    return dev;
+}
+int tc_sm_count() {
+    static PerDevice n;
+    return n.get([] {
+        int v = 0;
+        if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, tc_current_device()) != cudaSuccess || v <= 0)
+            v = 1;
+        return v;
+    });
+}
+
 // learned initial guess (k_nn.cu, tc_nn_api.cu)
 struct tc_net_impl;
 tc_net_impl* tcnn_impl(tc_net* n);

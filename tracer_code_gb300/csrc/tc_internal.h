@@ -16,6 +16,7 @@
 #include <stddef.h>
 
 #include "tracer_gpu.h"
+#include "tc_perdev.h"
 
 #define SP 2
 #define TC_MAXLEV 6

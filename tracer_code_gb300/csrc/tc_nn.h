@@ -16,8 +16,7 @@ int conv3x3_launch(cudaStream_t s, const __nv_bfloat16* x, int nb, int H, int W,
                    const __nv_bfloat16* wpack, const float* bias, int N, int relu, __nv_bfloat16* out, int cout_tot,
                    int cout_off, int cout_store, int* fail, const int* test_flag = nullptr);
 
-// SMs of the current device; map of an NHWC BF16 tensor (k_conv.cu)
-int nn_sm_count();
+// map of an NHWC BF16 tensor (k_conv.cu)
 bool nn_tensor_map(CUtensorMap* map, const __nv_bfloat16* x, int nb, int H, int W, int ctot, int c, int bx, int by,
                    int swizzle);
 
