@@ -492,6 +492,12 @@ tc_status tc_time_subcycle(tc_handle* h, int32_t k, int32_t reps, double* ms_per
  * panels and the banded coarse solve poll likewise and then wait for nothing.
  * on = 0 restores normal solves; the handle then solves as before. */
 tc_status tc_debug_wait_test(tc_handle* h, int32_t on);
+/* Refused launches, for tests (no counterpart in the reference).  With on != 0
+ * the handle's one-launch viscosity filter, coarse factorisation by panels,
+ * banded coarse solve and tile visits behave as on a device that refuses their
+ * clusters or cooperative grids: the kernels without them run, with the same
+ * results. */
+tc_status tc_debug_refuse_clusters(tc_handle* h, int32_t on);
 /* Level-1 FP32 smoother of the mixed solve (no counterpart in the reference).
  * By default it forms the 13 folded coefficients from five FP32 viscosity
  * fields inside each sweep; with fields = 0 it reads the 13 coefficient

@@ -422,7 +422,8 @@ bool vis_filter_fits(const Level& lv, int interpolate) {
     const int points = (lv.L.a + 1) * (lv.L.b + 1);
     return points <= (interpolate ? VF_MAX_SMOOTH : lv.c.M.on ? VF_MAX_RATIO_METRIC : VF_MAX_RATIO);
 }
-void launch_vis_filter(cudaStream_t s, const Level& lv, const VisFltArgs& q, int reset, const double* src, double* A,
+// false where the device does not take the cluster: nothing ran, the loop graphs can
+bool launch_vis_filter(cudaStream_t s, const Level& lv, const VisFltArgs& q, int reset, const double* src, double* A,
                        double* B, int derivatives, int kmin, int kmax, int RaT_nonzero, double visT2,
                        DevScalars* ds) {
     const int npts = (lv.L.a + 1) * (kmax - kmin + 1);
@@ -439,8 +440,15 @@ void launch_vis_filter(cudaStream_t s, const Level& lv, const VisFltArgs& q, int
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kernel, lv.L, lv.c, q, reset, src, A, B, (const double*)lv.dt_vis, kmin, kmax,
-                       RaT_nonzero, visT2, derivatives ? lv.vx : nullptr, lv.vz, lv.vxx, lv.vzz, lv.vxz, lv.ratio, ds); tc_note_launch();
+    if (lv.no_cluster ||
+        cudaLaunchKernelEx(&cfg, kernel, lv.L, lv.c, q, reset, src, A, B, (const double*)lv.dt_vis, kmin, kmax,
+                           RaT_nonzero, visT2, derivatives ? lv.vx : nullptr, lv.vz, lv.vxx, lv.vzz, lv.vxz, lv.ratio,
+                           ds) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    tc_note_launch();
+    return true;
 }
 
 // ---------------------------------------------------------------------------
@@ -1276,7 +1284,8 @@ __global__ void __launch_bounds__(2 * T) k_lu_panel(double* ABg, int* ipiv, int 
         }
     }
 }
-// false where the device does not hold a cluster of LUP_CL such CTAs
+// false where the device does not take a cluster of LUP_CL such CTAs (nothing ran); a launch
+// refused later leaves its error for the solve's next read
 template <int T>
 bool launch_lu_panels(cudaStream_t s, double* band, int* ipiv, int n, int kl, int ku, DevScalars* ds,
                       const int* test_flag) {
@@ -1312,12 +1321,16 @@ bool launch_lu_panels(cudaStream_t s, double* band, int* ipiv, int n, int kl, in
     for (int p = 0; p * LUP_NB < n; p++) {
         if (p == 0) cfg.gridDim.x = LUP_CL;
         else cfg.gridDim.x = LUP_CL * clusters;
-        cudaLaunchKernelEx(&cfg, k_lu_panel<T>, band, ipiv, n, kl, ku, p, ds, test_flag); tc_note_launch();
+        if (cudaLaunchKernelEx(&cfg, k_lu_panel<T>, band, ipiv, n, kl, ku, p, ds, test_flag) != cudaSuccess) {
+            if (p == 0) cudaGetLastError();
+            return p != 0;
+        }
+        tc_note_launch();
     }
     return true;
 }
 
-void launch_coarse_lu(cudaStream_t s, double* band, int* ipiv, int n, int kl, int ku, DevScalars* ds,
+void launch_coarse_lu(cudaStream_t s, const Level& lv, double* band, int* ipiv, int n, int kl, int ku, DevScalars* ds,
                       const int* test_flag) {
     const int ldab = 2 * kl + ku + 1;
     const size_t ring = sizeof(double) * (size_t)ldab * (kl + ku + 1 + LU1_AHEAD);
@@ -1330,7 +1343,8 @@ void launch_coarse_lu(cudaStream_t s, double* band, int* ipiv, int n, int kl, in
     }
     // one row per thread: the rows that two panels' steps reach
     const int rows = kl + 2 * LUP_NB;
-    if (rows <= 64 ? launch_lu_panels<64>(s, band, ipiv, n, kl, ku, ds, test_flag)
+    if (lv.no_cluster) {
+    } else if (rows <= 64 ? launch_lu_panels<64>(s, band, ipiv, n, kl, ku, ds, test_flag)
         : rows <= 128 ? launch_lu_panels<128>(s, band, ipiv, n, kl, ku, ds, test_flag)
         : rows <= 256 ? launch_lu_panels<256>(s, band, ipiv, n, kl, ku, ds, test_flag)
         : rows <= 512 && launch_lu_panels<512>(s, band, ipiv, n, kl, ku, ds, test_flag)) return;
@@ -1725,7 +1739,8 @@ __global__ void __launch_bounds__(CS_THREADS) k_coarse_solve(Lay L, const double
     pdl_done();
 }
 // The same with one warp and no rows in registers: bands and vectors beyond the kernel
-// above (kl > 496, or a vector that leaves no room for the pivots).
+// above (kl > 496, or a vector that leaves no room for the pivots), and devices that do
+// not take its cluster.
 template <typename TR>
 __global__ void __launch_bounds__(256) k_coarse_solve_wide(Lay L, const double* __restrict__ ABg,
                                                            const int* __restrict__ ipiv,
@@ -1778,7 +1793,7 @@ __global__ void __launch_bounds__(256) k_coarse_solve_wide(Lay L, const double* 
     pdl_done();
 }
 template <typename TR>
-static void coarse_solve(cudaStream_t s, const Lay& L, const double* band, const int* ipiv, const double* rowb,
+static void coarse_solve(cudaStream_t s, const Level& lv, const double* band, const int* ipiv, const double* rowb,
                          const TR* rhs, int n, int kl, int ku, TR* err, int Vbc, int* timeout_flag,
                          const int* test_flag) {
     const size_t sm = sizeof(double) * (size_t)n;
@@ -1797,20 +1812,27 @@ static void coarse_solve(cudaStream_t s, const Lay& L, const double* band, const
         at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
         cfg.attrs = at;
         cfg.numAttrs = ctas > 1 ? 2 : 1;
-        cudaLaunchKernelEx(&cfg, kernel, L, band, ipiv, rowb, rhs, n, kl, ku, err, Vbc, more...); tc_note_launch();
+        if ((ctas > 1 && lv.no_cluster) ||
+            cudaLaunchKernelEx(&cfg, kernel, lv.L, band, ipiv, rowb, rhs, n, kl, ku, err, Vbc, more...) != cudaSuccess)
+            return false;
+        tc_note_launch();
+        return true;
     };
     // two rows per thread above kl = 240: the 16 steps between re-basings reach kl + 16 rows
-    if (kl > CS_MAXKL || sm > 226 * 1024) go(k_coarse_solve_wide<TR>, 1);
-    else if (kl <= 240) go(k_coarse_solve<TR, 1>, CS_CL, timeout_flag, test_flag);
-    else go(k_coarse_solve<TR, 2>, CS_CL, timeout_flag, test_flag);
+    if (kl <= CS_MAXKL && sm <= 226 * 1024) {
+        if (kl <= 240 ? go(k_coarse_solve<TR, 1>, CS_CL, timeout_flag, test_flag)
+                      : go(k_coarse_solve<TR, 2>, CS_CL, timeout_flag, test_flag)) return;
+        cudaGetLastError();
+    }
+    go(k_coarse_solve_wide<TR>, 1);  // (an error here is left for the solve's next read)
 }
 void launch_coarse_solve(cudaStream_t s, const Level& lv, const double* band, const int* ipiv, const double* rowb,
                          int n, int kl, int ku, double* err, int Vbc, int* timeout_flag, const int* test_flag) {
-    coarse_solve(s, lv.L, band, ipiv, rowb, (const double*)lv.rhs, n, kl, ku, err, Vbc, timeout_flag, test_flag);
+    coarse_solve(s, lv, band, ipiv, rowb, (const double*)lv.rhs, n, kl, ku, err, Vbc, timeout_flag, test_flag);
 }
 void launch_coarse_solve32(cudaStream_t s, const Level& lv, const double* band, const int* ipiv, const double* rowb,
                            int n, int kl, int ku, float* err, int Vbc, int* timeout_flag, const int* test_flag) {
-    coarse_solve(s, lv.L, band, ipiv, rowb, (const float*)lv.rhs32, n, kl, ku, err, Vbc, timeout_flag, test_flag);
+    coarse_solve(s, lv, band, ipiv, rowb, (const float*)lv.rhs32, n, kl, ku, err, Vbc, timeout_flag, test_flag);
 }
 
 __global__ void k_copy(double* dst, const double* src, size_t n) {

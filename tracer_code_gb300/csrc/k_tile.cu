@@ -806,7 +806,7 @@ int launch_tile_visit(cudaStream_t s, const Level& lv, bool grid, float* S, cons
                       int nsweeps, int per_point, int Vbc, float* res, int* timeout_flag, const VisitXfer<float>* x,
                       const int* test_flag) {
     VisitPlan p;
-    if (nsweeps > kMaxSweeps || (grid && (nsweeps <= 5 || lv.tile_inbox == nullptr)) ||
+    if (lv.no_cluster || nsweeps > kMaxSweeps || (grid && (nsweeps <= 5 || lv.tile_inbox == nullptr)) ||
         !visit_plan(lv.L, grid ? tc_sm_count() : kMaxCluster, grid, per_point != 0, &p))
         return 1;
     TileParams Q;

@@ -718,8 +718,9 @@ bool vis_filter_runs(const Handle* h, int level, int interpolate) {
 }
 
 // smoother_vis (smoother.f90:166-263); work: smooth a copy of the viscosity there and leave
-// the level's own viscosity and derivatives (where vis_filter_runs)
-tc_status smoother_vis(Handle* h, int level, int interpolate, double* work = nullptr) {
+// the level's own viscosity and derivatives; *worked: whether that was done, else nothing was
+// (only k_vis_filter does it)
+tc_status smoother_vis(Handle* h, int level, int interpolate, double* work = nullptr, bool* worked = nullptr) {
     Level& lv = h->lev[level];
     int option, Niter;
     double lb, la;
@@ -752,11 +753,14 @@ tc_status smoother_vis(Handle* h, int level, int interpolate, double* work = nul
         const size_t by = sizeof(double) * lv.L.plane;
         if (vis_filter_runs(h, level, interpolate)) {
             if (!h->capturing) TRY(filter_state_to_device(h));
-            launch_vis_filter(h->st, lv, fa, reset, cur, work ? work : cur, oth, work ? 0 : 1, kmin, kmax, RaTnz,
-                              visT2, h->ds);
-            h->ratio_level = level;
-            return TC_OK;
+            if (launch_vis_filter(h->st, lv, fa, reset, cur, work ? work : cur, oth, work ? 0 : 1, kmin, kmax, RaTnz,
+                                  visT2, h->ds)) {
+                h->ratio_level = level;
+                if (worked) *worked = true;
+                return TC_OK;
+            }
         }
+        if (work) return TC_OK;
         // the test reads no eigenvalue ratio where it interpolates: one gradient after the loop
         const int nk = interpolate ? 2 : 3;
         auto pre = [&](cudaGraphConditionalHandle c) {
@@ -853,10 +857,12 @@ tc_status compute_viscosity(Handle* h, int level) {
     Level& f = h->lev[l1];
     Level& c = h->lev[level];
     const size_t by = sizeof(double) * f.L.plane;
-    const bool copy = !vis_filter_runs(h, l1, 1);  // else the filter works on a copy itself
+    bool worked = false;  // the filter worked on a copy itself
+    TRY(smoother_vis(h, l1, 1, f.bak[0], &worked));
+    const bool copy = !worked;
     double* src[6] = {cur_vis(h, l1), f.vx, f.vz, f.vxx, f.vzz, f.vxz};
     for (int q = 0; copy && q < 6; q++) CK(cudaMemcpyAsync(f.bak[q], src[q], by, cudaMemcpyDeviceToDevice, h->st));
-    TRY(smoother_vis(h, l1, 1, copy ? nullptr : f.bak[0]));
+    if (copy) TRY(smoother_vis(h, l1, 1));
     launch_restrict_vis(h->st, c, f, copy ? cur_vis(h, l1) : f.bak[0], cur_vis(h, level));
     launch_vis_bcs_init(h->st, c, cur_vis(h, level), h->p.RaT != 0.0 ? 1 : 0, h->p.visT * h->p.visT);
     if (level < h->grids) TRY(smoother_vis(h, level, 0));
@@ -1386,7 +1392,7 @@ tc_status multigrid(Handle* h) {
     // Compute_Matrix_coarse + DGBTRF (and the explicit inverse the coarse visits apply)
     auto coarse_setup = [&]() {
         launch_coarse_build(h->st, h->lev[G], h->band, h->rowb, h->kl, h->ku, h->p.Vbc);
-        launch_coarse_lu(h->st, h->band, h->ipiv, h->ngrid_coarse, h->kl, h->ku, h->ds,
+        launch_coarse_lu(h->st, h->lev[G], h->band, h->ipiv, h->ngrid_coarse, h->kl, h->ku, h->ds,
                          h->wait_test ? &h->ds->never_set : nullptr);
         if (!h->coarse_banded)
             launch_coarse_inverse(h->st, h->band, h->ipiv, h->ngrid_coarse, h->kl, h->ku, h->ainv);
@@ -2150,6 +2156,7 @@ tc_status create(Handle* h, const tc_params* in) {
         lv.tile_inbox = nullptr;
         lv.tile_count = nullptr;
         lv.tile_counts = 0;
+        lv.no_cluster = 0;
         if (p.solver_precision == 1 && h->fuse_visits && l < G && !tile_visit_fits(lv.L, p.Nmulti, 0)) {
             size_t words = 0;
             const int tiles = tile_grid_tiles(lv.L, p.Nmulti, &words);
@@ -3310,6 +3317,20 @@ tc_status tc_debug_wait_test(tc_handle* H, int32_t on) {
     Handle* h = &H->h;
     h->wait_test = (on != 0);
     // the cycle graphs bake in the visits' parameters: capture again
+    CycleGraphs& cg = *h->graphs;
+    if (cg.l1) cudaGraphExecDestroy(cg.l1);
+    if (cg.rest) cudaGraphExecDestroy(cg.rest);
+    if (cg.loop) cudaGraphExecDestroy(cg.loop);
+    cg.l1 = cg.rest = cg.loop = nullptr;
+    drop_step_graphs(h);
+    return TC_OK;
+}
+
+tc_status tc_debug_refuse_clusters(tc_handle* H, int32_t on) {
+    if (!H) return TC_ERR_ARG;
+    Handle* h = &H->h;
+    for (int l = 1; l <= h->grids; l++) h->lev[l].no_cluster = (on != 0);
+    // the cycle graphs bake in the kernels: capture again
     CycleGraphs& cg = *h->graphs;
     if (cg.l1) cudaGraphExecDestroy(cg.l1);
     if (cg.rest) cudaGraphExecDestroy(cg.rest);

@@ -193,6 +193,7 @@ struct Level {
     unsigned long long* tile_inbox;
     unsigned* tile_count;
     int tile_counts;
+    int no_cluster;  // 1: clusters and cooperative grids count as refused (tc_debug_refuse_clusters)
     int blk;        // when not fused: 0 = one k_sweep / k_sweep32 launch per sweep, n = n sweeps per k_sweep_blk launch
     MetricFold mfold;  // stretched grids: the tap weights of the computational derivatives
 };
@@ -225,7 +226,7 @@ void launch_vis_smooth(cudaStream_t s, const Level& lv, const double* vin, doubl
                        int kmax, int RaT_nonzero, double visT2, const double* cdev = nullptr);
 void launch_restrict_vis(cudaStream_t s, const Level& coarse, const Level& fine, const double* vfine, double* vcoarse);
 bool vis_filter_fits(const Level& lv, int interpolate);
-void launch_vis_filter(cudaStream_t s, const Level& lv, const VisFltArgs& q, int reset, const double* src, double* A,
+bool launch_vis_filter(cudaStream_t s, const Level& lv, const VisFltArgs& q, int reset, const double* src, double* A,
                        double* B, int derivatives, int kmin, int kmax, int RaT_nonzero, double visT2,
                        DevScalars* ds);
 void launch_vis_bcs_init(cudaStream_t s, const Level& coarse, double* v, int RaT_nonzero, double visT2);
@@ -241,7 +242,7 @@ void launch_prolong(cudaStream_t s, const Level& coarse, const Level& fine, cons
 void launch_stream_bcs(cudaStream_t s, const Level& lv, double* S, int Vbc);
 void launch_coarse_build(cudaStream_t s, const Level& lv, double* band, double* rowb, int kl, int ku, int Vbc);
 // test_flag: the timeout-path test's word (or null), as the visits'
-void launch_coarse_lu(cudaStream_t s, double* band, int* ipiv, int n, int kl, int ku, DevScalars* ds,
+void launch_coarse_lu(cudaStream_t s, const Level& lv, double* band, int* ipiv, int n, int kl, int ku, DevScalars* ds,
                       const int* test_flag = nullptr);
 void launch_coarse_inverse(cudaStream_t s, const double* band, const int* ipiv, int n, int kl, int ku, double* Ainv);
 void launch_coarse_solve(cudaStream_t s, const Level& lv, const double* band, const int* ipiv, const double* rowb,
