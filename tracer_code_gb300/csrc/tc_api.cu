@@ -145,7 +145,7 @@ struct Handle {
     int last_cycles = 0;
     long loop_cap = 100000;
     std::string err;
-    CycleGraphs* graphs = nullptr;
+    CycleGraphs* graphs = nullptr;  // two: stepped alone, in an ensemble
     bool no_graphs = false;
     bool no_device_loop = false;  // convergence and filter loops on the host (one read per pass)
     // filter loops as cached WHILE graphs (k_loop.cu), keyed by loop kind,
@@ -205,14 +205,14 @@ struct Handle {
     // queues its host work in `deferred`, which runs after every launch of
     // the graph in the order the eager step would have run it; the WHILE
     // bodies of the step's loops are captured on body_st
-    bool in_ensemble = false;  // stepped by tc_ensemble_run / tc_ensemble_step: no launches that need the whole GPU
+    bool in_ensemble = false;  // in a call that steps several handles: no launches that need the whole GPU
     bool capturing = false;
     cudaStream_t body_st = nullptr;
     DevScalars* hsnap = nullptr;  // pinned, kMaxSnap entries
     int nsnap = 0;
     std::vector<std::function<tc_status()>> deferred;
     bool step_graph = false, step_graph_failed = false;
-    std::map<int, struct StepGraph*> step_graphs;  // by whether the step sorts the tracers
+    std::map<int, struct StepGraph*> step_graphs;  // by whether the step sorts the tracers (and 2: in an ensemble)
     tc_stats_row stats_row{};                      // the row the last stats read formed
     long long sub_tab_key = -1;                    // the sweep tables now in sub_tab
     long long graph_steps = 0;                     // steps run as one graph launch
@@ -1543,7 +1543,7 @@ tc_status multigrid(Handle* h) {
     // p=1 is the only level-1 visit of every cycle table; the convergence test
     // follows it, then p=2..nsteps run unconditionally.
     const int dir1 = (h->multi[2] > h->multi[1]) ? 0 : 1;
-    CycleGraphs& cg = *h->graphs;
+    CycleGraphs& cg = h->graphs[h->in_ensemble ? 1 : 0];
     const bool use_graphs = (h->st != nullptr) && !h->no_graphs && !nonN;
     void (*f_l1)(Handle*, int) = mixed ? enqueue_l1_mixed : enqueue_l1;
     void (*f_rest)(Handle*, int) = mixed ? enqueue_rest_mixed : enqueue_rest;
@@ -1973,7 +1973,7 @@ tc_status create(Handle* h, const tc_params* in) {
     cudaError_t e = cudaStreamCreateWithFlags(&h->st, cudaStreamNonBlocking);
     if (e != cudaSuccess) { h->err = cudaGetErrorString(e); return TC_ERR_CUDA; }
     h->own_stream = true;
-    h->graphs = new CycleGraphs();
+    h->graphs = new CycleGraphs[2];
     h->no_graphs = (std::getenv("TC_NO_GRAPHS") != nullptr);
     h->no_device_loop = (std::getenv("TC_HOST_LOOP") != nullptr);
     h->fuse_visits = (std::getenv("TC_NO_FUSED_VISITS") == nullptr) && visit_cluster_setup() > 0;
@@ -2398,18 +2398,27 @@ void drop_step_graphs(Handle* h) {
     h->epoch++;
 }
 
-// From its first ensemble step on a handle uses no launch that waits for the
-// whole GPU (tile_form): its graphs are captured again without them.
-void enter_ensemble(Handle* h) {
-    if (h->in_ensemble) return;
-    h->in_ensemble = true;
-    CycleGraphs& cg = *h->graphs;
-    if (cg.l1) cudaGraphExecDestroy(cg.l1);
-    if (cg.rest) cudaGraphExecDestroy(cg.rest);
-    if (cg.loop) cudaGraphExecDestroy(cg.loop);
-    cg.l1 = cg.rest = cg.loop = nullptr;
+// The graphs that bake in launch shapes and kernels: captured again at their next use.
+void drop_graphs(Handle* h) {
+    for (int f = 0; f < 2 && h->graphs; f++) {
+        CycleGraphs& cg = h->graphs[f];
+        if (cg.l1) cudaGraphExecDestroy(cg.l1);
+        if (cg.rest) cudaGraphExecDestroy(cg.rest);
+        if (cg.loop) cudaGraphExecDestroy(cg.loop);
+        cg.l1 = cg.rest = cg.loop = nullptr;
+    }
     drop_step_graphs(h);
 }
+
+// A call that steps several handles side by side: for as long as it lasts they use no
+// launch that waits for the whole GPU (tile_form), with graphs of their own.
+struct EnsembleCall {
+    tc_handle* const* hs;
+    int n;
+    EnsembleCall(tc_handle* const* hs_, int n_) : hs(hs_), n(n_) { mark(n > 1); }
+    ~EnsembleCall() { mark(false); }
+    void mark(bool on);
+};
 
 // The step can run as one captured graph: every loop of it on the device,
 // no host branch on a device value, and everything the first step builds
@@ -2423,7 +2432,7 @@ bool step_graph_ready(const Handle* h, bool own) {
     if (h->p.learned_guess == 1 || h->p.learned_guess == 2) return false;
     if (h->rec_raw && h->rec_count < h->rec_cap) return false;
     if (h->tstep < 1 || h->time == 0.0 || !h->lu_valid || (h->sub_on && !h->sub_valid)) return false;
-    return h->graphs != nullptr && h->graphs->loop != nullptr;
+    return h->graphs != nullptr && (h->graphs[0].loop != nullptr || h->graphs[1].loop != nullptr);
 }
 
 // what a captured step needs before its capture begins (allocations are
@@ -2508,7 +2517,7 @@ tc_status finish_step(Handle* h, const StepGraph& sg, tc_stats_row* row, int32_t
 // *ran when the step must run eagerly (a capture the CUDA runtime refused).
 tc_status step_as_graph(Handle* h, tc_stats_row* row, int32_t* cycles, double* dt_out, bool* ran) {
     *ran = false;
-    const int key = sorts_this_step(h) ? 1 : 0;
+    const int key = (sorts_this_step(h) ? 1 : 0) + (h->in_ensemble ? 2 : 0);
     StepGraph* sg = nullptr;
     auto it = h->step_graphs.find(key);
     if (it != h->step_graphs.end()) {
@@ -2536,6 +2545,11 @@ tc_status step_as_graph(Handle* h, tc_stats_row* row, int32_t* cycles, double* d
 struct tc_handle {
     Handle h;
 };
+namespace {
+void EnsembleCall::mark(bool on) {
+    for (int i = 0; i < n; i++) hs[i]->h.in_ensemble = on;
+}
+}  // namespace
 
 namespace {
 // time one replay of the launches `fn` enqueues, captured as a CUDA graph (ms)
@@ -2741,15 +2755,10 @@ tc_status tc_destroy(tc_handle* H) {
     for (void* q : h->allocs) cudaFree(q);
     if (h->eq_donor) cudaFree(h->eq_donor);
     if (h->hs) cudaFreeHost(h->hs);
-    if (h->graphs) {
-        if (h->graphs->l1) cudaGraphExecDestroy(h->graphs->l1);
-        if (h->graphs->rest) cudaGraphExecDestroy(h->graphs->rest);
-        if (h->graphs->loop) cudaGraphExecDestroy(h->graphs->loop);
-        delete h->graphs;
-    }
+    drop_graphs(h);
+    delete[] h->graphs;
     for (auto& kv : h->flt_graphs)
         if (kv.second) cudaGraphExecDestroy(kv.second);
-    drop_step_graphs(h);
     if (h->hsnap) cudaFreeHost(h->hsnap);
     if (h->body_st) cudaStreamDestroy(h->body_st);
     if (h->own_stream && h->st) cudaStreamDestroy(h->st);
@@ -3010,12 +3019,7 @@ tc_status tc_autotune(tc_handle* H, int32_t* choices) {
         }
     }
     // the cycle graphs bake in launch shapes: capture again at the next solve
-    CycleGraphs& cg = *h->graphs;
-    if (cg.l1) cudaGraphExecDestroy(cg.l1);
-    if (cg.rest) cudaGraphExecDestroy(cg.rest);
-    if (cg.loop) cudaGraphExecDestroy(cg.loop);
-    cg.l1 = cg.rest = cg.loop = nullptr;
-    drop_step_graphs(h);
+    drop_graphs(h);
     return TC_OK;
 }
 
@@ -3043,12 +3047,7 @@ tc_status tc_set_launch_shapes(tc_handle* H, const int32_t* choices) {
         lv.visit_cfg = (v > 1 && v < 1000) ? v : 0;
         lv.blk = (v > 1000) ? v - 1000 : 0;
     }
-    CycleGraphs& cg = *h->graphs;
-    if (cg.l1) cudaGraphExecDestroy(cg.l1);
-    if (cg.rest) cudaGraphExecDestroy(cg.rest);
-    if (cg.loop) cudaGraphExecDestroy(cg.loop);
-    cg.l1 = cg.rest = cg.loop = nullptr;
-    drop_step_graphs(h);
+    drop_graphs(h);
     return TC_OK;
 }
 
@@ -3057,7 +3056,7 @@ tc_status tc_ensemble_step(tc_handle* const* hs, int32_t n, int32_t nthreads, tc
     if (!hs || n < 1 || nthreads < 1) return TC_ERR_ARG;
     for (int i = 0; i < n; i++)
         if (!hs[i]) return TC_ERR_ARG;
-    for (int i = 0; i < n; i++) enter_ensemble(&hs[i]->h);
+    const EnsembleCall together(hs, n);
     std::atomic<int> next{0};
     std::vector<tc_status> st((size_t)n, TC_OK);
     auto work = [&]() {
@@ -3116,10 +3115,11 @@ tc_status tc_ensemble_create(int32_t nthreads, tc_ensemble** out) {
 tc_status tc_ensemble_run(tc_ensemble* e, tc_handle* const* hs, int32_t n, tc_stats_row* rows, int32_t* cycles,
                           double* dts, tc_status* status) {
     if (!e || !hs || n < 1) return TC_ERR_ARG;
+    for (int i = 0; i < n; i++)
+        if (!hs[i]) return TC_ERR_ARG;
+    const EnsembleCall together(hs, n);
     bool ready = !e->failed;
     for (int i = 0; i < n; i++) {
-        if (!hs[i]) return TC_ERR_ARG;
-        enter_ensemble(&hs[i]->h);
         ready = ready && step_graph_ready(&hs[i]->h, false) && hs[i]->h.device == e->device;
     }
     tc_ensemble::Entry* en = nullptr;
@@ -3317,12 +3317,7 @@ tc_status tc_debug_wait_test(tc_handle* H, int32_t on) {
     Handle* h = &H->h;
     h->wait_test = (on != 0);
     // the cycle graphs bake in the visits' parameters: capture again
-    CycleGraphs& cg = *h->graphs;
-    if (cg.l1) cudaGraphExecDestroy(cg.l1);
-    if (cg.rest) cudaGraphExecDestroy(cg.rest);
-    if (cg.loop) cudaGraphExecDestroy(cg.loop);
-    cg.l1 = cg.rest = cg.loop = nullptr;
-    drop_step_graphs(h);
+    drop_graphs(h);
     return TC_OK;
 }
 
@@ -3331,12 +3326,7 @@ tc_status tc_debug_refuse_clusters(tc_handle* H, int32_t on) {
     Handle* h = &H->h;
     for (int l = 1; l <= h->grids; l++) h->lev[l].no_cluster = (on != 0);
     // the cycle graphs bake in the kernels: capture again
-    CycleGraphs& cg = *h->graphs;
-    if (cg.l1) cudaGraphExecDestroy(cg.l1);
-    if (cg.rest) cudaGraphExecDestroy(cg.rest);
-    if (cg.loop) cudaGraphExecDestroy(cg.loop);
-    cg.l1 = cg.rest = cg.loop = nullptr;
-    drop_step_graphs(h);
+    drop_graphs(h);
     return TC_OK;
 }
 
@@ -3345,12 +3335,7 @@ tc_status tc_debug_sweep_fields(tc_handle* H, int32_t fields) {
     Handle* h = &H->h;
     if (h->lev[1].g32 == nullptr) return TC_ERR_UNSUPPORTED;
     h->lev[1].use_g32 = fields ? 1 : 0;
-    CycleGraphs& cg = *h->graphs;
-    if (cg.l1) cudaGraphExecDestroy(cg.l1);
-    if (cg.rest) cudaGraphExecDestroy(cg.rest);
-    if (cg.loop) cudaGraphExecDestroy(cg.loop);
-    cg.l1 = cg.rest = cg.loop = nullptr;
-    drop_step_graphs(h);
+    drop_graphs(h);
     return TC_OK;
 }
 
