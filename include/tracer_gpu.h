@@ -402,22 +402,28 @@ tc_status tc_step_host(tc_handle* h, double* T, double* Cnew, double* SF, double
  * on this handle's GPU and in its solver precision, the per-sweep smoother
  * kernel under eight block shapes of at most 256 threads, then visits of 1
  * to 6 sweeps per launch of the tiled smoother (FP64: 1 or 2) and fused
- * cluster visits of every shape that fits (1 or 2 points per thread strip,
- * 1 to 16 CTAs), with CUDA-graph replays, and keeps the fastest of each.
+ * cluster visits of every shape that fits (the default one, and 1 or 2 points
+ * per thread strip on 1 to 16 CTAs), with CUDA-graph replays, and keeps the
+ * fastest of each.  In the mixed solver it also times, on levels too large for
+ * one cluster, the fused visit over the whole grid, which a handle uses only
+ * when it is stepped alone: in ensembles the fastest of the others holds.
  * Results are unchanged by the choice (the arithmetic per point does not
  * depend on the launch shape).  If `choices` is not NULL it receives (block
  * x, block y, visit) for levels 1..grids-1, visit = 0 for one launch per
  * sweep, 1000 + n for n sweeps per launch, 1 for the default fused shape,
- * else 100 x points per strip + CTAs.  Needs uploaded state; the levels'
+ * else 100 x points per strip + CTAs; 10000 is added where the visit over the
+ * whole grid is faster still.  Needs uploaded state; the levels'
  * corrections are restored afterwards. */
 tc_status tc_autotune(tc_handle* h, int32_t* choices);
 /* Applies launch shapes in tc_autotune's `choices` format (3 ints per level
- * 1..grids-1: sweep block x, block y, visit = 0 one launch per sweep / 1
- * default fused visit / 100*P + C / 1000 + n for n sweeps per launch of the
- * tiled smoother, n = 1..2, or 1..6 in the mixed solver), e.g. shapes tuned once on
- * another handle of the same grid and precision.  TC_ERR_ARG (nothing
- * changed) if a block has more than 256 threads or a visit shape does not fit
- * its level.  Shapes do not change the arithmetic. */
+ * 1..grids-1: sweep block x, block y, visit = 0 one launch per sweep / 1 an
+ * untuned handle's visit (fused wherever one fits) / 100*P + C / 1000 + n for n
+ * sweeps per launch of the tiled smoother, n = 1..2, or 1..6 in the mixed
+ * solver / 10000 + any of these: over the whole grid when stepped alone, else
+ * that), e.g. shapes tuned once on another handle of the same grid and
+ * precision.  TC_ERR_ARG (nothing changed) if a block has more than 256
+ * threads or a visit shape does not fit its level.  Shapes do not change the
+ * arithmetic. */
 tc_status tc_set_launch_shapes(tc_handle* h, const int32_t* choices);
 
 /* Ensemble of independent cases (no reference counterpart: the reference

@@ -896,14 +896,13 @@ static void sweep_factors(int Niter, int n, int dir, bool cheb_pp, double* c, do
 // How the mixed solve's tile smoother (k_tile.cu) runs a visit of `level`: in one
 // cluster where the level fits (the other SMs stay free), else over the grid, a
 // cooperative launch that waits for all SMs: not in an ensemble, whose cases
-// share them.
+// share them.  There the level's fuse, visit_cfg and blk hold.
 enum { kTileNone = 0, kTileCluster, kTileGrid };
 static int tile_form(const Handle* h, int level, int per_point) {
     const Level& lv = h->lev[level];
-    if (!(h->p.solver_precision == 1 && h->fuse_visits && lv.fuse && lv.visit_cfg == 0 && level < h->grids))
-        return kTileNone;
-    if (tile_visit_fits(lv.L, h->p.Nmulti, per_point)) return kTileCluster;
-    return (lv.tile_inbox != nullptr && !h->in_ensemble) ? kTileGrid : kTileNone;
+    if (!(h->p.solver_precision == 1 && h->fuse_visits && level < h->grids)) return kTileNone;
+    if (lv.grid && !h->in_ensemble) return kTileGrid;
+    return (lv.fuse && lv.visit_cfg == 0 && tile_visit_fits(lv.L, h->p.Nmulti, per_point)) ? kTileCluster : kTileNone;
 }
 
 // Would iterate_stream / iterate_stream32 smooth `level` in direction dir as
@@ -911,9 +910,10 @@ static int tile_form(const Handle* h, int level, int per_point) {
 static bool visit_fuses(Handle* h, int level, int dir) {
     const Level& lv = h->lev[level];
     const bool mixed = (h->p.solver_precision == 1);
-    if (!(h->fuse_visits && lv.fuse && level > 1 && level < h->grids && h->p.Nmulti <= 128)) return false;
+    if (!(h->fuse_visits && level > 1 && level < h->grids && h->p.Nmulti <= 128)) return false;
     const bool pp = (dir != 1 && level == h->ratio_level);
     if (tile_form(h, level, pp ? 1 : 0) != kTileNone) return true;
+    if (!lv.fuse) return false;
     if (!visit_cluster_fits(lv.L, h->p.Nmulti, mixed ? 1 : 0, lv.visit_cfg)) return false;
     return mixed || !pp || h->ctab_level == level;
 }
@@ -1078,10 +1078,9 @@ void iterate_stream32(Handle* h, int level, int dir, int pro = 0, int rst = 0, i
     const int Niter = h->p.Nmulti;
     const bool cheb_pp = (level == h->ratio_level);
     const int pp = (dir != 1 && cheb_pp) ? 1 : 0;
-    // lv.fuse with no explicit shape: the tile smoother (k_tile.cu), the whole visit
-    // in one launch
+    // the tile smoother (k_tile.cu): the whole visit in one launch
     const int tiles = tile_form(h, level, pp);
-    if (h->fuse_visits && lv.fuse && Niter <= 128) {
+    if (h->fuse_visits && (lv.fuse || tiles != kTileNone) && Niter <= 128) {
         double cv[128], tv[128];
         cheb_temps(Niter, dir, tv, cv);
         VisitXfer<float> x;
@@ -1108,8 +1107,9 @@ void iterate_stream32(Handle* h, int level, int dir, int pro = 0, int rst = 0, i
                                   level > 1 ? lv.res32 : nullptr, &h->ds->visit_timeout, &x, tf) == 0)
                 return;
         }
-        if (level > 1 && launch_visit_cluster32(h->st, lv, cur_e32(h, level), cv, tv, Niter, pp, h->p.Vbc,
-                                                &h->ds->visit_timeout, &x, tf) == 0)
+        if (lv.fuse && level > 1 &&
+            launch_visit_cluster32(h->st, lv, cur_e32(h, level), cv, tv, Niter, pp, h->p.Vbc, &h->ds->visit_timeout, &x,
+                                   tf) == 0)
             return;
     }
     if (pro) launch_prolong32(h->st, h->lev[level + 1], lv, cur_e32(h, level + 1), cur_e32(h, level), h->p.Vbc);
@@ -2144,6 +2144,8 @@ tc_status create(Handle* h, const tc_params* in) {
         if (p.solver_precision == 1 && l > 1 && !(h->fuse_visits && visit_cluster_fits(lv.L, p.Nmulti, 1)) &&
             sweep_blk_tiles(lv.L) <= n_sms)
             lv.blk = 6;
+        lv.blk_untuned = lv.blk;
+        lv.grid = 0;
         lv.coef32 = lv.dts32 = lv.cA32 = lv.cB32 = lv.rhs32 = lv.res32 = nullptr;
         lv.e32[0] = lv.e32[1] = nullptr;
         lv.e32cur = 0;
@@ -2164,6 +2166,7 @@ tc_status create(Handle* h, const tc_params* in) {
                 TRY(dalloc_t(h, &lv.tile_inbox, words));
                 TRY(dalloc_t(h, &lv.tile_count, (size_t)tiles));
                 lv.tile_counts = tiles;
+                lv.grid = 1;
             }
         }
         tcs::LevSpacing s;
@@ -2927,6 +2930,9 @@ tc_status tc_step(tc_handle* H, tc_stats_row* row, int32_t* cycles, double* dt_o
 }
 
 
+// added to a visit's shape: over the whole grid when the handle is stepped alone
+static constexpr int kShapeGrid = 10000;
+
 tc_status tc_autotune(tc_handle* H, int32_t* choices) {
     if (!H) return TC_ERR_ARG;
     Handle* h = &H->h;
@@ -2975,6 +2981,7 @@ tc_status tc_autotune(tc_handle* H, int32_t* choices) {
         };
         lv.fuse = 0;
         lv.visit_cfg = 0;
+        lv.grid = 0;
         double best_v = 1e30;
         int best_blk = 0;
         const bool gf = lv.g32 && lv.use_g32;
@@ -3006,6 +3013,13 @@ tc_status tc_autotune(tc_handle* H, int32_t* choices) {
         }
         lv.fuse = (best_cfg >= 0) ? 1 : 0;
         lv.visit_cfg = (best_cfg > 0) ? best_cfg : 0;
+        // last the visit over the whole grid; the shape found so far holds in ensembles
+        if (lv.tile_inbox != nullptr) {
+            lv.grid = 1;
+            double ms = 0;
+            TRY(time_visits(&ms));
+            if (!(ms < best_v)) lv.grid = 0;
+        }
         for (int q = 0; q < 2; q++) {
             CK(cudaMemcpyAsync(mixed ? (void*)lv.e32[q] : (void*)lv.err[q], save[q], bytes, cudaMemcpyDeviceToDevice,
                                h->st));
@@ -3015,7 +3029,8 @@ tc_status tc_autotune(tc_handle* H, int32_t* choices) {
         if (choices) {
             choices[3 * (l - 1) + 0] = lv.sweep_bx;
             choices[3 * (l - 1) + 1] = lv.sweep_by;
-            choices[3 * (l - 1) + 2] = lv.fuse ? (lv.visit_cfg ? lv.visit_cfg : 1) : (lv.blk > 0 ? 1000 + lv.blk : 0);
+            choices[3 * (l - 1) + 2] = (lv.fuse ? (lv.visit_cfg ? lv.visit_cfg : 1) : (lv.blk > 0 ? 1000 + lv.blk : 0)) +
+                                       (lv.grid ? kShapeGrid : 0);
         }
     }
     // the cycle graphs bake in launch shapes: capture again at the next solve
@@ -3029,7 +3044,12 @@ tc_status tc_set_launch_shapes(tc_handle* H, const int32_t* choices) {
     const bool mixed = (h->p.solver_precision == 1);
     const int G = h->grids;
     for (int l = 1; l < G; l++) {
-        const int bx = choices[3 * (l - 1)], by = choices[3 * (l - 1) + 1], v = choices[3 * (l - 1) + 2];
+        const int bx = choices[3 * (l - 1)], by = choices[3 * (l - 1) + 1];
+        int v = choices[3 * (l - 1) + 2];
+        if (v >= kShapeGrid) {
+            if (h->lev[l].tile_inbox == nullptr) return TC_ERR_ARG;
+            v -= kShapeGrid;
+        }
         if (bx < 1 || by < 1 || bx * by > 256 || (bx * by) % 32 != 0 || v < 0) return TC_ERR_ARG;
         if (v > 1000) {
             if (!(v == 1001 || v == 1002 || (v >= 1003 && v <= 1006 && mixed))) return TC_ERR_ARG;
@@ -3042,10 +3062,11 @@ tc_status tc_set_launch_shapes(tc_handle* H, const int32_t* choices) {
         Level& lv = h->lev[l];
         lv.sweep_bx = choices[3 * (l - 1)];
         lv.sweep_by = choices[3 * (l - 1) + 1];
-        const int v = choices[3 * (l - 1) + 2];
+        const int v = choices[3 * (l - 1) + 2] % kShapeGrid;
         lv.fuse = (v != 0 && v < 1000) ? 1 : 0;
         lv.visit_cfg = (v > 1 && v < 1000) ? v : 0;
-        lv.blk = (v > 1000) ? v - 1000 : 0;
+        lv.blk = (v > 1000) ? v - 1000 : (v == 1) ? lv.blk_untuned : 0;
+        lv.grid = lv.tile_inbox != nullptr && choices[3 * (l - 1) + 2] >= (v == 1 ? 1 : kShapeGrid);
     }
     drop_graphs(h);
     return TC_OK;

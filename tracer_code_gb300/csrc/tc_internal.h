@@ -193,7 +193,9 @@ struct Level {
     unsigned long long* tile_inbox;
     unsigned* tile_count;
     int tile_counts;
+    int grid;       // 1 = such a visit when the handle is stepped alone, else as below
     int no_cluster;  // 1: clusters and cooperative grids count as refused (tc_debug_refuse_clusters)
+    int blk_untuned;  // blk before any tuning
     int blk;        // when not fused: 0 = one k_sweep / k_sweep32 launch per sweep, n = n sweeps per k_sweep_blk launch
     MetricFold mfold;  // stretched grids: the tap weights of the computational derivatives
 };
