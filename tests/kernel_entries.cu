@@ -103,6 +103,14 @@ int entry_solve(const double* AB, const int* ipiv, const double* rowb, int a, in
     return 0;
 }
 
+// whether a level of a x b cells takes the one-launch viscosity filter
+int entry_vis_filter_fits(int a, int b, int stretched, int interpolate) {
+    Level lv{};
+    lv.L = layout(a, b);
+    lv.c.M.on = stretched;
+    return vis_filter_fits(lv, interpolate) ? 1 : 0;
+}
+
 // x [nb][H][W][x_tot], dz [nb][H][W][cout] BF16; part: entry_wgrad_splits x cout x 9 x cin
 int entry_wgrad_splits(int nb, int H, int W, int cin) { return wgrad_splits(nb, H, W, cin); }
 int entry_wgrad(const uint16_t* x, int x_tot, int x_off, int cin, const uint16_t* dz, int cout, int nb, int H, int W,

@@ -262,14 +262,11 @@ void launch_vis_smooth(cudaStream_t s, const Level& lv, const double* vin, doubl
 // points per SM at a time, and L2 latency.  The graph's loop took four nodes a step, 20 to
 // 25 us whatever the level, and twelve copies around an interpolation: the viscosities of
 // levels 2 to 4 of a 256x64 grid 330 + 320 + 131 us, now 116 + 65 + 35.  Larger levels keep
-// the graphs: with the ratio one cluster's FP64 pipes cost as much as the nodes at 16,700
-// points (151 us against 145); stretched grids take some 30 divisions a point.
+// the graphs: see vis_filter_fits.
 // ---------------------------------------------------------------------------
 #define VF_THREADS 512
 #define VF_CL 16
-#define VF_MAX_SMOOTH 17000  // points, without and with the ratio in each pass
-#define VF_MAX_RATIO 12000
-#define VF_MAX_RATIO_METRIC 4500
+#define VF_MAX_RATIO_METRIC 4500  // points of a stretched level with the ratio in each pass
 template <bool METRIC>
 __global__ void __launch_bounds__(VF_THREADS) k_vis_filter(Lay L, LevConst c, VisFltArgs q, int reset,
                                                            const double* src, double* A, double* B,
@@ -418,9 +415,18 @@ __global__ void __launch_bounds__(VF_THREADS) k_vis_filter(Lay L, LevConst c, Vi
         if (status != 0) ds->flt_status = status;
     }
 }
+// The time goes with the points a thread has, the graph's hardly with the level.  A viscosity
+// in one launch against the graph, spacings that are no powers of two:
+//   only smoothing        one point a thread (176x44) 101 us against 209, two (224x56) 150
+//                         against 204, three (272x68) 202 against 195
+//   with the ratio        one (176x44) 146 against 165, two (192x48) 231 against 162
+//   smoothing, stretched  one (176x44) 281 against 318, two (192x48) 495 against 317
+//   ratio, stretched      some 30 divisions a point: 128x32 374 against 420, 176x44 710
+//                         against 434
 bool vis_filter_fits(const Level& lv, int interpolate) {
-    const int points = (lv.L.a + 1) * (lv.L.b + 1);
-    return points <= (interpolate ? VF_MAX_SMOOTH : lv.c.M.on ? VF_MAX_RATIO_METRIC : VF_MAX_RATIO);
+    const int a = lv.L.a, b = lv.L.b, threads = VF_THREADS * VF_CL;
+    if (!interpolate && lv.c.M.on) return (a + 1) * (b + 1) <= VF_MAX_RATIO_METRIC;
+    return (a + 1) * (b - 1) <= (interpolate && !lv.c.M.on ? 2 : 1) * threads;
 }
 // false where the device does not take the cluster: nothing ran, the loop graphs can
 bool launch_vis_filter(cudaStream_t s, const Level& lv, const VisFltArgs& q, int reset, const double* src, double* A,
