@@ -111,6 +111,11 @@ int entry_vis_filter_fits(int a, int b, int stretched, int interpolate) {
     return vis_filter_fits(lv, interpolate) ? 1 : 0;
 }
 
+// whether a visit of a x b cells with the per-point factor takes the row-strip kernel
+int entry_visit_cluster_beats_tiles(int a, int b, int nsweeps) {
+    return visit_cluster_beats_tiles(layout(a, b), nsweeps) ? 1 : 0;
+}
+
 // x [nb][H][W][x_tot], dz [nb][H][W][cout] BF16; part: entry_wgrad_splits x cout x 9 x cin
 int entry_wgrad_splits(int nb, int H, int W, int cin) { return wgrad_splits(nb, H, W, cin); }
 int entry_wgrad(const uint16_t* x, int x_tot, int x_off, int cin, const uint16_t* dz, int cout, int nb, int H, int W,

@@ -645,6 +645,18 @@ int visit_cluster_fits(const Lay& L, int nsweeps, int fp32, int cfg) {
     return visit_shape(L, nsweeps, fp32 != 0, cfg, &s) ? 1 : 0;
 }
 
+// FP32 visits with the per-point factor: whether this kernel beats the tile visits
+// (k_tile.cu).  It does with one point a thread (a visit of 70 sweeps takes 30.5 to 32.5 us
+// whatever the level, the tiles 31.4 to 33.9: 64x64 31.5 against 33.9, 40x24 30.3 against 32.6),
+// except where the tiles are one CTA or one row of at least four (16x16 30.6 against 26.6,
+// 64x16 30.6 against 27.8).  With two points a thread (72x56 53.1 against 37.2) it does not,
+// nor with the uniform factor.
+bool visit_cluster_beats_tiles(const Lay& L, int nsweeps) {
+    VisitShape s;
+    return visit_shape(L, nsweeps, true, 0, &s) && s.p == 1 && (L.a - 1) * (L.b - 1) > 440 &&
+           !(L.a >= 64 && L.b <= 24);
+}
+
 template <typename T>
 static void cheb_table_t(cudaStream_t s, const Lay& L, const double* tvals, int nsweeps, const T* cA, const T* cB,
                          T* tab) {

@@ -902,6 +902,7 @@ static int tile_form(const Handle* h, int level, int per_point) {
     const Level& lv = h->lev[level];
     if (!(h->p.solver_precision == 1 && h->fuse_visits && level < h->grids)) return kTileNone;
     if (lv.grid && !h->in_ensemble) return kTileGrid;
+    if (level > 1 && per_point && visit_cluster_beats_tiles(lv.L, h->p.Nmulti)) return kTileNone;
     return (lv.fuse && lv.visit_cfg == 0 && tile_visit_fits(lv.L, h->p.Nmulti, per_point)) ? kTileCluster : kTileNone;
 }
 

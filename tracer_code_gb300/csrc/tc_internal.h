@@ -258,6 +258,7 @@ void launch_copy_plane(cudaStream_t s, double* dst, const double* src, size_t n)
 // (k_visit.cu) one whole smoother visit of a small level as one cluster launch
 int visit_cluster_setup();
 int visit_cluster_fits(const Lay& L, int nsweeps, int fp32, int cfg = 0);
+bool visit_cluster_beats_tiles(const Lay& L, int nsweeps);
 void launch_cheb_table(cudaStream_t s, const Level& lv, const double* tvals, int nsweeps, double* tab);
 // grid transfers a visit can do in the same launch (nullptr = none): add the
 // prolongation of the next coarser level's correction ec before the first
