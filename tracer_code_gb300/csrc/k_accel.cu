@@ -503,8 +503,6 @@ void launch_accel_window(cudaStream_t s, const Level& l1, double* psi, double* p
     Range2 r{1, l1.L.a - 1, 1, l1.L.b - 1};
     const int nsm = tc_sm_count();
     const int npts = (l1.L.a - 1) * (l1.L.b - 1);
-    // grid-stride over the points with one wave of CTAs (three per SM: the
-    // kernel's launch bounds), so that the block sums and their fold stay few
     // one CTA of 256 threads per SM, grid-stride over the points: the block
     // sums of the up to 20 FP64 products cost per thread, so few threads with
     // several points each are fastest (measured at 1024x256 with one smoother launch

@@ -569,8 +569,9 @@ void launch_level_coefs(cudaStream_t s, const Level& lv, const double* vis, int 
 // ---------------------------------------------------------------------------
 
 // One FP64 sweep, a point per thread.  What bounds it is the FP64 pipe, 14 operations a
-// point after the wait (c * dt is formed before it, ghost signs change as bits): 1024x256
-// points 8.6 -> 8.4 us a sweep with 17 before (now 8.2, floor 6.1), 512x128 3.5 -> 3.3.
+// point after the wait (c * dt is formed before it, ghost signs change as bits): 8.2 us a
+// sweep of 1024x256 points (the pipe alone 6.1), 3.3 of 512x128; with 17 operations and the
+// next launch released at the end 8.6 and 3.5.
 __global__ void __launch_bounds__(256, 1) k_sweep(Lay L, Range2 r, const double* Sin, double* Sout,
                         const double* __restrict__ coef, const double* rhs,
                         const double* __restrict__ dts, const double* __restrict__ cA, const double* __restrict__ cB,

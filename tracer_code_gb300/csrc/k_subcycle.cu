@@ -311,8 +311,8 @@ __device__ __forceinline__ void store_stream4(const Lay& L, float4* S, int i, in
     for (int g = 0; g < n; g++) S[idx[g]] = f4_scale(sg[g], v);
 }
 
-template <int P, int GR, int NT, int MB>
-__global__ void __launch_bounds__(NT, MB) k_subcycle_build4(SubArgs<float> A, const float* __restrict__ Ac) {
+template <int P, int GR, int NT>
+__global__ void __launch_bounds__(NT, 1) k_subcycle_build4(SubArgs<float> A, const float* __restrict__ Ac) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     // planes without the global layout's row padding
     Lay LS = A.LS, LG = A.LG;
@@ -596,12 +596,12 @@ size_t build_smem(const Lay& LS, const Lay& LG) {
     return sizeof(T) * (4 * LS.plane + 2 * LG.plane);
 }
 
-template <int P, int GR, int NT, int MB>
+template <int P, int GR, int NT>
 int launch_build4_as(cudaStream_t s, const SubArgs<float>& A, float* Ac, size_t smem) {
-    if (cudaFuncSetAttribute(k_subcycle_build4<P, GR, NT, MB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+    if (cudaFuncSetAttribute(k_subcycle_build4<P, GR, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
         cudaSuccess)
         return -1;
-    k_subcycle_build4<P, GR, NT, MB><<<(A.nS + 4 * GR - 1) / (4 * GR), NT, smem, s>>>(A, Ac);
+    k_subcycle_build4<P, GR, NT><<<(A.nS + 4 * GR - 1) / (4 * GR), NT, smem, s>>>(A, Ac);
     tc_note_launch();
     return cudaPeekAtLastError() == cudaSuccess ? 0 : -1;
 }
@@ -616,8 +616,8 @@ int launch_build4(cudaStream_t s, const SubArgs<float>& A, float* Ac) {
     // else one (a 93x11 level, 606 us)
     const int strips = A.LS.b / 2;
     if ((A.LS.a - 1) * strips <= 512 && 2 * smem <= 200 * 1024)
-        return launch_build4_as<2, 2, 512, 1>(s, A, Ac, 2 * smem);
-    return launch_build4_as<1, 1, 1024, 1>(s, A, Ac, smem);
+        return launch_build4_as<2, 2, 512>(s, A, Ac, 2 * smem);
+    return launch_build4_as<1, 1, 1024>(s, A, Ac, smem);
 }
 
 template <typename T>

@@ -82,9 +82,6 @@ struct TileParams {
 // not kept: the taps one column off need register moves, and a sweep is bound by
 // latency, not by multiply-add issue (256x64: 42.9 us a visit against 41.8).
 typedef float2 f2;
-__device__ __forceinline__ f2 pack2(float a, float b) { return make_float2(a, b); }
-__device__ __forceinline__ float lo2(f2 v) { return v.x; }
-__device__ __forceinline__ float hi2(f2 v) { return v.y; }
 __device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) { return make_float2(fmaf(a.x, b.x, c.x), fmaf(a.y, b.y, c.y)); }
 __device__ __forceinline__ f2 mul2(f2 a, f2 b) { return make_float2(a.x * b.x, a.y * b.y); }
 __device__ __forceinline__ f2 ld2(const float* p) { return *reinterpret_cast<const f2*>(p); }
@@ -159,8 +156,8 @@ __device__ __forceinline__ void patch_coefs(Patch<PR>& P, const PatchEdge& E, co
         if (E.jr == 0) cf[0][4] = -cf[0][4];
         if (E.jr == 1) cf[1][4] = -cf[1][4];
 #pragma unroll
-        for (int d = 0; d < TC_NCOEF; d++) P.cf[q][d] = pack2(cf[0][d], cf[1][d]);
-        P.dt[q] = pack2(dt[0], dt[1]);
+        for (int d = 0; d < TC_NCOEF; d++) P.cf[q][d] = make_float2(cf[0][d], cf[1][d]);
+        P.dt[q] = make_float2(dt[0], dt[1]);
     }
 }
 template <int PR>
@@ -173,7 +170,7 @@ __device__ __forceinline__ void patch_rhs(Patch<PR>& P, const Lay& L, int x, int
             const bool act = x + j >= 1 && x + j <= L.a - 1 && y + q >= 1 && y + q <= L.b - 1;
             r[j] = act ? ld_state(rhs + IX(L, x + j, y + q)) : 0.f;
         }
-        P.rh[q] = pack2(r[0], r[1]);
+        P.rh[q] = make_float2(r[0], r[1]);
     }
 }
 template <int W, int PR>
@@ -187,7 +184,7 @@ __device__ __forceinline__ void patch_ghosts(Patch<PR>& P, const PatchEdge& E, f
     if (!E.fix) return;
     if (E.jr == 1) {
 #pragma unroll
-        for (int q = 0; q < PR; q++) p[q * W + 3] = hi2(P.own[q]);
+        for (int q = 0; q < PR; q++) p[q * W + 3] = P.own[q].y;
     }
 #pragma unroll
     for (int q = 0; q + 2 < PR; q++)
@@ -215,8 +212,8 @@ __device__ __forceinline__ void patch_residual(const Patch<PR>& P, const PatchEd
     }
 #pragma unroll
     for (int q = 0; q < PR + 2; q++) {
-        A[q] = pack2(hi2(Lf[q]), lo2(M[q + 1]));
-        B[q] = pack2(hi2(M[q + 1]), lo2(Rt[q]));
+        A[q] = make_float2(Lf[q].y, M[q + 1].x);
+        B[q] = make_float2(M[q + 1].y, Rt[q].x);
     }
 #pragma unroll
     for (int q = 0; q < PR; q++) acc[q] = fma2(P.cf[q][0], M[q + 2], P.rh[q]);
@@ -257,8 +254,8 @@ __device__ __forceinline__ void patch_sweep(Patch<PR>& P, const PatchEdge& E, co
     // next to an interior point is stored again with it
 #pragma unroll
     for (int q = 0; q < PR; q++) {
-        const f2 cp = PP ? pack2(2.0f / (lo2(ca[q]) + lo2(cb[q]) * temp), 2.0f / (hi2(ca[q]) + hi2(cb[q]) * temp))
-                         : pack2(c, c);
+        const f2 cp = PP ? make_float2(2.0f / (ca[q].x + cb[q].x * temp), 2.0f / (ca[q].y + cb[q].y * temp))
+                         : make_float2(c, c);
         P.own[q] = fma2(mul2(cp, P.dt[q]), acc[q], P.own[q]);
         st2(pn + q * W, P.own[q]);
     }
@@ -400,8 +397,8 @@ __global__ void __launch_bounds__(NT, 1) k_tile_visit(const __grid_constant__ Ti
                 A[j] = act ? __ldg(cA + IX(L, x + j, y + q)) : 1.f;
                 B[j] = act ? __ldg(cB + IX(L, x + j, y + q)) : 0.f;
             }
-            ca[q] = pack2(A[0], A[1]);
-            cb[q] = pack2(B[0], B[1]);
+            ca[q] = make_float2(A[0], A[1]);
+            cb[q] = make_float2(B[0], B[1]);
         }
     }
     // the exchange list, in pieces of four columns: for each neighbour the owned
@@ -555,7 +552,7 @@ __global__ void __launch_bounds__(NT, 1) k_tile_visit(const __grid_constant__ Ti
 #pragma unroll
                 for (int j = 0; j < PC; j++)
                     if (x + j >= 1 && x + j <= a - 1 && y + q <= b - 1)
-                        store_stream<float>(L, Sg, x + j, y + q, j ? hi2(P.own[q]) : lo2(P.own[q]), Q.Vbc);
+                        store_stream<float>(L, Sg, x + j, y + q, j ? P.own[q].y : P.own[q].x, Q.Vbc);
         }
         if (need_res) {
             float* rb = buf + (size_t)(first ^ 1) * bsz;
@@ -568,7 +565,7 @@ __global__ void __launch_bounds__(NT, 1) k_tile_visit(const __grid_constant__ Ti
                 for (int q = 0; q < PR; q++)
 #pragma unroll
                     for (int j = 0; j < PC; j++) {
-                        const float r = j ? hi2(acc[q]) : lo2(acc[q]);
+                        const float r = j ? acc[q].y : acc[q].x;
                         if (Q.rc != nullptr) rb[o + q * W + j] = r;
                         else if (owned && x + j >= 1 && x + j <= a - 1 && y + q <= b - 1)
                             res[IX(L, x + j, y + q)] = r;
