@@ -1119,7 +1119,9 @@ __global__ void __launch_bounds__(2 * T) k_lu_panel(double* ABg, int* ipiv, int 
         if (ahead) {
             // The FP64 pipe is the panel's while this CTA holds the pivot chain: these
             // columns wait until it has passed -- at once, with the steps of panel p-1
-            // done, or just before it comes, by the time they have until then.
+            // done, or just before it comes, by the time they have until then.  (n = 1089,
+            // kl = 62: 1.21 ms; all at once 1.72; the lines at 3 and 8 instead of 6 and 10 1.22,
+            // at 9 and 12 1.27.  kl = 202: 3.17, 4.89, 3.26, 3.67; kl = 300: 3.14, 4.51, 3.23, 3.55)
             auto chain_passed = [] { asm volatile("bar.sync 3, %0;" ::"n"(2 * T) : "memory"); };
             const int pause = c < 6 ? -1 : c < 10 ? 0 : c - 1;
             int ju = 0, info = 0;
@@ -1301,8 +1303,8 @@ bool launch_lu_panels(cudaStream_t s, double* band, int* ipiv, int n, int kl, in
     cudaFuncSetAttribute(k_lu_panel<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     // the columns behind the panel two to four per SM, on up to seven clusters with the
     // panel's: an eighth of the chip stays free for the next launch's panel, whose CTAs then
-    // share no SM with this launch's (n = 2600, kl = 202: 3.23 ms; with eight clusters 3.62,
-    // with six 3.47)
+    // share no SM with this launch's (n = 2600, kl = 202: 3.17 ms; with eight clusters 3.47,
+    // with six 3.38; n = 1800, kl = 300: 3.14, 5.48 and 3.31; the same below kl = 126)
     const int clusters = 1 + std::min(6, (kl + ku + 31) / 32);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(LUP_CL * clusters, 1, 1);
